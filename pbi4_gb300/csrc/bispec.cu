@@ -1,5 +1,5 @@
-// bispec.cu -- shell tables, shell-filtered k-maps, CUDA-core triangle sums,
-// exact triangle counts and the bispectrum output rows.
+// bispec.cu -- shell tables, shell-filtered k-maps, exact triangle counts and
+// the bispectrum output rows.
 //
 // Reference: bispectrumI4.f90 measure_bk (1-198), measure_bk_multipoles
 // (200-516), measure_bk_cross (518-761), count_triangles (763-915).
@@ -23,10 +23,6 @@
 #include <vector>
 
 namespace pbi4g {
-
-constexpr int kTP = 4;   // pairs per thread tile
-constexpr int kTQ = 8;   // q maps per thread tile
-constexpr int kGroupThreads = 256;
 
 // ------------------------------------------------------------- Shells ---
 // Smallest multiple of 4 above 3 kmax that the map transform handles fast
@@ -117,117 +113,6 @@ int Shells::build(int N_, float kbin_, float kcenter_, int nb_, int iopen_, int 
     PBI4G_CHECK(nmodes_d.ensure(sizeof(double) * nb));
     PBI4G_CUDA(cudaMemcpyAsync(nmodes_d.p, nm.data(), sizeof(double) * nb, cudaMemcpyHostToDevice, st));
     PBI4G_CUDA(cudaStreamSynchronize(st));
-    return PBI4G_OK;
-}
-
-// ------------------------------------------------------------ TriPlan ---
-// Output slot (m, s) = m * nsets + s.  Non-cross: S = sum M_i M_j Q_{s,l}, pair
-// (i, j) of set-0 maps, q = map s*nb + l-1.  Cross: S = sum Q_i M_j M_l, pair
-// (j, l) of set-0 maps, q = map qset*nb + i-1.
-int TriPlan::build(const Shells &sh, int nsets_, int cross_, int max_pairs, int qoff) {
-    nsets = nsets_;
-    cross = cross_;
-    const int nb = sh.nb;
-    std::map<std::pair<int, int>, int> pidx;  // pair -> index in first-appearance order
-    std::vector<int2> plist;
-    std::vector<int> qlist;
-    std::map<int, int> qidx;
-    struct E { int p, q, slot; };
-    std::vector<E> ents;
-    for (int64_t m = 0; m < sh.itot; m++) {
-        const int l = sh.tri[3 * m], j = sh.tri[3 * m + 1], i = sh.tri[3 * m + 2];
-        for (int s = 0; s < nsets; s++) {
-            int pa, pb, qm;
-            if (!cross) { pa = i - 1; pb = j - 1; qm = qoff + s * nb + l - 1; }
-            else { pa = j - 1; pb = l - 1; qm = cross * nb + i - 1; }  // cross = set index of the q field
-            auto pk = std::make_pair(pb, pa);
-            auto it = pidx.find(pk);
-            int p;
-            if (it == pidx.end()) { p = (int)plist.size(); pidx[pk] = p; plist.push_back(make_int2(pa, pb)); }
-            else p = it->second;
-            qidx[qm] = 0;
-            ents.push_back({p, qm, (int)(m * nsets + s)});
-        }
-    }
-    // q order: sorted map index
-    for (auto &kv : qidx) { kv.second = (int)qlist.size(); qlist.push_back(kv.first); }
-    for (auto &e : ents) e.q = qidx[e.q];
-    np = (int)plist.size();
-    nq = (int)qlist.size();
-    nslots = (int)(sh.itot * nsets);
-    // tiles
-    std::map<std::pair<int, int>, int> tidx;
-    std::vector<int4> tl;
-    std::vector<int> stab;
-    for (auto &e : ents) {
-        auto key = std::make_pair(e.p / kTP, e.q / kTQ);
-        auto it = tidx.find(key);
-        int t;
-        if (it == tidx.end()) {
-            t = (int)tl.size();
-            tidx[key] = t;
-            tl.push_back(make_int4(key.first * kTP, key.second * kTQ, 0, t * kTP * kTQ));
-            stab.resize(stab.size() + kTP * kTQ, -1);
-        } else t = it->second;
-        stab[(size_t)t * kTP * kTQ + (e.p % kTP) * kTQ + (e.q % kTQ)] = e.slot;
-    }
-    // Pair blocks of <= max_pairs consecutive pairs; inside a block tiles are
-    // ordered (q tile, pair tile) so the threads of a warp share a q tile.
-    // Groups are runs of <= kGroupThreads tiles of one block.
-    std::vector<int> order(tl.size());
-    for (size_t k = 0; k < order.size(); k++) order[k] = (int)k;
-    const int pblk = std::max(kTP, (max_pairs / kTP) * kTP);
-    std::sort(order.begin(), order.end(), [&](int a, int b) {
-        const int ba = tl[a].x / pblk, bb = tl[b].x / pblk;
-        if (ba != bb) return ba < bb;
-        return tl[a].y != tl[b].y ? tl[a].y < tl[b].y : tl[a].x < tl[b].x;
-    });
-    std::vector<int4> tiles_sorted;
-    std::vector<int> stab_sorted;
-    std::vector<int4> gl;
-    size_t k = 0;
-    while (k < order.size()) {
-        const int blk = tl[order[k]].x / pblk;
-        size_t e = k;
-        while (e < order.size() && tl[order[e]].x / pblk == blk) e++;
-        for (size_t g0 = k; g0 < e; g0 += kGroupThreads) {
-            const size_t g1 = std::min(e, g0 + (size_t)kGroupThreads);
-            int pmin = 1 << 30, pmax = 0;
-            for (size_t u = g0; u < g1; u++) {
-                pmin = std::min(pmin, tl[order[u]].x);
-                pmax = std::max(pmax, tl[order[u]].x + kTP);
-            }
-            const int t0 = (int)tiles_sorted.size();
-            for (size_t u = g0; u < g1; u++) {
-                int4 t = tl[order[u]];
-                const int ns = (int)tiles_sorted.size();
-                stab_sorted.insert(stab_sorted.end(), stab.begin() + (size_t)t.w,
-                                   stab.begin() + (size_t)t.w + kTP * kTQ);
-                t.z = (int)gl.size();
-                t.w = ns * kTP * kTQ;
-                tiles_sorted.push_back(t);
-            }
-            gl.push_back(make_int4(t0, (int)tiles_sorted.size(), pmin, pmax));
-        }
-        k = e;
-    }
-    ntiles = (int)tiles_sorted.size();
-    ngroups = (int)gl.size();
-    max_group_pairs = 0;
-    for (auto &g : gl) max_group_pairs = std::max(max_group_pairs, g.w - g.z);
-    // pad pair list to a multiple of kTP with a harmless pair (0,0)
-    while ((int)plist.size() % kTP) plist.push_back(make_int2(0, 0));
-    while ((int)qlist.size() % kTQ) qlist.push_back(qlist.empty() ? 0 : qlist[0]);
-    PBI4G_CHECK(pairs.ensure(sizeof(int2) * plist.size()));
-    PBI4G_CUDA(cudaMemcpy(pairs.p, plist.data(), sizeof(int2) * plist.size(), cudaMemcpyHostToDevice));
-    PBI4G_CHECK(qmap.ensure(sizeof(int) * qlist.size()));
-    PBI4G_CUDA(cudaMemcpy(qmap.p, qlist.data(), sizeof(int) * qlist.size(), cudaMemcpyHostToDevice));
-    PBI4G_CHECK(tiles.ensure(sizeof(int4) * std::max<size_t>(1, tiles_sorted.size())));
-    PBI4G_CUDA(cudaMemcpy(tiles.p, tiles_sorted.data(), sizeof(int4) * tiles_sorted.size(), cudaMemcpyHostToDevice));
-    PBI4G_CHECK(slots.ensure(sizeof(int) * std::max<size_t>(1, stab_sorted.size())));
-    PBI4G_CUDA(cudaMemcpy(slots.p, stab_sorted.data(), sizeof(int) * stab_sorted.size(), cudaMemcpyHostToDevice));
-    PBI4G_CHECK(groups.ensure(sizeof(int4) * std::max<size_t>(1, gl.size())));
-    PBI4G_CUDA(cudaMemcpy(groups.p, gl.data(), sizeof(int4) * gl.size(), cudaMemcpyHostToDevice));
     return PBI4G_OK;
 }
 
@@ -353,188 +238,6 @@ int build_indicator_spectra(const Shells &sh, int m0, int count, typename Cx<R>:
 }
 template int build_indicator_spectra<float>(const Shells &, int, int, float2 *, cudaStream_t, int64_t *);
 template int build_indicator_spectra<double>(const Shells &, int, int, double2 *, cudaStream_t, int64_t *);
-
-// ------------------------------------------------------ triangle sums ---
-// CUDA-core form (FP32 plain / FP64).  Each CTA owns a group of register
-// tiles (kTP pairs x kTQ q maps per thread) and a contiguous range of the
-// contraction (grid points).  Per chunk of kc points inside one grid row the
-// CTA stages the q maps and the pair-source maps in shared memory (k
-// contiguous), forms the pair products, then every thread runs its tile.
-// FP32 chunk sums are folded into Kahan-compensated running sums.
-template <class T> struct VecOf;
-template <> struct VecOf<float> { static constexpr int W = 4; using V = float4; using V2 = float2; };
-template <> struct VecOf<double> { static constexpr int W = 2; using V = double2; using V2 = double2; };
-
-template <class T> __device__ __forceinline__ void vload(const T *p, T v[VecOf<T>::W]);
-template <> __device__ __forceinline__ void vload<float>(const float *p, float v[4]) {
-    const float4 a = *reinterpret_cast<const float4 *>(p);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-}
-template <> __device__ __forceinline__ void vload<double>(const double *p, double v[2]) {
-    const double2 a = *reinterpret_cast<const double2 *>(p);
-    v[0] = a.x; v[1] = a.y;
-}
-
-// Accumulation of one chunk into the running sum: Kahan-compensated for FP32.
-template <class T> struct Runner {
-    T sum = 0, comp = 0;
-    __device__ __forceinline__ void add(T v) {
-        T y = v - comp;
-        T t = sum + y;
-        comp = (t - sum) - y;
-        sum = t;
-    }
-};
-template <> struct Runner<double> {
-    double sum = 0, comp = 0;
-    __device__ __forceinline__ void add(double v) { sum += v; }
-};
-
-constexpr int kKCmax = 64;
-
-// Shared layout (k-major, the tile index contiguous): sQ[k][q], sP[k][p], so a
-// warp whose threads share one q tile reads it by broadcast and reads its
-// consecutive pair tiles as one contiguous 512-byte row segment.
-template <class T>
-__global__ void __launch_bounds__(kGroupThreads) trisum_kernel(
-    int N, int kc, const T *__restrict__ maps, size_t mstride, int rs, int nb, int nq, const int *__restrict__ qmap,
-    const int2 *__restrict__ pairs, const int4 *__restrict__ tiles, const int4 *__restrict__ groups,
-    const int *__restrict__ slots, int ngroups, int ksplit, long long K, int nslots, double *__restrict__ partial,
-    int qrow, int prow) {
-    using V2 = typename VecOf<T>::V2;
-    constexpr int ARS = kKCmax + (sizeof(T) == 4 ? 4 : 2);  // sA row stride (k contiguous)
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int g = blockIdx.x % ngroups, split = blockIdx.x / ngroups;
-    const int4 G = groups[g];
-    const int ntile = G.y - G.x, p0g = G.z, npg = G.w - G.z;
-    T *sQ = reinterpret_cast<T *>(smem_raw);  // [kKCmax][qrow]
-    T *sP = sQ + (size_t)kKCmax * qrow;       // [kKCmax][prow]
-    T *sA = sP + (size_t)kKCmax * prow;       // [nb][ARS]
-    const int my = threadIdx.x;
-    int4 tile = make_int4(0, 0, 0, 0);
-    if (my < ntile) tile = tiles[G.x + my];
-    const int tp = tile.x - p0g, tq = tile.y;
-
-    const long long nchunks = K / kc;
-    const long long cb = nchunks * split / ksplit, ce = nchunks * (split + 1) / ksplit;
-
-    T acc[kTP][kTQ];
-    Runner<T> run[kTP][kTQ];
-#pragma unroll
-    for (int a = 0; a < kTP; a++)
-#pragma unroll
-        for (int b = 0; b < kTQ; b++) acc[a][b] = 0;
-
-    const int hv = kc / 2;  // vec2 loads per staged row
-    for (long long ch = cb; ch < ce; ch++) {
-        const long long k0 = ch * kc;
-        for (int idx = threadIdx.x; idx < (nq + nb) * hv; idx += blockDim.x) {
-            const int m = idx / hv, c = idx - m * hv;
-            const int map = m < nq ? qmap[m] : m - nq;
-            // N is even, so a pair of points never straddles a grid row
-            const long long p = k0 + 2 * c;
-            const V2 v = *reinterpret_cast<const V2 *>(maps + (size_t)map * mstride + (size_t)(p / N) * rs +
-                                                       (size_t)(p % N));
-            if (m < nq) {
-                sQ[(size_t)(2 * c) * qrow + m] = v.x;
-                sQ[(size_t)(2 * c + 1) * qrow + m] = v.y;
-            } else {
-                T *dst = sA + (size_t)(m - nq) * ARS + 2 * c;
-                dst[0] = v.x;
-                dst[1] = v.y;
-            }
-        }
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < npg * kc; idx += blockDim.x) {
-            const int pp = idx % npg, k = idx / npg;
-            const int2 pr = pairs[p0g + pp];
-            sP[(size_t)k * prow + pp] = sA[(size_t)pr.x * ARS + k] * sA[(size_t)pr.y * ARS + k];
-        }
-        __syncthreads();
-        if (my < ntile) {
-#pragma unroll 4
-            for (int kk = 0; kk < kc; kk++) {
-                T av[kTP], qv[kTQ];
-                vload<T>(sP + (size_t)kk * prow + tp, av);
-                if (VecOf<T>::W == 2) vload<T>(sP + (size_t)kk * prow + tp + 2, av + 2);
-#pragma unroll
-                for (int b = 0; b < kTQ; b += VecOf<T>::W) vload<T>(sQ + (size_t)kk * qrow + tq + b, qv + b);
-#pragma unroll
-                for (int a = 0; a < kTP; a++)
-#pragma unroll
-                    for (int b = 0; b < kTQ; b++) acc[a][b] = fma(av[a], qv[b], acc[a][b]);
-            }
-#pragma unroll
-            for (int a = 0; a < kTP; a++)
-#pragma unroll
-                for (int b = 0; b < kTQ; b++) {
-                    run[a][b].add(acc[a][b]);
-                    acc[a][b] = 0;
-                }
-        }
-        __syncthreads();
-    }
-    if (my < ntile) {
-        const int *st = slots + tile.w;
-#pragma unroll
-        for (int a = 0; a < kTP; a++)
-#pragma unroll
-            for (int b = 0; b < kTQ; b++) {
-                const int s = st[a * kTQ + b];
-                if (s >= 0) partial[(size_t)split * nslots + s] = (double)run[a][b].sum - (double)run[a][b].comp;
-            }
-    }
-}
-
-__global__ void reduce_partial_kernel(int nslots, int ksplit, const double *__restrict__ partial,
-                                      double *__restrict__ S, int accumulate) {
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nslots; s += gridDim.x * blockDim.x) {
-        double v = 0;
-        for (int k = 0; k < ksplit; k++) v += partial[(size_t)k * nslots + s];
-        S[s] = accumulate ? S[s] + v : v;
-    }
-}
-
-int reduce_partials(int nslots, int ksplit, const double *partial, double *S, bool accumulate, cudaStream_t st) {
-    reduce_partial_kernel<<<(nslots + 255) / 256, 256, 0, st>>>(nslots, ksplit, partial, S, accumulate ? 1 : 0);
-    PBI4G_LAUNCH_CHECK();
-    return PBI4G_OK;
-}
-
-template <class T>
-int triangle_sums(const Shells &sh, const TriPlan &tp, const T *maps, size_t mstride, int rowlen, int rs,
-                  long long K, DevBuf &partial, double *S, bool accumulate, cudaStream_t st, int64_t *launches) {
-    const int N = rowlen;
-    int kc = kKCmax;
-    while (kc > 4 && K % kc) kc /= 2;
-    if (K < 1 || K % kc || (N & 1) || (rs & 1) || (mstride & 1))
-        return set_error(PBI4G_ERR_UNSUPPORTED, "triangle sums: %lld points in rows of %d have no even chunk width",
-                         K, N);
-    const int qpad = ((tp.nq + kTQ - 1) / kTQ) * kTQ;  // q tiles read up to 8 columns per tile
-    const int gpad = ((tp.max_group_pairs + kTP - 1) / kTP) * kTP;
-    const int qrow = qpad + 4, prow = gpad + 4;          // 16-B aligned rows, staggered banks
-    const int ARS = kKCmax + (sizeof(T) == 4 ? 4 : 2);
-    const size_t smem = sizeof(T) * ((size_t)kKCmax * (qrow + prow) + (size_t)sh.nb * ARS);
-    if (smem > 220 * 1024) return set_error(PBI4G_ERR_UNSUPPORTED, "triangle sums: %zu B shared memory", smem);
-    const int target = 152 * 2;
-    int ksplit = std::max(1, target / std::max(1, tp.ngroups));
-    ksplit = (int)std::min<long long>(ksplit, std::max<long long>(1, K / kc / 8));
-    PBI4G_CHECK(partial.ensure(sizeof(double) * (size_t)ksplit * tp.nslots));
-    auto kern = trisum_kernel<T>;
-    PBI4G_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<tp.ngroups * ksplit, kGroupThreads, smem, st>>>(
-        N, kc, maps, mstride, rs, sh.nb, qpad, tp.qmap.as<int>(), tp.pairs.as<int2>(), tp.tiles.as<int4>(),
-        tp.groups.as<int4>(), tp.slots.as<int>(), tp.ngroups, ksplit, K, tp.nslots, partial.as<double>(), qrow, prow);
-    PBI4G_LAUNCH_CHECK();
-    PBI4G_CHECK(reduce_partials(tp.nslots, ksplit, partial.as<double>(), S, accumulate, st));
-    *launches += 2;
-    return PBI4G_OK;
-}
-
-template int triangle_sums<float>(const Shells &, const TriPlan &, const float *, size_t, int, int, long long,
-                                  DevBuf &, double *, bool, cudaStream_t, int64_t *);
-template int triangle_sums<double>(const Shells &, const TriPlan &, const double *, size_t, int, int, long long,
-                                   DevBuf &, double *, bool, cudaStream_t, int64_t *);
 
 // ------------------------------------------------------------ outputs ---
 __global__ void bk_finalize_kernel(int64_t itot, int nb, int nsets, int cross, const int *__restrict__ tri,
@@ -735,7 +438,7 @@ int triangle_counts(Shells &sh, cudaStream_t st, int64_t *launches) {
     // enumeration, bispectrumI4.f90:887-896), so the non-cross pair layout
     // applies: pairs from the plain copies [0, nb), q from the weighted copies
     TriPlan tp;
-    PBI4G_CHECK(tp.build(sh, 1, 0, 128, nb));
+    PBI4G_CHECK(tp.build(sh, 1, 0, true, nb));
     PBI4G_CHECK(S.ensure(sizeof(double) * tp.nslots));
     PBI4G_CHECK(triangle_sums<double>(sh, tp, rep.as<double>(), (size_t)npad, 64, 64, npad, partial, S.as<double>(),
                                       false, st, launches));

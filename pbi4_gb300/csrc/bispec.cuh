@@ -35,23 +35,23 @@ struct Shells {
 int map_grid_for_kmax(int N, int kmax);
 int shell_map_grid(int N, float kbin, float kcenter, int nb);
 
-// Sparse "pair x q" contraction S[slot] = sum_x P_a(x) P_b(x) Q(x) arranged as
-// register tiles; built once per (shells, number of q sets).
+// Sparse contraction S[slot] = sum_x M_f(x) M_g(x) Q(x) on CUDA cores arranged as
+// register tiles (trisum_simt.cu): a tile holds tf consecutive factor maps f, tg
+// consecutive maps g and tq consecutive shells q of every q set.  Built once per (shells,
+// number of q sets, type).
 struct TriPlan {
     int nsets = 1;       // q sets (1: B0; 3: B0, B2, B4; cross: 1 with q from the second field)
-    int cross = 0;
-    int np = 0, nq = 0;  // pairs, q maps
+    int fp64 = 0, tf = 0, tg = 0, tq = 0, max_warps = 0;  // the kernel's tile shape and CTA size
+    int setrows = 0;     // map rows between the q sets
+    int nrows = 0;       // maps staged: [0, nrows)
     int nslots = 0;      // itot * nsets
-    int ngroups = 0;
-    DevBuf pairs;        // int2 [np]: source maps of each pair (within the pair set)
-    DevBuf qmap;         // int [nq]: map index of each q (within all maps)
-    DevBuf tiles;        // int4 [ntiles]: (pair0, q0, group, slot table offset)
-    DevBuf slots;        // int [ntiles][TP][TQ]: output slot or -1
-    DevBuf groups;       // int4 [ngroups]: (tile0, tile1, pair0, pair1)
-    std::vector<int> group_tiles;
-    int ntiles = 0, max_group_pairs = 0;
+    int ntiles = 0, ngroups = 0, group_warps = 0;  // tiles; tile groups, of at most group_warps warps of tiles
+    DevBuf tiles;        // int4 [ntiles]: (first f, first g, first q of set 0, unused)
+    DevBuf slots;        // int [ntiles][nsets][tq][tf][tg]: output slot or -1
+    DevBuf groups;       // int2 [ngroups]: tiles [x, y)
+    DevBuf run;          // FP64 running sums of the FP32 form, one column per thread
     // qoff: added to the map index of every non-cross q (a second copy of the maps)
-    int build(const Shells &sh, int nsets, int cross, int max_pairs = 256, int qoff = 0);
+    int build(const Shells &sh, int nsets, int cross, bool fp64, int qoff = 0);
 };
 
 // Build the half spectra of all `count` maps on the map grid Nm into `out`
@@ -71,14 +71,18 @@ template <class R>
 int build_indicator_spectra(const Shells &sh, int m0, int count, typename Cx<R>::T *out, cudaStream_t st,
                             int64_t *launches);
 
-// Triangle sums on CUDA cores: S[slot] for all slots of tp over K points,
-// maps FP32/FP64 laid out as rows of `rowlen` points with row stride rs
-// (rowlen + 2 for padded C2R output).  maps: base of all maps, map m at
-// maps + m * mstride.  Result S (double, nslots) on device; with accumulate the
-// sums are added to S (a contraction streamed in point ranges).
+// Triangle sums on CUDA cores: S[slot] for all slots of tp over K points, maps
+// FP32/FP64 laid out as rows of `rowlen` points with row stride rs (rowlen + 2 for
+// padded C2R output; FP32 maps have contiguous points, rs = rowlen).  maps: base of
+// all maps, map m at maps + m * mstride.  K, rs and mstride are multiples of 16
+// bytes.  Result S (double, nslots) on device; with accumulate the sums are added
+// to S (a contraction streamed in point ranges).
 template <class T>
-int triangle_sums(const Shells &sh, const TriPlan &tp, const T *maps, size_t mstride, int rowlen, int rs,
-                  long long K, DevBuf &partial, double *S, bool accumulate, cudaStream_t st, int64_t *launches);
+int triangle_sums(const Shells &sh, TriPlan &tp, const T *maps, size_t mstride, int rowlen, int rs, long long K,
+                  DevBuf &partial, double *S, bool accumulate, cudaStream_t st, int64_t *launches);
+
+// S[slot] (+)= the sum of nparts partial results [nparts][nslots], in a fixed order.
+int reduce_partials(int nslots, int nparts, const double *partial, double *S, bool accumulate, cudaStream_t st);
 
 // Output rows of measure_bk (9), measure_bk_multipoles (11), measure_bk_cross (5).
 // With bp the shot-noise factor is read from bp->pow_sn (graph-captured form).

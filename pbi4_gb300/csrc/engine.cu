@@ -106,7 +106,7 @@ int BkEngine::run(const typename Cx<R>::T *const src[3], const int fac[3], const
     const int nm = nmaps();
     const bool fp64 = sizeof(R) == 8;
     if (tp_nsets != nsets || tp_cross != cross || tp_fp64 != (int)fp64) {
-        PBI4G_CHECK(tp.build(sh, cross ? 1 : nsets, cross, fp64 ? 128 : 256));
+        PBI4G_CHECK(tp.build(sh, cross ? 1 : nsets, cross, fp64));
         tp_nsets = nsets;
         tp_cross = cross;
         tp_fp64 = fp64;

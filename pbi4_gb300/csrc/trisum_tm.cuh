@@ -34,8 +34,4 @@ int triangle_sums_tm(const Shells &sh, TmPlan &tp, const MapPlanes &pl, DevBuf &
 // PBI4G_ERR_TIMEOUT if a bounded wait inside the last launch gave up (synchronises st).
 int tm_check_error(TmPlan &tp, cudaStream_t st);
 
-// deterministic reduction of [ksplit][nslots] partial sums into S (added to S
-// with accumulate) (bispec.cu)
-int reduce_partials(int nslots, int ksplit, const double *partial, double *S, bool accumulate, cudaStream_t st);
-
 }  // namespace pbi4g
