@@ -14,16 +14,17 @@
 //
 // What bounds it: HBM, once the FP64 pipe is kept out (0.5 TFMA/s here: the chain
 // product, division, product, sum of one float32 component, its division by hz alone ten
-// FP64 operations, took 1.27 ms for 10^7 particles against 71 us of traffic).
+// FP64 operations, took 1.27 ms for 10^7 particles against 71 us of traffic; this form takes 103 us).
 //  * A line-of-sight component that is zero shifts by an exact zero: no arithmetic.
 //  * float32: the shifted position is formed in float32 pairs (shift_f32), whose error is
 //    far below half an ulp of the rounded result; only where it could decide the rounding
 //    does the lane run the reference's FP64 operations.
-//  * float64: divisions by hz and box as products with their reciprocals and residual
-//    corrections (div_by), 5 FP64 operations.
+//  * divisions by hz and box as products with their reciprocals and residual corrections
+//    (div_by): 5 operations, in float64 on the slow pipe.
 //  * the wrap of a value in [0, 2 box) is at most one exact subtraction, not an fmod.
-// Loads run over the catalogue as it lies (any alignment), and the three rows of a tile
-// are put together in shared memory, so both sides are coalesced.
+// Loads run over the catalogue as it lies (any alignment) into shared memory, a thread then
+// takes whole particles: both sides are coalesced, and the branch on a zero component is
+// uniform.
 #include <float.h>
 #include <math.h>
 
@@ -35,13 +36,13 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kTile = 512;                       // particles per tile
-constexpr int kPer = 3 * kTile / kThreads;       // components per thread
-constexpr int kRow = kTile + 5;                  // shared row: a half-warp's components fall on distinct banks
+constexpr int kPer = 3 * kTile / kThreads;       // components a thread loads
 
 struct CatArgs {
     double l[3];         // line of sight
     double hz, opz;      // rsd_mode 1: the shift is vel l / hz (1 + z)
     double rhz, rbox;    // correctly rounded reciprocals; 0: divide
+    float rboxf;         // the same in float32
     float ch[3], cl[3];  // the shift's factor of vel as a float32 pair
     bool zero[3];        // the factor is zero: no shift
     int mode;
@@ -68,6 +69,15 @@ __device__ __forceinline__ double div_by(double a, double b, double r) {
     double q = __dmul_rn(a, r);
     q = __fma_rn(__fma_rn(-q, b, a), r, q);
     return __fma_rn(__fma_rn(-q, b, a), r, q);
+}
+
+// the same in float32, for a = +0 or in [2^-40, 2^40] (the quotients of a wrapped position)
+__device__ __forceinline__ float div_by(float a, float b, float r) {
+    const unsigned u = __float_as_uint(a);
+    if (r == 0.f || (u != 0u && u - ((127u - 40u) << 23) > (80u << 23))) return __fdiv_rn(a, b);
+    float q = __fmul_rn(a, r);
+    q = __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
+    return __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
 }
 
 // the reference's operations: the shift in FP64 (one rounding each, no contraction), the
@@ -104,15 +114,22 @@ __device__ __forceinline__ float shift_f32(float p, float v, const CatArgs &a, i
 
 // float32 -> float64 in integer arithmetic (conversions run at the FP64 pipe's rate)
 __device__ __forceinline__ double widen(float q) {
-    const unsigned u = __float_as_uint(q), ex = (u >> 23) & 255;
-    if (ex == 0 || ex == 255 || (u >> 31)) return (double)q;
-    return __longlong_as_double(((long long)u << 29) + (896LL << 52));
+    const unsigned u = __float_as_uint(q);
+    unsigned m = u & 0x7fffffffu;
+    long long bias = 896;
+    if (m < 0x00800000u) {  // zero or subnormal: scaled into the normal range, exactly
+        m = __float_as_uint(fabsf(q) * 0x1p64f);
+        bias = m ? 896 - 64 : 0;
+    } else if (m >= 0x7f800000u) {  // inf, NaN: exponent 2047
+        bias = 2047 - 255;
+    }
+    return __longlong_as_double(((long long)(u >> 31) << 63) | (((long long)m << 29) + (bias << 52)));
 }
 
 // one component: shift, wrap, scale, clip
 __device__ __forceinline__ double position(float p, float v, bool shift, float box, const CatArgs &a, int d) {
     if (shift && !(pick(a.zero, d) && isfinite(v))) p = shift_f32(p, v, a, d);
-    const float q = __fdiv_rn(remainder_np<float>(__fadd_rn(p, box), box), box);
+    const float q = div_by(remainder_np<float>(__fadd_rn(p, box), box), box, a.rboxf);
     return q < 1.f || isnan(q) ? widen(q) : 1.0;  // np.minimum keeps NaN
 }
 __device__ __forceinline__ double position(double p, double v, bool shift, double box, const CatArgs &a, int d) {
@@ -125,7 +142,7 @@ template <class T>
 __global__ void __launch_bounds__(kThreads) catalog_positions_kernel(int64_t n, const T *__restrict__ pos,
                                                                     const T *__restrict__ vel, const CatArgs a, T box,
                                                                     double *__restrict__ out) {
-    __shared__ double row[3 * kRow];
+    __shared__ T sp[3 * kTile], sv[3 * kTile];
     const int t = threadIdx.x;
     const int64_t ntiles = (n + kTile - 1) / kTile;
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -140,19 +157,26 @@ __global__ void __launch_bounds__(kThreads) catalog_positions_kernel(int64_t n, 
         }
 #pragma unroll
         for (int j = 0; j < kPer; j++) {
-            const int e = t + j * kThreads, i = e / 3, d = e - 3 * i;
-            if (e < ne) row[d * kRow + i] = position(p[j], v[j], vel != nullptr, box, a, d);
+            sp[t + j * kThreads] = p[j];
+            if (vel) sv[t + j * kThreads] = v[j];
         }
         __syncthreads();
 #pragma unroll
-        for (int d = 0; d < 3; d++)
-            for (int i = t; i < np; i += kThreads) __stcs(out + (size_t)d * n + base + i, row[d * kRow + i]);
+        for (int k = 0; k < kTile / kThreads; k++) {
+            const int i = t + k * kThreads;
+            if (i >= np) break;
+#pragma unroll
+            for (int d = 0; d < 3; d++)
+                __stcs(out + (size_t)d * n + base + i,
+                       position(sp[3 * i + d], vel ? sv[3 * i + d] : (T)0, vel != nullptr, box, a, d));
+        }
         __syncthreads();
     }
 }
 
 // 1 / b for div_by, or 0 where b is too near the ends of the exponent range for it
 double reciprocal(double b) { return fabs(b) > 0x1p-300 && fabs(b) < 0x1p300 ? 1.0 / b : 0.0; }
+float reciprocal(float b) { return fabsf(b) > 0x1p-30f && fabsf(b) < 0x1p30f ? 1.0f / b : 0.0f; }
 
 }  // namespace
 
@@ -177,6 +201,7 @@ int pbi4g_catalog_positions(int64_t npart, const void *d_pos, const void *d_vel,
     a.mode = rsd_mode;
     a.rhz = reciprocal(hz);
     a.rbox = reciprocal(box);
+    a.rboxf = reciprocal((float)box);
     for (int d = 0; d < 3; d++) {
         a.l[d] = d_vel ? los[d] : 0;
         // a zero shift: 0 / hz (1 + z) is a zero for finite hz and 1 + z
