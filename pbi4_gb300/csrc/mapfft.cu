@@ -290,12 +290,12 @@ __device__ __forceinline__ void store_floats(float *dst, const float2 (&v)[P]) {
 
 // The x pass's operand-plane stores of one tile of map m: lane = W consecutive
 // points of a row (the z values z[j] .. z[j + W/2 - 1] of row l), written as one
-// W-element store per plane at ((chunk maps + m) 64 + point % 64).
+// W-element store per plane at ((chunk maps + row of m) 64 + point % 64).
 template <int W>
 __device__ __forceinline__ void store_planes(const XArgs &a, const float2 *buf, int m, int nrows, int npt, size_t c0,
                                              float sb, float sa, int warp, int nw, int lane) {
     constexpr int P = W / 2;
-    const int Nm = a.Nm;
+    const int Nm = a.Nm, prow = a.info[m].prow;
     for (int pl = 32 * W * warp + W * lane; pl < npt; pl += 32 * W * nw) {
         int l = (int)(((float)pl + 0.5f) * a.inv_nm);
         l -= l * Nm > pl ? 1 : 0;
@@ -308,7 +308,7 @@ __device__ __forceinline__ void store_planes(const XArgs &a, const float2 *buf, 
             v[i] = fftd::cscale(z[i], sb);
         }
         const size_t ck = c0 + (pl >> 6), t = pl & 63;
-        const size_t ib = (ck * a.count + m) * 64 + t;  // element index in the B planes
+        const size_t ib = (ck * a.count + prow) * 64 + t;  // element index in the B planes
         if (a.oform == 1) {
             unsigned hw[P], lw[P];
 #pragma unroll
@@ -522,6 +522,7 @@ int MapTransform::build(const Shells &s, int nm) {
         const int b = m % nb;
         MapInfo &mi = info_h[m];
         mi.shell = b;
+        mi.prow = MapPlanes::row_of(m, nm, nb);
         mi.kxn = kxn[b];
         mi.ncol = ncol[b];
         mi.col0 = col0[b];

@@ -21,6 +21,7 @@ namespace pbi4g {
 
 struct MapInfo {
     int shell;        // 0-based shell of the map (map m: set m / nb, shell m % nb)
+    int prow;         // its row in the operand planes (MapPlanes::row_of)
     int kxn;          // columns kx < kxn hold modes of the shell
     int ncol;         // (kx, ky) columns of the z pass
     int col0;         // first column of the shell in MapTransform::cols
@@ -35,8 +36,10 @@ struct MapInfo {
 // tensor-core forms.  Points are grouped in chunks of 64 consecutive points
 // (point = (z Nm + y) Nm + x, counted from the first point of the z-slab the
 // planes hold; the slab's point count is a multiple of 64), and every array is
-// chunk-major, [chunk][map][64 points], so the operand tile of a chunk (64 maps
-// x 64 points) is one contiguous block:
+// chunk-major, [chunk][row][64 points], so the operand tile of a chunk (up to 64
+// rows x 64 points) is one contiguous block.  Row of map m (set m / nb, shell
+// m % nb): shell-major, row = (m % nb) sets + m / nb, so that the maps of a range of
+// shells are consecutive rows in every set:
 //   form 1 (FP16 hi+lo): bhi, blo FP16 with v 2^mexp[m] = hi + lo (|v 2^mexp| <= 2^14);
 //   form 2 (BF16):       bhi BF16 of v;
 //   form 0 (TF32 hi+lo): bhi FP32 = v with the 13 low mantissa bits cleared, blo = v - bhi;
@@ -51,6 +54,7 @@ struct MapPlanes {
     void *bhi = nullptr, *blo = nullptr;
     float *a32 = nullptr;
     const int *mexp = nullptr;
+    static __host__ __device__ int row_of(int m, int nmaps, int nb) { return (m % nb) * (nmaps / nb) + m / nb; }
     static size_t bytes(int form, long long npts, int nmaps, int nb) {
         const size_t b = form == 0 ? 8 : (form == 1 ? 4 : 2);  // B bytes per point and map
         return b * (size_t)npts * nmaps + 4 * (size_t)npts * nb;

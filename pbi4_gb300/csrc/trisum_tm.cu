@@ -5,8 +5,16 @@
 // B2/B4 sums with the delta_2 / delta_4 maps of shell l), recast as a
 // contraction over the grid points x:
 //     C[p, q] = sum_x A[p, x] B[q, x],  A[p, x] = M_i(x) M_j(x) for the pair p = (i, j),
-//                                       B[q, x] = map q (maps in set-major, shell-minor order).
+//                                       B[q, x] = map q (plane rows: shell-major, set-minor).
 // Only the (p, q) entries that are triangles are kept.
+//
+// Which pairs: a chunk costs a unit (128 pairs x a window of plane rows) about the same
+// whatever it holds, so the plan makes few units.  With one q set the three factors of a
+// triangle are alike and any of its pairs may be the A row: 489 pairs meet the triangles of
+// 48 shells, where the pairs i <= j are 1176 (4 units instead of 10: 5.1 ms against 14.0 ms
+// at 300^3 points).  With three sets the pairs are sorted so that a tile's triangles lie in
+// a short range of shells, and a unit takes a window of 16 to 64 rows of it (40 shells: 9
+// units instead of 14, 7.3 ms against 12.2 ms at 256^3 points).
 //
 // Operand forms (FP32 accumulation in every form):
 //   TF32 split: hi = v with the 13 low mantissa bits cleared (exact in TF32),
@@ -18,29 +26,35 @@
 //     fp16(v), lo = fp16(v - hi); the same three products with kind::f16 (K = 16).
 //   BF16: one bf16 product, kind::f16 with bf16 operands (K = 16).
 //
-// Data path per chunk of 64 grid points (one CTA per (M tile of 128 pairs,
-// N tile of 64 maps, K range)):
+// Data path per chunk of 64 grid points (one CTA per (unit, K range)):
 //   * the x pass of the map transform writes the maps as operand planes
-//     [map][point] (FP16 hi / lo, BF16, or TF32 hi / lo) plus the set-0 maps in
+//     [row][point] (FP16 hi / lo, BF16, or TF32 hi / lo) plus the set-0 maps in
 //     FP32 (the pair factors), so the B tiles need no conversion here;
-//   * a TMA warp loads each chunk's B tile(s) (64 maps x 64 points, 128-byte
+//   * a TMA warp loads each chunk's B tiles (the window's rows x 64 points, 128-byte
 //     swizzled: the K-major operand layout itself) and the FP32 set-0 maps of
-//     the chunk into a ring of shared-memory stages;
-//   * three producer warpgroups take the chunks in turn (thread = TMEM lane =
-//     pair row): they form the 64 products of their pair, split them and store
-//     them straight into a tensor-memory A stage with tcgen05.st (the A operand
-//     never touches shared memory);
-//   * an MMA warp issues the MMAs (A in TMEM, B from the stage) into one of
-//     two TMEM accumulators, a fresh one per chunk, and commits them to a
+//     the chunk into a ring of shared-memory stages, one instruction an operand;
+//   * three producer warpgroups take the chunks in turn.  16-bit forms: a thread takes
+//     four pair rows that share a map and 16 points of each (the 16x256b layout of
+//     tcgen05.st), so the shared map is read once for four products: 20 shared loads
+//     for 64 products instead of 32.  It splits the products and stores them straight
+//     into a tensor-memory A stage (the A operand never touches shared memory);
+//   * two MMA warps issue the MMAs (A in TMEM, B from the stage) of alternate chunks
+//     into one of two TMEM accumulators, a fresh one per chunk, and commit them to a
 //     per-chunk completion barrier that frees the A stage, the accumulator and
 //     (with the producers' release) the shared-memory stage.  The tensor core
 //     adds the products of one instruction to the accumulator with truncation,
 //     so keeping each accumulation to one chunk keeps that error near 1e-6;
-//   * two drain warpgroups (32 accumulator columns each) add each chunk's
+//   * two drain warpgroups (half of the unit's columns each) add each chunk's
 //     accumulator into FP32 registers (round to nearest) and fold those into a
 //     Kahan-compensated sum every 16 chunks (kept in the TMEM columns the
 //     accumulators and A stages leave free), then write the final sums (FP64,
 //     scaled back by the FP16 exponents) of the triangle slots.
+//
+// What bounds it: the latency of the hand-offs around a chunk, 0.49 us a unit and chunk
+// (256^3 box, 2 units: 0.81 ms).  Leaving parts out of it took: barriers alone 0.38 ms,
+// with the TMA copies 0.51, with the MMAs too 0.60, with the pair products 0.69, with
+// their TMEM stores 0.81.  Neither more accumulators (their sums then live in L2 or shared
+// memory: 1.25 ms) nor polling waits (0.99 ms) shortened it.
 // Every wait is bounded: a wait that runs out sets an abort flag that ends all
 // roles, records the error for the host, and the CTA waits (bounded) for its
 // own MMAs and copies in flight before it frees its tensor memory.
@@ -52,6 +66,8 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <queue>
+#include <type_traits>
 #include <vector>
 
 #include "bispec.cuh"
@@ -65,7 +81,7 @@ namespace {
 using namespace tcx;
 
 constexpr int kM = 128;          // pairs per unit (MMA M = TMEM lanes)
-constexpr int kN = 64;           // maps per unit (MMA N)
+constexpr int kN = 64;           // plane rows per unit at most (MMA N: 16, 32, 48 or 64)
 constexpr int kKB = 32;          // FP32 values per 128-byte swizzle row (one K block)
 constexpr int kBlocks = 2;       // K blocks per chunk
 constexpr int kKC = kKB * kBlocks;  // grid points per chunk
@@ -77,25 +93,13 @@ constexpr int kMmaWarp = kProdWarps + kDrainWarps;
 constexpr int kMmaWarps = 2;     // MMA issuers, chunks alternating (a thread's MMAs of a chunk stay in order)
 constexpr int kTmaWarp = kMmaWarp + kMmaWarps;
 constexpr int kThreads = (kTmaWarp + 1) * 32;  // 736
-#ifndef PBI4G_TM_FOLD
-#define PBI4G_TM_FOLD 16
-#endif
-constexpr int kFold = PBI4G_TM_FOLD;  // chunks summed in registers before a Kahan fold
-constexpr int kFoldGroup = 8;    // running sums a drain thread folds per batch of loads (one TMEM x8 load)
-// TMEM accumulators (one chunk each) and the FP16 form's A stages (build-time tuning)
-#ifndef PBI4G_TM_ACC
-#define PBI4G_TM_ACC 2
-#endif
-#ifndef PBI4G_TM_F16_ASTAGES
-#define PBI4G_TM_F16_ASTAGES 4
-#endif
-constexpr int kAcc = PBI4G_TM_ACC;
+constexpr int kFold = 16;  // chunks summed in registers before a Kahan fold
+constexpr int kAcc = 2;          // TMEM accumulators (one chunk each)
 constexpr int kDone = 16;        // per-chunk MMA completion barriers (ring)
 constexpr int kMaxAStages = 6;   // producer -> MMA barriers (one per A stage)
 constexpr uint32_t kColAcc = 0;  // kAcc accumulators of kN columns, then the A stages
 constexpr uint32_t kColA = kAcc * kN;
 constexpr uint32_t kTmemCols = 512;
-constexpr uint32_t kBTile = kN * 128;    // one B tile: 64 maps x 128 bytes
 static_assert(kMaxStages <= kDone, "a stage's MMA barrier must not have cycled when the stage is reused");
 constexpr uint32_t kTfMask = 0xFFFFE000u;
 
@@ -109,18 +113,16 @@ template <> struct Form<kFormTF32> {
     static constexpr int kBTiles = 4;  // hi, hi, lo, lo: 32 FP32 points per 128-byte row
     static constexpr int kKStep = 8;
     static constexpr bool kSplit = true;
-    static constexpr uint32_t kIdesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(kN >> 3) << 17) |
-                                       ((uint32_t)(kM >> 4) << 24);
+    static constexpr uint32_t kIdesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(kM >> 4) << 24);  // N to be added (idesc_n)
 };
 // FP16 split: A stage = 32 hi + 32 lo packed columns, 4 K-steps of 16, 3 products
 template <> struct Form<kFormF16> {
     static constexpr uint32_t kACols = kKC;
-    static constexpr int kAStages = PBI4G_TM_F16_ASTAGES;
+    static constexpr int kAStages = 4;
     static constexpr int kBTiles = 2;  // hi, lo: 64 FP16 points per 128-byte row
     static constexpr int kKStep = 16;
     static constexpr bool kSplit = true;
-    static constexpr uint32_t kIdesc = (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(kN >> 3) << 17) |
-                                       ((uint32_t)(kM >> 4) << 24);
+    static constexpr uint32_t kIdesc = (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(kM >> 4) << 24);  // N to be added (idesc_n)
 };
 // BF16: A stage = 32 packed columns, 4 K-steps of 16, 1 product
 template <> struct Form<kFormBF16> {
@@ -129,8 +131,7 @@ template <> struct Form<kFormBF16> {
     static constexpr int kBTiles = 1;
     static constexpr int kKStep = 16;
     static constexpr bool kSplit = false;
-    static constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kN >> 3) << 17) |
-                                       ((uint32_t)(kM >> 4) << 24);
+    static constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kM >> 4) << 24);  // N to be added (idesc_n)
 };
 // A waiter on an mbarrier names the phase by its parity, so each A stage and each
 // accumulator must be consumed by one issuing thread, chunk after chunk: issuer w
@@ -148,22 +149,24 @@ static_assert(Form<kFormTF32>::kAStages % kMmaWarps == 0 && Form<kFormF16>::kASt
 static_assert(kColA + Form<kFormTF32>::kAStages * Form<kFormTF32>::kACols <= kTmemCols, "TMEM budget");
 static_assert(kColA + Form<kFormF16>::kAStages * Form<kFormF16>::kACols <= kTmemCols, "TMEM budget");
 
+__device__ __forceinline__ uint32_t idesc_n(int ncols) { return (uint32_t)(ncols >> 3) << 17; }
+
 // D[tmem] (+)= A[tmem] . B[smem]^T
 template <int F>
-__device__ __forceinline__ void umma_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t b, uint32_t accum) {
+__device__ __forceinline__ void umma_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t b, uint32_t idesc, uint32_t accum) {
     if constexpr (F == kFormTF32)
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "setp.ne.b32 p, %3, 0;\n\t"
             "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %4, p;\n\t}" ::"r"(d_tmem),
-            "r"(a_tmem), "l"(b), "r"(accum), "r"(Form<F>::kIdesc)
+            "r"(a_tmem), "l"(b), "r"(accum), "r"(idesc)
             : "memory");
     else
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "setp.ne.b32 p, %3, 0;\n\t"
             "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %4, p;\n\t}" ::"r"(d_tmem),
-            "r"(a_tmem), "l"(b), "r"(accum), "r"(Form<F>::kIdesc)
+            "r"(a_tmem), "l"(b), "r"(accum), "r"(idesc)
             : "memory");
 }
 
@@ -176,11 +179,12 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
                  : "memory");
 }
 
-__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *tm, int x, int y, int z, uint64_t *bar) {
+// box at (0, row y, 0, chunk z) of a chunk view (make_chunk_view)
+__device__ __forceinline__ void tma_load_chunk(void *dst, const CUtensorMap *tm, int y, int z, uint64_t *bar) {
     asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
-        "[%5];" ::"r"(smem_u32(dst)),
-        "l"(reinterpret_cast<uint64_t>(tm)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %2, "
+        "%4}], [%5];" ::"r"(smem_u32(dst)),
+        "l"(reinterpret_cast<uint64_t>(tm)), "r"(0), "r"(y), "r"(z), "r"(smem_u32(bar))
         : "memory");
 }
 
@@ -259,24 +263,21 @@ __device__ __forceinline__ void pack_prod2(float u0, float v0, float u1, float v
     }
 }
 
-// The drain's Kahan sums live in the TMEM columns the accumulators and A stages
-// leave free when there are 2 kN of them (every form with two accumulators),
-// else in an L2-resident global scratch per CTA.  In TMEM the folds cost no L2
-// round trips: with two accumulators the triangle sums at 256^3 took 1.00 ms
-// against 1.08 ms for four accumulators and the sums in L2 (two A stages instead
-// of four: 1.33 ms).
+// The drain's Kahan sums live in the TMEM columns that two accumulators and the A stages
+// leave free: in an L2 scratch beside four accumulators the folds waited on L2 round trips
+// (1.08 ms against 1.00 ms at 256^3), and halving the A stages instead took 1.33 ms.
 template <int F>
-constexpr bool kahan_in_tmem() {
+constexpr bool kahan_fits() {
     return kColA + (uint32_t)Form<F>::kAStages * Form<F>::kACols + 2 * kN <= kTmemCols;
 }
+static_assert(kahan_fits<kFormTF32>() && kahan_fits<kFormF16>() && kahan_fits<kFormBF16>(), "TMEM budget");
 
 struct TmArgs {
     long long nchunks;     // points / kKC, rounded up
-    int nunits, ksplit, nslots, nA, nstages, nmaps;
-    uint32_t stage_bytes, ablock;
-    float *kahan;          // [grid][2][kN][kM] running sums of each CTA (forms whose sums do not fit in TMEM)
-    const int2 *units;     // (M tile, N tile) per unit
-    const int2 *prow;      // [nunits][kM] staged rows (i, j) of each pair's factors, (-1, -1) for none
+    int nunits, ksplit, nslots, nA, nstages, nmaps, nb;
+    uint32_t stage_bytes, ablock;  // ablock: bytes of one K block of the pair factors (rows padded to 8)
+    const int4 *units;     // (M tile, first plane row, rows, warps of pairs) per unit
+    const int2 *prow;      // [tiles][kM] staged rows (u, v) of each pair's factors, (-1, -1) for none
     const int *slots;      // [nunits][kM][kN] output slot or -1
     const int *mexp;       // FP16 form: per-map exponent e, map stored times 2^e (|M| 2^e <= 2^14)
     double *partial;       // [ksplit][nslots]
@@ -284,10 +285,15 @@ struct TmArgs {
     uint32_t wait_limit;   // polls of a main-loop wait (kWaitLimit unless a diagnostic limit is set)
 };
 
+// Tensor maps of one launch: the pair factors, and the B planes (16 bits: hi and lo in bh;
+// TF32: in bh and bl) with boxes of 16, 32, 48 and 64 rows (a unit's window).
+struct TmMaps {
+    CUtensorMap a, bh[4], bl[4];
+};
+
 template <int F, bool D>
 __global__ void __launch_bounds__(kThreads, 1)
-    trisum_tm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmBh,
-                     const __grid_constant__ CUtensorMap tmBl, const TmArgs a) {
+    trisum_tm_kernel(const __grid_constant__ TmMaps tm, const TmArgs a) {
     using FM = Form<F>;
     constexpr int AST = FM::kAStages;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -306,32 +312,29 @@ __global__ void __launch_bounds__(kThreads, 1)
     int2 *prow_s = reinterpret_cast<int2 *>(tmem_slot + 4);
     int *qexp_s = reinterpret_cast<int *>(prow_s + kM);  // [kN] FP16 exponent of each B row
     // running sums of the drain, then the compensation: TMEM columns kColK .. kColK + 2 kN
-    // of the thread's lane, or [kN][kM] floats each in a global scratch per CTA (each
-    // thread reads back only what it wrote)
-    constexpr bool KT = kahan_in_tmem<F>();
+    // of the thread's lane
     constexpr uint32_t kColK = kColA + (uint32_t)AST * FM::kACols;
-    float *run_g = KT ? nullptr : a.kahan + (size_t)blockIdx.x * 2 * kN * kM;
-    float *comp_g = KT ? nullptr : run_g + kN * kM;
 
     const int unit = blockIdx.x % a.nunits, split = blockIdx.x / a.nunits;
-    const int2 U = a.units[unit];
+    const int4 U = a.units[unit];
+    const int q0 = U.y, ncols = U.z, nwp = U.w;  // nwp: warps (quadrants of 32 TMEM lanes) that hold pairs
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const long long cb = a.nchunks * split / a.ksplit, ce = a.nchunks * (split + 1) / a.ksplit;
     const int n = (int)(ce - cb);
 
-    for (int r = tid; r < kM; r += kThreads) prow_s[r] = a.prow[(size_t)unit * kM + r];
+    for (int r = tid; r < kM; r += kThreads) prow_s[r] = a.prow[(size_t)U.x * kM + r];
     for (int r = tid; r < kN; r += kThreads) {
-        const int q = U.y * kN + r;
-        qexp_s[r] = (F == kFormF16 && q < a.nmaps) ? a.mexp[q] : 0;
+        const int q = q0 + r, ns = a.nmaps / a.nb;  // plane row -> map
+        qexp_s[r] = (F == kFormF16 && q < a.nmaps) ? a.mexp[(q % ns) * a.nb + q / ns] : 0;
     }
     if (tid == 0) {
         for (int s = 0; s < kMaxStages; s++) {
             mbar_init(&full[s], 1);
-            mbar_init(&sfree[s], 128);  // the warpgroup that consumed the stage's pair factors
+            mbar_init(&sfree[s], nwp);  // the warpgroup's warps that consumed the stage's pair factors
         }
-        for (int s = 0; s < kMaxAStages; s++) mbar_init(&prod[s], 128);  // one warpgroup per chunk
+        for (int s = 0; s < kMaxAStages; s++) mbar_init(&prod[s], nwp);  // one warpgroup per chunk
         for (int s = 0; s < kDone; s++) mbar_init(&done[s], 1);
-        for (int s = 0; s < kAcc; s++) mbar_init(&accfree[s], kDrainWarps * 32);
+        for (int s = 0; s < kAcc; s++) mbar_init(&accfree[s], kDrainWarps / 4 * nwp);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -344,7 +347,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    // stage: pair-factor blocks [kBlocks][ablock] (FP32, 32 points a row) | B tiles [kBTiles][kBTile]
+    // stage: pair-factor blocks [kBlocks][ablock] (FP32, 32 points a row) | B tiles [kBTiles][rows 128]
     auto stage_ptr = [&](int s) { return base + (size_t)s * a.stage_bytes; };
     auto fail = [&]() {
         *abort_flag = 1;
@@ -353,12 +356,23 @@ __global__ void __launch_bounds__(kThreads, 1)
 
     if (warp < kProdWarps) {
         // ------------------------------------------------------------ producers
+        // (the TMEM rows of quadrants without pairs are never written: their products
+        // stay in rows that no slot reads)
         const int quad = warp & 3, grp = warp >> 2;
-        const int row = quad * 32 + lane;
-        const int2 pr = prow_s[row];
         const uint32_t lane_addr = tmem + ((uint32_t)(quad * 32) << 16);
+        // TF32: thread = row; 16-bit forms: thread = 4 rows (lane / 4 + 8 k) that share the
+        // map v, and 4 points of each 16 (lane % 4)
+        const int row = quad * 32 + (F == kFormTF32 ? lane : lane >> 2);
+        const int2 pr = prow_s[row];
+        uint32_t uo[4], vo = 0;  // byte offsets of the thread's first points in a K block
+        if constexpr (F != kFormTF32) {
+            auto off = [&](int r) { return (uint32_t)(r * 128 + (((lane & 3) ^ (r & 7)) << 4)); };
+            vo = off(max(pr.y, 0));
+#pragma unroll
+            for (int k = 0; k < 4; k++) uo[k] = off(max(prow_s[row + 8 * k].x, 0));
+        }
         Ring rs(grp, nst);  // stage and full-barrier phase of chunk i
-        for (int i = grp; i < n; i += kGroups, rs.step(kGroups, nst)) {
+        for (int i = quad < nwp ? grp : n; i < n; i += kGroups, rs.step(kGroups, nst)) {
             const int s = rs.idx, as = i % AST;
             if (!warp_wait<D>(&full[s], (uint32_t)rs.phase, abort_flag, a.wait_limit)) { fail(); break; }
             // the A stage is free once the MMAs of chunk i - AST completed (MMAs complete in order)
@@ -368,17 +382,17 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             const unsigned char *stg = stage_ptr(s);
             const uint32_t acol = kColA + (uint32_t)as * FM::kACols;
-#pragma unroll
+#pragma unroll 1  // (unrolled, its loads do not fit in the registers: spills go to L2 beside 227 KB of shared memory)
             for (int kb = 0; kb < kBlocks; kb++) {
                 const unsigned char *blk = stg + kb * a.ablock;
                 if constexpr (F == kFormTF32) {
 #pragma unroll
-                    for (int q16 = 0; q16 < 2; q16++) {
-                        uint32_t hi[16], lo[16];
+                    for (int q8 = 0; q8 < 4; q8++) {
+                        uint32_t hi[8], lo[8];
                         if (pr.x >= 0) {
 #pragma unroll
-                            for (int c4 = 0; c4 < 4; c4++) {
-                                const int c = 4 * q16 + c4;
+                            for (int c4 = 0; c4 < 2; c4++) {
+                                const int c = 2 * q8 + c4;
                                 const float4 u =
                                     *reinterpret_cast<const float4 *>(blk + pr.x * 128 + ((c ^ (pr.x & 7)) << 4));
                                 const float4 v =
@@ -402,70 +416,68 @@ __global__ void __launch_bounds__(kThreads, 1)
                             }
                         } else {
 #pragma unroll
-                            for (int e = 0; e < 16; e++) hi[e] = lo[e] = 0u;
-                        }
-                        const uint32_t col = acol + (uint32_t)(kb * kKB + 16 * q16);
-                        tmem_st16(lane_addr + col, hi);
-                        tmem_st16(lane_addr + col + kKC, lo);
-                    }
-                } else {
-                    // 32 points -> 16 packed columns (point 2c in the low half of column c), in
-                    // two halves of 16 points (fewer live registers: 23 warps fit in 80 each)
-#pragma unroll
-                    for (int q8 = 0; q8 < 2; q8++) {
-                        uint32_t hi[8], lo[8];
-                        if (pr.x >= 0) {
-#pragma unroll
-                            for (int c4 = 0; c4 < 4; c4++) {
-                                const int c = 4 * q8 + c4;
-                                const float4 u =
-                                    *reinterpret_cast<const float4 *>(blk + pr.x * 128 + ((c ^ (pr.x & 7)) << 4));
-                                const float4 v =
-                                    *reinterpret_cast<const float4 *>(blk + pr.y * 128 + ((c ^ (pr.y & 7)) << 4));
-                                pack_prod2<F>(u.x, v.x, u.y, v.y, hi[2 * c4], lo[2 * c4]);
-                                pack_prod2<F>(u.z, v.z, u.w, v.w, hi[2 * c4 + 1], lo[2 * c4 + 1]);
-                            }
-                        } else {
-#pragma unroll
                             for (int e = 0; e < 8; e++) hi[e] = lo[e] = 0u;
                         }
-                        const uint32_t col = acol + (uint32_t)(kb * (kKB / 2) + 8 * q8);
+                        const uint32_t col = acol + (uint32_t)(kb * kKB + 8 * q8);
                         tmem_st8(lane_addr + col, hi);
-                        if (FM::kSplit) tmem_st8(lane_addr + col + kKC / 2, lo);
+                        tmem_st8(lane_addr + col + kKC, lo);
+                    }
+                } else {
+                    // 32 points -> 16 packed columns (points 2c, 2c + 1 in column c).  Column
+                    // block n holds the points 16 n + 4 t .. of lane % 4 = t in columns
+                    // 8 n + 2 t, 8 n + 2 t + 1: one 16-byte load a row (XOR 64: the next 16
+                    // points under the swizzle), the shared map's loaded once for four rows.
+                    const float4 v0 = *reinterpret_cast<const float4 *>(blk + vo);
+                    const float4 v1 = *reinterpret_cast<const float4 *>(blk + (vo ^ 64));
+                    const uint32_t col = lane_addr + acol + (uint32_t)(kb * (kKB / 2));
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {  // lanes 0-15, 16-31 of the quadrant: rows k = 2 h, 2 h + 1
+                        uint32_t hi[8], lo[8];
+#pragma unroll
+                        for (int k = 0; k < 2; k++) {
+                            const float4 u0 = *reinterpret_cast<const float4 *>(blk + uo[2 * h + k]);
+                            const float4 u1 = *reinterpret_cast<const float4 *>(blk + (uo[2 * h + k] ^ 64));
+                            pack_prod2<F>(u0.x, v0.x, u0.y, v0.y, hi[2 * k], lo[2 * k]);
+                            pack_prod2<F>(u0.z, v0.z, u0.w, v0.w, hi[2 * k + 1], lo[2 * k + 1]);
+                            pack_prod2<F>(u1.x, v1.x, u1.y, v1.y, hi[4 + 2 * k], lo[4 + 2 * k]);
+                            pack_prod2<F>(u1.z, v1.z, u1.w, v1.w, hi[5 + 2 * k], lo[5 + 2 * k]);
+                        }
+                        tmem_st_16x256b_x2(col + ((uint32_t)(16 * h) << 16), hi);
+                        if (FM::kSplit) tmem_st_16x256b_x2(col + ((uint32_t)(16 * h) << 16) + kKC / 2, lo);
                     }
                 }
             }
-            mbar_arrive(&sfree[s]);  // the stage's pair factors are consumed
+            __syncwarp();  // one arrival a warp on each barrier
+            if (lane == 0) mbar_arrive(&sfree[s]);  // the stage's pair factors are consumed
             tmem_wait_st();
             tc_fence_before();
-            mbar_arrive(&prod[as]);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&prod[as]);
         }
     } else if (warp < kMmaWarp) {
         // ---------------------------------------------------------------- drain
         // each chunk's accumulator is added into FP32 registers (round to nearest);
         // every kFold chunks those are folded into a Kahan-compensated sum (in TMEM, or
         // an L2-resident scratch), written out at the end
+        // (the two warpgroups take half of the unit's columns each, in groups of 8)
         const int quad = warp & 3, cgrp = (warp - kProdWarps) >> 2;
-        const int row = quad * 32 + lane, c0 = 32 * cgrp;
+        // NG: groups of 8 columns per warpgroup (a unit of 16 NG columns)
+        auto drain = [&](auto ng) {
+        constexpr int NG = decltype(ng)::value;
+        const int row = quad * 32 + lane, c0 = 8 * NG * cgrp;
         const uint32_t lane_addr = tmem + ((uint32_t)(quad * 32) << 16);
         const uint32_t krun = lane_addr + kColK + (uint32_t)c0, kcomp = krun + kN;
-        float mid[32];
+        float mid[8 * NG];
 #pragma unroll
-        for (int e = 0; e < 32; e++) mid[e] = 0.f;
-        if constexpr (KT) {
+        for (int e = 0; e < 8 * NG; e++) mid[e] = 0.f;
+        {
             const uint32_t z[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
 #pragma unroll
-            for (int h = 0; h < 32; h += 8) {
+            for (int h = 0; h < 8 * NG; h += 8) {
                 tmem_st8(krun + h, z);
                 tmem_st8(kcomp + h, z);
             }
             tmem_wait_st();
-        } else {
-#pragma unroll
-            for (int e = 0; e < 32; e++) {
-                run_g[(c0 + e) * kM + row] = 0.f;
-                comp_g[(c0 + e) * kM + row] = 0.f;
-            }
         }
         bool ok = true;
 #pragma unroll 1
@@ -473,90 +485,70 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int b = i % kAcc;
             if (!warp_wait<D>(&done[i % kDone], ph(i, kDone), abort_flag, a.wait_limit)) { fail(); ok = false; break; }
             tc_fence_after();
+            const uint32_t src = lane_addr + kColAcc + (uint32_t)b * kN + c0;
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                uint32_t ac[16];
-                tmem_ld16(lane_addr + kColAcc + (uint32_t)b * kN + c0 + 16 * h, ac);
+            for (int h = 0; h < NG; h += 2) {
+                uint32_t ac[8], ad[8];
+                tmem_ld8(src + 8 * h, ac);
+                if (h + 1 < NG) tmem_ld8(src + 8 * h + 8, ad);
                 tmem_wait_ld();
 #pragma unroll
-                for (int e = 0; e < 16; e++) mid[16 * h + e] += __uint_as_float(ac[e]);
+                for (int e = 0; e < 8; e++) mid[8 * h + e] += __uint_as_float(ac[e]);
+                if (h + 1 < NG) {
+#pragma unroll
+                    for (int e = 0; e < 8; e++) mid[(8 * h + 8 + e) % (8 * NG)] += __uint_as_float(ad[e]);
+                }
             }
             tc_fence_before();
-            mbar_arrive(&accfree[b]);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&accfree[b]);
             if ((i + 1) % kFold == 0 || i == n - 1) {
-                // each group's loads are issued before its first store, so the fold
-                // costs a few TMEM (or L2) round trips
 #pragma unroll
-                for (int h = 0; h < 32; h += kFoldGroup) {
-                    if constexpr (KT) {
-                        uint32_t rr[kFoldGroup], cc[kFoldGroup];
-                        tmem_ld8(krun + h, rr);
-                        tmem_ld8(kcomp + h, cc);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int e = 0; e < kFoldGroup; e++) {
-                            const float rv = __uint_as_float(rr[e]), y = mid[h + e] - __uint_as_float(cc[e]);
-                            const float t2 = rv + y;
-                            cc[e] = __float_as_uint((t2 - rv) - y);
-                            rr[e] = __float_as_uint(t2);
-                            mid[h + e] = 0.f;
-                        }
-                        tmem_st8(krun + h, rr);
-                        tmem_st8(kcomp + h, cc);
-                    } else {
-                        float rv[kFoldGroup], cv[kFoldGroup];
-#pragma unroll
-                        for (int e = 0; e < kFoldGroup; e++) {
-                            rv[e] = __ldcg(run_g + (c0 + h + e) * kM + row);
-                            cv[e] = __ldcg(comp_g + (c0 + h + e) * kM + row);
-                        }
-#pragma unroll
-                        for (int e = 0; e < kFoldGroup; e++) {
-                            const float y = mid[h + e] - cv[e];
-                            const float t2 = rv[e] + y;
-                            cv[e] = (t2 - rv[e]) - y;
-                            rv[e] = t2;
-                            mid[h + e] = 0.f;
-                        }
-#pragma unroll
-                        for (int e = 0; e < kFoldGroup; e++) {
-                            __stcg(run_g + (c0 + h + e) * kM + row, rv[e]);
-                            __stcg(comp_g + (c0 + h + e) * kM + row, cv[e]);
-                        }
-                    }
-                }
-                if constexpr (KT) tmem_wait_st();  // the next fold reads these columns back
-            }
-        }
-        if (__all_sync(0xffffffffu, ok && !*abort_flag)) {
-            const int *sl = a.slots + ((size_t)unit * kM + row) * kN;
-            const int2 pr = prow_s[row];
-            const int pe = (F == kFormF16 && pr.x >= 0) ? a.mexp[pr.x] + a.mexp[pr.y] - 14 : 0;
-            if constexpr (KT) {
-#pragma unroll 1
-                for (int h = 0; h < 32; h += 8) {
+                for (int h = 0; h < 8 * NG; h += 8) {
                     uint32_t rr[8], cc[8];
                     tmem_ld8(krun + h, rr);
                     tmem_ld8(kcomp + h, cc);
                     tmem_wait_ld();
 #pragma unroll
                     for (int e = 0; e < 8; e++) {
-                        const int slot = sl[c0 + h + e];
-                        if (slot < 0) continue;
-                        const double v = (double)__uint_as_float(rr[e]) - (double)__uint_as_float(cc[e]);
-                        a.partial[(size_t)split * a.nslots + slot] =
-                            F == kFormF16 ? ldexp(v, -(pe + qexp_s[c0 + h + e])) : v;
+                        const float rv = __uint_as_float(rr[e]), y = mid[h + e] - __uint_as_float(cc[e]);
+                        const float t2 = rv + y;
+                        cc[e] = __float_as_uint((t2 - rv) - y);
+                        rr[e] = __float_as_uint(t2);
+                        mid[h + e] = 0.f;
                     }
+                    tmem_st8(krun + h, rr);
+                    tmem_st8(kcomp + h, cc);
                 }
-            } else {
-#pragma unroll 4
-                for (int e = 0; e < 32; e++) {
-                    const int slot = sl[c0 + e];
+                tmem_wait_st();  // the next fold reads these columns back
+            }
+        }
+        if (__all_sync(0xffffffffu, ok && !*abort_flag)) {
+            const int *sl = a.slots + ((size_t)unit * kM + row) * kN;
+            const int2 pr = prow_s[row];
+            const int pe = (F == kFormF16 && pr.x >= 0) ? a.mexp[pr.x] + a.mexp[pr.y] - 14 : 0;
+#pragma unroll 1
+            for (int h = 0; h < 8 * NG; h += 8) {
+                uint32_t rr[8], cc[8];
+                tmem_ld8(krun + h, rr);
+                tmem_ld8(kcomp + h, cc);
+                tmem_wait_ld();
+#pragma unroll
+                for (int e = 0; e < 8; e++) {
+                    const int slot = sl[c0 + h + e];
                     if (slot < 0) continue;
-                    const double v = (double)run_g[(c0 + e) * kM + row] - (double)comp_g[(c0 + e) * kM + row];
-                    a.partial[(size_t)split * a.nslots + slot] = F == kFormF16 ? ldexp(v, -(pe + qexp_s[c0 + e])) : v;
+                    const double v = (double)__uint_as_float(rr[e]) - (double)__uint_as_float(cc[e]);
+                    a.partial[(size_t)split * a.nslots + slot] =
+                        F == kFormF16 ? ldexp(v, -(pe + qexp_s[c0 + h + e])) : v;
                 }
             }
+        }
+        };
+        if (quad < nwp) {
+            if (ncols == 64) drain(std::integral_constant<int, 4>{});
+            else if (ncols == 48) drain(std::integral_constant<int, 3>{});
+            else if (ncols == 32) drain(std::integral_constant<int, 2>{});
+            else drain(std::integral_constant<int, 1>{});
         }
     } else if (warp < kTmaWarp) {
         // ------------------------------------------ MMA issue (one thread per MMA warp)
@@ -567,6 +559,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int mw = warp - kMmaWarp;
             int last_commit = -1;
             bool ok = true;
+            const uint32_t idesc = FM::kIdesc | idesc_n(ncols), btile = (uint32_t)ncols * 128;
             Ring rs(mw, nst);
             for (int i = mw; i < n; i += kMmaWarps, rs.step(kMmaWarps, nst)) {
                 const int b = i % kAcc, as = i % AST, s = rs.idx;
@@ -584,21 +577,21 @@ __global__ void __launch_bounds__(kThreads, 1)
                     uint32_t a_hi, a_lo;
                     if constexpr (F == kFormTF32) {
                         // FP32 rows: K-step of 8 = 32 bytes; tiles hi0, hi1, lo0, lo1
-                        dh = db + (((uint32_t)(kk / 4) * kBTile + (uint32_t)(kk % 4) * 32) >> 4);
-                        dl = dh + ((2 * kBTile) >> 4);
+                        dh = db + (((uint32_t)(kk / 4) * btile + (uint32_t)(kk % 4) * 32) >> 4);
+                        dl = dh + ((2 * btile) >> 4);
                         a_hi = ahi + 8 * kk;
                         a_lo = a_hi + kKC;
                     } else {
                         // 16-bit rows: K-step of 16 = 32 bytes; tiles hi, lo
                         dh = db + (uint32_t)kk * 2;
-                        dl = dh + (kBTile >> 4);
+                        dl = dh + (btile >> 4);
                         a_hi = ahi + 8 * kk;
                         a_lo = a_hi + kKC / 2;
                     }
-                    umma_ta<F>(d, a_hi, dh, kk == 0 ? 0u : 1u);
+                    umma_ta<F>(d, a_hi, dh, idesc, kk == 0 ? 0u : 1u);
                     if (FM::kSplit) {
-                        umma_ta<F>(d, a_hi, dl, 1u);
-                        umma_ta<F>(d, a_lo, dh, 1u);
+                        umma_ta<F>(d, a_hi, dl, idesc, 1u);
+                        umma_ta<F>(d, a_lo, dh, idesc, 1u);
                     }
                 }
                 umma_commit(&done[i % kDone]);
@@ -610,8 +603,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
     } else if (lane == 0) {
         // --------------------------------------------------------- TMA issue (one thread)
-        const uint32_t tx = kBlocks * (uint32_t)a.nA * 128 + FM::kBTiles * kBTile;
-        const int q0 = U.y * kN;
+        const uint32_t tx = kBlocks * a.ablock + FM::kBTiles * (uint32_t)ncols * 128;
+        const CUtensorMap *tmBh = &tm.bh[ncols / 16 - 1], *tmBl = &tm.bl[ncols / 16 - 1];
         int issued = 0;
         bool ok = true;
         Ring rs(0, nst);
@@ -629,18 +622,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             unsigned char *bt = stg + kBlocks * a.ablock;
             mbar_expect_tx(&full[s], tx);
             const int c = (int)(cb + j);  // chunk: 64 consecutive points, one block of every plane
-#pragma unroll
-            for (int kb = 0; kb < kBlocks; kb++) tma_load_3d(stg + kb * a.ablock, &tmA, kb * kKB, 0, c, &full[s]);
-            if constexpr (F == kFormTF32) {
-#pragma unroll
-                for (int kb = 0; kb < kBlocks; kb++) {
-                    tma_load_3d(bt + kb * kBTile, &tmBh, kb * kKB, q0, c, &full[s]);
-                    tma_load_3d(bt + (2 + kb) * kBTile, &tmBl, kb * kKB, q0, c, &full[s]);
-                }
-            } else {
-                tma_load_3d(bt, &tmBh, 0, q0, c, &full[s]);
-                if (FM::kSplit) tma_load_3d(bt + kBTile, &tmBl, 0, q0, c, &full[s]);
-            }
+            tma_load_chunk(stg, &tm.a, 0, c, &full[s]);
+            tma_load_chunk(bt, tmBh, q0, c, &full[s]);  // 16 bits: hi, and lo after it
+            if (F == kFormTF32) tma_load_chunk(bt + 2 * ncols * 128, tmBl, q0, c, &full[s]);
             issued = j + 1;
         }
         if (!ok) fail();
@@ -692,21 +676,25 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// 3D view of a chunk-major operand array [nchunks][rows][64 points] (element
-// size esize): box box_pts x box_rows x 1 at (point within the chunk, first
-// row, chunk), 128-byte swizzle (box_pts esize = 128 bytes: the K-major operand
-// layout), zero fill past the last row.
+// 4D view of chunk-major operand arrays [nchunks][rows][64 points] (element size esize): a
+// box is (128 bytes of points, box_rows rows, all `nblk` blocks, one chunk), 128-byte swizzle
+// (the K-major operand layout), one block after the other in shared memory.  The blocks are
+// the 128-byte point blocks of the rows (FP32: two, 128 bytes apart) or the hi and lo planes
+// (16 bits: `blk_stride` bytes apart), so that one instruction loads a whole operand: the
+// issuing thread's loads bounded the chunk loop at four a chunk.  Rows past the last one are
+// filled with zeros.
 int make_chunk_view(CUtensorMap *tm, const void *base, CUtensorMapDataType dt, int esize, long long nchunks,
-                    int rows, int box_pts, int box_rows) {
+                    int rows, int box_rows, int nblk, size_t blk_stride) {
     EncodeTiledFn enc = encode_fn();
     if (!enc) return set_error(PBI4G_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-    if (box_pts * esize != 128 || reinterpret_cast<uintptr_t>(base) % 16)
+    if (reinterpret_cast<uintptr_t>(base) % 16 || blk_stride % 16)
         return set_error(PBI4G_ERR_INVALID, "operand chunk view: alignment");
-    const cuuint64_t gdim[3] = {(cuuint64_t)MapPlanes::kChunk, (cuuint64_t)rows, (cuuint64_t)nchunks};
-    const cuuint64_t gstride[2] = {(cuuint64_t)MapPlanes::kChunk * esize, (cuuint64_t)rows * MapPlanes::kChunk * esize};
-    const cuuint32_t box[3] = {(cuuint32_t)box_pts, (cuuint32_t)box_rows, 1};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    const CUresult r = enc(tm, dt, 3, const_cast<void *>(base), gdim, gstride, box, estr,
+    const size_t row_bytes = (size_t)MapPlanes::kChunk * esize;
+    const cuuint64_t gdim[4] = {(cuuint64_t)(128 / esize), (cuuint64_t)rows, (cuuint64_t)nblk, (cuuint64_t)nchunks};
+    const cuuint64_t gstride[3] = {row_bytes, blk_stride, (cuuint64_t)rows * row_bytes};
+    const cuuint32_t box[4] = {(cuuint32_t)(128 / esize), (cuuint32_t)box_rows, (cuuint32_t)nblk, 1};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    const CUresult r = enc(tm, dt, 4, const_cast<void *>(base), gdim, gstride, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return set_error(PBI4G_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
@@ -716,65 +704,268 @@ int make_chunk_view(CUtensorMap *tm, const void *base, CUtensorMapDataType dt, i
 }  // namespace
 
 // ------------------------------------------------------------- host plan ---
+// Pairs of shells (x <= y) that hold every triangle of an equal-set contraction.  With one q
+// set the three factors of a triangle are alike, so any of its three pairs may be the A row
+// and the third shell the B row: the fewest pairs that meet every triangle are wanted.
+// Splitting the shells at `a` and keeping the pairs inside each part covers every triangle
+// (two of three shells fall in one part); of those, pairs that no triangle needs are left out,
+// the triangles inside a part are covered greedily, and redundant pairs are dropped.  The best
+// `a` is taken: 48 shells need 489 pairs of 1176, 24 need 133 of 300.
+static std::vector<std::pair<int, int>> covering_pairs(const Shells &sh) {
+    const int nb = sh.nb, np = nb * (nb + 1) / 2;
+    const size_t nt = (size_t)sh.itot;
+    auto id = [](int x, int y) { return x <= y ? y * (y + 1) / 2 + x : x * (x + 1) / 2 + y; };
+    std::vector<std::vector<int>> of(np);
+    std::vector<int> edge(3 * nt);
+    for (size_t t = 0; t < nt; t++) {
+        const int l = sh.tri[3 * t] - 1, j = sh.tri[3 * t + 1] - 1, i = sh.tri[3 * t + 2] - 1;
+        int e[3] = {id(i, j), id(i, l), id(j, l)};
+        for (int k = 0; k < 3; k++) {
+            edge[3 * t + k] = e[k];
+            bool seen = false;
+            for (int m = 0; m < k; m++) seen |= e[m] == e[k];
+            if (!seen) of[e[k]].push_back((int)t);
+        }
+    }
+    std::vector<char> best;
+    int nbest = 1 << 30;
+    std::vector<int> by_size(np);
+    for (int e = 0; e < np; e++) by_size[e] = e;
+    std::stable_sort(by_size.begin(), by_size.end(), [&](int x, int y) { return of[x].size() < of[y].size(); });
+    // splits tried: all of [0, 0.6 nb) for few shells, at least three for many (0.6 s at 256)
+    const int amax = std::max(1, (int)(0.6 * nb)),
+              ntry = (int)std::min<long long>(amax, std::max<long long>(3, 400000 / std::max<int64_t>(1, sh.itot)));
+    for (int k = 0; k < ntry; k++) {
+        const int a = ntry == amax ? k : (int)((0.2 + 0.4 * k / std::max(1, ntry - 1)) * nb);
+        std::vector<char> keep(np, 0);
+        std::vector<int> cov(nt, 0), cnt(np, 0);
+        for (size_t t = 0; t < nt; t++) {
+            const int l = sh.tri[3 * t] - 1, j = sh.tri[3 * t + 1] - 1, i = sh.tri[3 * t + 2] - 1;
+            if (i < a && j < a && l >= a) keep[id(i, j)] = 1;  // i <= j <= l: two low, one high
+            if (i < a && j >= a) keep[id(j, l)] = 1;           // one low, two high
+        }
+        for (int e = 0; e < np; e++)
+            if (keep[e])
+                for (int t : of[e]) cov[t]++;
+        // greedy cover of the rest: the pair that meets most uncovered triangles next (counts
+        // only fall, so a stale entry of the queue is pushed back with its present count)
+        std::priority_queue<std::pair<int, int>> queue;
+        for (int e = 0; e < np; e++) {
+            for (int t : of[e]) cnt[e] += cov[t] == 0;
+            if (!keep[e] && cnt[e] > 0) queue.push({cnt[e], -e});
+        }
+        while (!queue.empty()) {
+            const auto [c, ne] = queue.top();
+            const int b = -ne;
+            queue.pop();
+            if (cnt[b] <= 0) continue;
+            if (cnt[b] < c) {
+                queue.push({cnt[b], -b});
+                continue;
+            }
+            keep[b] = 1;
+            for (int t : of[b])
+                if (cov[t]++ == 0)
+                    for (int k3 = 0; k3 < 3; k3++) {
+                        const int e = edge[3 * (size_t)t + k3];
+                        bool seen = false;
+                        for (int m = 0; m < k3; m++) seen |= edge[3 * (size_t)t + m] == e;
+                        if (!seen) cnt[e]--;
+                    }
+        }
+        int n = 0;
+        for (int e : by_size) {
+            if (!keep[e]) continue;
+            bool need = false;
+            for (int t : of[e]) need |= cov[t] == 1;
+            if (need) {
+                n++;
+                continue;
+            }
+            keep[e] = 0;
+            for (int t : of[e]) cov[t]--;
+        }
+        if (n < nbest) {
+            nbest = n;
+            best = keep;
+        }
+    }
+    std::vector<std::pair<int, int>> out;
+    for (int y = 0; y < nb; y++)
+        for (int x = 0; x <= y; x++)
+            if (best[id(x, y)]) out.push_back({x, y});
+    return out;
+}
+
 int TmPlan::build(const Shells &sh, int nsets_) {
     nsets = nsets_;
     const int nb = sh.nb;
     nA = nb;
-    // pairs (i, j) of set-0 shells, sorted by (j, i): consecutive TMEM lanes share j
-    std::map<std::pair<int, int>, int> pidx;
-    for (int64_t m = 0; m < sh.itot; m++) {
-        const int j = sh.tri[3 * m + 1], i = sh.tri[3 * m + 2];
-        pidx.emplace(std::make_pair(j - 1, i - 1), 0);
-    }
-    std::vector<int2> plist;
-    for (auto &kv : pidx) {
-        kv.second = (int)plist.size();
-        plist.push_back(make_int2(kv.first.second, kv.first.first));  // (i, j)
-    }
-    npairs = (int)plist.size();
     nslots = (int)(sh.itot * nsets);
-    const int nq = nsets * nb;  // q = map index s * nb + l - 1
-    const int nmt = (npairs + kM - 1) / kM, nnt = (nq + kN - 1) / kN;
-    struct E { int p, q, slot; };
-    std::vector<E> ents;
-    ents.reserve((size_t)sh.itot * nsets);
-    std::vector<char> need((size_t)nmt * nnt, 0);
+    // the plane rows and slots of each pair (x <= y): its triangles
+    struct E { int q, slot; };
+    std::map<std::pair<int, int>, std::vector<E>> ent;
+    if (nsets == 1)
+        for (auto &p : covering_pairs(sh)) ent[p];
     for (int64_t m = 0; m < sh.itot; m++) {
-        const int l = sh.tri[3 * m], j = sh.tri[3 * m + 1], i = sh.tri[3 * m + 2];
-        const int p = pidx.at(std::make_pair(j - 1, i - 1));
-        for (int s = 0; s < nsets; s++) {
-            const int q = s * nb + l - 1;
-            ents.push_back({p, q, (int)(m * nsets + s)});
-            need[(size_t)(p / kM) * nnt + q / kN] = 1;
-        }
-    }
-    std::vector<int2> h_units;
-    std::map<std::pair<int, int>, int> uidx;
-    // units ordered N tile outer, M tile inner: CTAs of one K range are adjacent in the grid
-    for (int nt = 0; nt < nnt; nt++)
-        for (int mt = 0; mt < nmt; mt++)
-            if (need[(size_t)mt * nnt + nt]) {
-                uidx[std::make_pair(mt, nt)] = (int)h_units.size();
-                h_units.push_back(make_int2(mt, nt));
+        const int l = sh.tri[3 * m] - 1, j = sh.tri[3 * m + 1] - 1, i = sh.tri[3 * m + 2] - 1;
+        if (nsets == 1) {
+            const int c[3][3] = {{i, j, l}, {i, l, j}, {j, l, i}};
+            for (auto &t : c) {
+                auto it = ent.find({t[0], t[1]});
+                if (it == ent.end()) continue;
+                it->second.push_back({t[2], (int)m});
+                break;
             }
-    nunits = (int)h_units.size();
-    std::vector<int2> h_prow((size_t)nunits * kM, make_int2(-1, -1));
-    std::vector<int> h_slots((size_t)nunits * kM * kN, -1);
-    for (int u = 0; u < nunits; u++)
-        for (int r = 0; r < kM; r++) {
-            const int p = h_units[u].x * kM + r;
-            if (p < npairs) h_prow[(size_t)u * kM + r] = plist[p];
+        } else {
+            for (int s = 0; s < nsets; s++) ent[{i, j}].push_back({l * nsets + s, (int)(m * nsets + s)});
         }
-    for (auto &e : ents) {
-        const int u = uidx.at(std::make_pair(e.p / kM, e.q / kN));
-        h_slots[((size_t)u * kM + e.p % kM) * kN + e.q % kN] = e.slot;
     }
-    PBI4G_CHECK(units.ensure(sizeof(int2) * std::max(1, nunits)));
-    PBI4G_CHECK(prow.ensure(sizeof(int2) * std::max<size_t>(1, h_prow.size())));
-    PBI4G_CHECK(slots.ensure(sizeof(int) * std::max<size_t>(1, h_slots.size())));
+    for (auto it = ent.begin(); it != ent.end();) it = it->second.empty() ? ent.erase(it) : std::next(it);
+    npairs = (int)ent.size();
+    // Groups of four pairs that share a map v: every pair belongs to one of its two maps, the
+    // larger one at first.  From the last map down, the pairs that do not fill a group of
+    // four are handed to their other map (the smallest first, so that neighbouring v give
+    // theirs to the same one): nearly all groups come out full.
+    std::vector<std::vector<int>> own(nb);  // v -> maps u
+    for (auto &kv : ent) own[kv.first.second].push_back(kv.first.first);
+    struct G { int v, u[4], n, lo, hi; };
+    std::vector<G> groups;
+    for (int v = nb - 1; v >= 0; v--) {
+        std::sort(own[v].begin(), own[v].end());
+        size_t rest = own[v].size() % 4, k = 0;
+        std::vector<int> mine;
+        for (; k < own[v].size(); k++) {
+            const int u = own[v][k];
+            if (rest > 0 && u < v) {  // to a map that is still to come
+                own[u].push_back(v);
+                rest--;
+            } else {
+                mine.push_back(u);
+            }
+        }
+        std::sort(mine.begin(), mine.end());
+        for (size_t m = mine.size(); m > 0;) {  // from the largest down: what is left over is small
+            G g = {v, {-1, -1, -1, -1}, 0, 1 << 30, -1};
+            for (; g.n < 4 && m > 0; m--) {
+                const int u = mine[m - 1];
+                g.u[g.n++] = u;
+                for (auto &e : ent[{std::min(u, v), std::max(u, v)}]) {
+                    g.lo = std::min(g.lo, e.q);
+                    g.hi = std::max(g.hi, e.q);
+                }
+            }
+            groups.push_back(g);
+        }
+    }
+    // M tiles: the groups in an order that keeps each tile's range of plane rows short, their
+    // warps (8 groups) spread evenly; units: windows of up to 64 rows of a tile's range.  The
+    // order with the least cost is taken (a unit's cost per chunk: a fixed part and its rows).
+    const int nw = ((int)groups.size() + 7) / 8, nt = (nw + 3) / 4;
+    auto first_group = [&](int t) { return std::min((int)groups.size(), 8 * (int)((long long)nw * t / nt)); };
+    struct U { int t, q, n; };
+    auto layout = [&](const std::vector<G> &gs, std::vector<U> &us) {
+        int cost = 0;
+        us.clear();
+        for (int t = 0; t < nt; t++) {
+            std::vector<char> used((size_t)nsets * nb + 1, 0);
+            for (int g = first_group(t); g < first_group(t + 1); g++)
+                for (int k = 0; k < gs[g].n; k++)
+                    for (auto &e : ent[{std::min(gs[g].u[k], gs[g].v), std::max(gs[g].u[k], gs[g].v)}]) used[e.q] = 1;
+            for (int q = 0; q < nsets * nb;) {
+                if (!used[q]) {
+                    q++;
+                    continue;
+                }
+                int last = q;
+                for (int r = q; r < std::min(q + kN, nsets * nb); r++)
+                    if (used[r]) last = r;
+                const int n = (last - q + 16) / 16 * 16;
+                us.push_back({t, q, n});
+                cost += 96 + n;
+                q = last + 1;
+            }
+        }
+        return cost;
+    };
+    std::vector<G> gbest;
+    std::vector<U> ubest, utry;
+    int cbest = 1 << 30;
+    for (int key = 0; key < 4; key++) {
+        std::vector<G> gs = groups;
+        std::stable_sort(gs.begin(), gs.end(), [key](const G &a, const G &b) {
+            if (key == 0) return a.lo != b.lo ? a.lo < b.lo : a.hi < b.hi;
+            if (key == 1) return a.hi != b.hi ? a.hi < b.hi : a.lo < b.lo;
+            if (key == 2) return a.lo + a.hi < b.lo + b.hi;
+            return a.v != b.v ? a.v < b.v : a.u[0] < b.u[0];
+        });
+        const int c = layout(gs, utry);
+        if (c < cbest) {
+            cbest = c;
+            gbest = gs;
+            ubest = utry;
+        }
+    }
+    ntiles = nt;
+    // Rows of a warp: group g takes the TMEM lanes g + 8 k.  Two neighbouring groups read
+    // their maps' rows in one shared-memory phase; rows r and r' fall on the same banks when
+    // bit 2 of both is the same (128-byte swizzle), so groups are paired, and their maps
+    // ordered, to have it differ.
+    std::vector<int2> h_prow((size_t)std::max(1, nt) * kM, make_int2(-1, -1));
+    std::map<std::pair<int, int>, std::pair<int, int>> at;  // pair -> (tile, row)
+    for (int t = 0; t < nt; t++) {
+        std::vector<G> gs(gbest.begin() + first_group(t), gbest.begin() + first_group(t + 1));
+        auto ones = [](const G &g) {
+            int c = 0;
+            for (int k = 0; k < g.n; k++) c += g.u[k] >> 2 & 1;
+            return c;
+        };
+        std::stable_sort(gs.begin(), gs.end(), [&](const G &a, const G &b) { return ones(a) < ones(b); });
+        std::vector<G> order;
+        for (size_t lo = 0, hi = gs.size(); lo < hi;) {
+            order.push_back(gs[lo++]);
+            if (lo < hi) order.push_back(gs[--hi]);
+        }
+        for (size_t g = 0; g < order.size(); g++) {
+            G &o = order[g];
+            std::stable_sort(o.u, o.u + o.n, [g](int a, int b) {
+                const int x = a >> 2 & 1, y = b >> 2 & 1;
+                return g % 2 ? x > y : x < y;
+            });
+            for (int k = 0; k < 4; k++) {
+                const int row = (int)(g / 8) * 32 + (int)(g % 8) + 8 * k;
+                // rows of a short group repeat its shared map (their products go nowhere)
+                h_prow[(size_t)t * kM + row] = make_int2(k < o.n ? o.u[k] : o.v, o.v);
+                if (k < o.n) at[{std::min(o.u[k], o.v), std::max(o.u[k], o.v)}] = {t, row};
+            }
+        }
+    }
+    // the units of one K range are adjacent in the grid
+    nunits = (int)ubest.size();
+    std::vector<int4> h_units;
+    std::vector<int> h_slots((size_t)std::max(1, nunits) * kM * kN, -1);
+    max_cols = 16;
+    for (auto &u : ubest) {
+        h_units.push_back(make_int4(u.t, u.q, u.n, nw * (u.t + 1) / nt - nw * u.t / nt));
+        max_cols = std::max(max_cols, u.n);
+    }
+    std::vector<int> first_unit(nt + 1, 0);  // (the units of a tile are consecutive)
+    for (int u = 0; u < nunits; u++) first_unit[ubest[u].t + 1] = u + 1;
+    for (auto &kv : ent) {
+        const auto [t, row] = at.at(kv.first);
+        for (auto &e : kv.second)
+            for (int u = first_unit[t]; u < first_unit[t + 1]; u++)
+                if (e.q >= ubest[u].q && e.q < ubest[u].q + ubest[u].n) {
+                    h_slots[((size_t)u * kM + row) * kN + e.q - ubest[u].q] = e.slot;
+                    break;
+                }
+    }
+    PBI4G_CHECK(units.ensure(sizeof(int4) * std::max(1, nunits)));
+    PBI4G_CHECK(prow.ensure(sizeof(int2) * h_prow.size()));
+    PBI4G_CHECK(slots.ensure(sizeof(int) * h_slots.size()));
     PBI4G_CHECK(err.ensure(sizeof(int)));
     if (nunits) {
-        PBI4G_CUDA(cudaMemcpy(units.p, h_units.data(), sizeof(int2) * h_units.size(), cudaMemcpyHostToDevice));
+        PBI4G_CUDA(cudaMemcpy(units.p, h_units.data(), sizeof(int4) * h_units.size(), cudaMemcpyHostToDevice));
         PBI4G_CUDA(cudaMemcpy(prow.p, h_prow.data(), sizeof(int2) * h_prow.size(), cudaMemcpyHostToDevice));
         PBI4G_CUDA(cudaMemcpy(slots.p, h_slots.data(), sizeof(int) * h_slots.size(), cudaMemcpyHostToDevice));
     }
@@ -787,11 +978,10 @@ bool tm_supported(const Shells &sh) {
 }
 
 template <int F>
-static int launch_tm(const CUtensorMap &tmA, const CUtensorMap &tmBh, const CUtensorMap &tmBl, const TmArgs &a,
-                     size_t smem, int grid, cudaStream_t st) {
+static int launch_tm(const TmMaps &tm, const TmArgs &a, size_t smem, int grid, cudaStream_t st) {
     auto kern = a.wait_limit < kWaitLimit ? trisum_tm_kernel<F, true> : trisum_tm_kernel<F, false>;
     PBI4G_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<grid, kThreads, smem, st>>>(tmA, tmBh, tmBl, a);
+    kern<<<grid, kThreads, smem, st>>>(tm, a);
     PBI4G_LAUNCH_CHECK();
     return PBI4G_OK;
 }
@@ -818,18 +1008,24 @@ int triangle_sums_tm(const Shells &sh, TmPlan &tp, const MapPlanes &pl, DevBuf &
     if (pl.nb != sh.nb || pl.npts < kKC || pl.npts > (long long)sh.Nm * sh.Nm * sh.Nm || pl.nchunks * kKC != pl.npts)
         return set_error(PBI4G_ERR_INVALID, "tensor-core triangle sums: operand planes do not match the shells");
     static_assert(MapPlanes::kChunk == kKC, "a planes chunk is a contraction chunk");
-    CUtensorMap tmA, tmBh, tmBl;
+    TmMaps tm;
     const long long nc = pl.nchunks;
-    PBI4G_CHECK(make_chunk_view(&tmA, pl.a32, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, nc, sh.nb, kKB, tp.nA));
-    if (form == 0) {
-        PBI4G_CHECK(make_chunk_view(&tmBh, pl.bhi, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, nc, pl.nmaps, kKB, kN));
-        PBI4G_CHECK(make_chunk_view(&tmBl, pl.blo, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, nc, pl.nmaps, kKB, kN));
-    } else if (form == 1) {
-        PBI4G_CHECK(make_chunk_view(&tmBh, pl.bhi, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, nc, pl.nmaps, kKC, kN));
-        PBI4G_CHECK(make_chunk_view(&tmBl, pl.blo, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, nc, pl.nmaps, kKC, kN));
-    } else {
-        PBI4G_CHECK(make_chunk_view(&tmBh, pl.bhi, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, nc, pl.nmaps, kKC, kN));
-        tmBl = tmBh;  // unused: one product
+    const int arows = (tp.nA + 7) / 8 * 8;
+    PBI4G_CHECK(make_chunk_view(&tm.a, pl.a32, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, nc, sh.nb, arows, kBlocks, 128));
+    for (int b = 0; b < 4; b++) {
+        const int n = 16 * (b + 1);
+        if (form == 0) {
+            PBI4G_CHECK(make_chunk_view(&tm.bh[b], pl.bhi, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, nc, pl.nmaps, n,
+                                        kBlocks, 128));
+            PBI4G_CHECK(make_chunk_view(&tm.bl[b], pl.blo, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, nc, pl.nmaps, n,
+                                        kBlocks, 128));
+        } else {
+            const size_t lo = form == 1 ? (size_t)((const char *)pl.blo - (const char *)pl.bhi) : 0;
+            PBI4G_CHECK(make_chunk_view(&tm.bh[b], pl.bhi,
+                                        form == 1 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
+                                        2, nc, pl.nmaps, n, form == 1 ? 2 : 1, form == 1 ? lo : 128));
+            tm.bl[b] = tm.bh[b];  // unused
+        }
     }
     TmArgs a;
     a.nchunks = nc;
@@ -852,9 +1048,10 @@ int triangle_sums_tm(const Shells &sh, TmPlan &tp, const MapPlanes &pl, DevBuf &
     a.nslots = tp.nslots;
     a.nA = tp.nA;
     a.nmaps = pl.nmaps;
-    a.ablock = (uint32_t)(((tp.nA + 7) / 8) * 8 * 128);
+    a.nb = pl.nb;
+    a.ablock = (uint32_t)arows * 128;
     const int btiles = form == 0 ? Form<kFormTF32>::kBTiles : (form == 1 ? Form<kFormF16>::kBTiles : 1);
-    a.stage_bytes = kBlocks * a.ablock + (uint32_t)btiles * kBTile;
+    a.stage_bytes = kBlocks * a.ablock + (uint32_t)btiles * (uint32_t)tp.max_cols * 128;
     // barriers, TMEM address, abort flag, pair table, B-row exponents
     const size_t fixed =
         1024 + 8 * (2 * kMaxStages + kMaxAStages + kDone + kAcc) + 16 + sizeof(int2) * kM + sizeof(int) * kN;
@@ -862,7 +1059,7 @@ int triangle_sums_tm(const Shells &sh, TmPlan &tp, const MapPlanes &pl, DevBuf &
     while (a.nstages > 3 && fixed + (size_t)a.nstages * a.stage_bytes > 227 * 1024) a.nstages--;
     const size_t smem = fixed + (size_t)a.nstages * a.stage_bytes;
     if (smem > 227 * 1024) return set_error(PBI4G_ERR_UNSUPPORTED, "tensor-core triangle sums: %zu B smem", smem);
-    a.units = tp.units.as<int2>();
+    a.units = tp.units.as<int4>();
     a.prow = tp.prow.as<int2>();
     a.slots = tp.slots.as<int>();
     PBI4G_CHECK(tp.mexp.ensure(sizeof(int) * std::max(1, pl.nmaps)));
@@ -873,16 +1070,9 @@ int triangle_sums_tm(const Shells &sh, TmPlan &tp, const MapPlanes &pl, DevBuf &
     a.wait_limit = tp.wait_limit > 0 && tp.wait_limit < kWaitLimit ? tp.wait_limit : kWaitLimit;
     PBI4G_CUDA(cudaMemsetAsync(tp.err.p, 0, sizeof(int), st));
     const int grid = tp.nunits * a.ksplit;
-    a.kahan = nullptr;
-    const bool kt = form == 0 ? kahan_in_tmem<kFormTF32>()
-                              : (form == 1 ? kahan_in_tmem<kFormF16>() : kahan_in_tmem<kFormBF16>());
-    if (!kt) {  // the running sums do not fit beside the accumulators and A stages in TMEM
-        PBI4G_CHECK(tp.kahan.ensure(sizeof(float) * 2 * kN * kM * (size_t)grid));
-        a.kahan = tp.kahan.as<float>();
-    }
-    if (form == 0) PBI4G_CHECK(launch_tm<kFormTF32>(tmA, tmBh, tmBl, a, smem, grid, st));
-    else if (form == 1) PBI4G_CHECK(launch_tm<kFormF16>(tmA, tmBh, tmBl, a, smem, grid, st));
-    else PBI4G_CHECK(launch_tm<kFormBF16>(tmA, tmBh, tmBl, a, smem, grid, st));
+    if (form == 0) PBI4G_CHECK(launch_tm<kFormTF32>(tm, a, smem, grid, st));
+    else if (form == 1) PBI4G_CHECK(launch_tm<kFormF16>(tm, a, smem, grid, st));
+    else PBI4G_CHECK(launch_tm<kFormBF16>(tm, a, smem, grid, st));
     PBI4G_CHECK(reduce_partials(tp.nslots, a.ksplit, partial.as<double>(), S, accumulate, st));
     *launches += 2;
     return PBI4G_OK;

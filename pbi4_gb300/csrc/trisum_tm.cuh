@@ -5,13 +5,16 @@
 
 namespace pbi4g {
 
-// Unit layout of the tcgen05 contraction for one (shells, q sets) layout:
-// units of one 128-pair M tile and one 64-map N tile; q = map index (set-major).
+// Unit layout of the tcgen05 contraction for one (shells, q sets) layout: units of one
+// M tile of up to 128 pairs and one window of up to 64 consecutive plane rows
+// (MapPlanes::row_of).  Pairs come in groups of four that share a factor map.
 struct TmPlan {
-    int nsets = 1, npairs = 0, nslots = 0, nunits = 0, nA = 0;
-    DevBuf units, prow, slots, err;
+    int nsets = 1, npairs = 0, nslots = 0, nunits = 0, ntiles = 0, nA = 0, max_cols = 0;
+    DevBuf units;    // int4 [nunits]: (M tile, first plane row, rows: 16, 32, 48 or 64, warps of pairs)
+    DevBuf prow;     // int2 [ntiles][128]: the maps (u, v) of each pair; v is the group's shared map
+    DevBuf slots;    // int [nunits][128][64]: output slot or -1
+    DevBuf err;
     DevBuf mexp;     // FP16 form: per-map power-of-two exponents
-    DevBuf kahan;    // per-CTA running sums when they do not fit in TMEM beside the accumulators
     uint32_t wait_limit = 0;  // diagnostic: polls before a main-loop wait gives up (0: the default)
     int build(const Shells &sh, int nsets);
 };
