@@ -17,18 +17,30 @@
 //  * assign_direct -- one global atomic per contribution (small / sparse inputs).
 #include "common.cuh"
 #include "assign.cuh"
+#include "fixed.cuh"
 
 #include <math.h>
 #include <string.h>
 
+#include <type_traits>
+
+#define PBI4G_UNROLL _Pragma("unroll")
+
 namespace pbi4g {
+
+// t mod N for a cell index (t is in [-2, 2N) for positions in [0, 1]; any other t takes the
+// 64-bit division)
+__device__ __forceinline__ int wrap_mod(long long t, int N) {
+    if (t >= 0 && t < 2LL * N) return (int)(t >= N ? t - N : t);
+    return (int)(t % N);
+}
 
 // Per-axis stencil of one particle coordinate p in [0,1]: first cell index
 // (0-based, not yet wrapped) and the nintp weights.  `cic_nint` selects the
 // single-grid CIC offset h = v - nint(v) (powerI4.f90:120) instead of
 // h = v - int(v) (double grid, powerI4.f90:216-217).
-template <class W>
-__device__ __forceinline__ void axis_stencil(double p, int N, int nintp, bool shifted, bool cic_nint, int &first,
+template <class W, int nintp>
+__device__ __forceinline__ void axis_stencil(double p, int N, bool shifted, bool cic_nint, int &first,
                                              W w[4]) {
     // vr = dble(Nv)*pos + 1 with the product and the sum rounded separately (no FMA
     // contraction), as the oracle's ISO C and an FMA-free Fortran build compute it
@@ -37,7 +49,7 @@ __device__ __forceinline__ void axis_stencil(double p, int N, int nintp, bool sh
     double h;
     if (nintp == 4) {
         long long iv = (long long)v;           // int(vr)
-        first = (int)((iv - 2) % N);            // mod(ivr - 3 + 1 + N, N)
+        first = wrap_mod(iv - 2, N);            // mod(ivr - 3 + 1 + N, N)
         h = v - (double)iv;
         W hh = (W)h, h2 = hh * hh;
         w[0] = ((W)1 - hh) * ((W)1 - hh) * ((W)1 - hh) / (W)6;
@@ -46,7 +58,7 @@ __device__ __forceinline__ void axis_stencil(double p, int N, int nintp, bool sh
         w[2] = (W)1 - w[0] - w[1] - w[3];
     } else if (nintp == 3) {
         long long iv = llround(v);             // nint(vr)
-        first = (int)((iv - 2) % N);
+        first = wrap_mod(iv - 2, N);
         h = v - (double)iv;
         W hh = (W)h, h2 = hh * hh;
         w[0] = (W)0.5 * ((W)0.5 - hh) * ((W)0.5 - hh);
@@ -55,14 +67,14 @@ __device__ __forceinline__ void axis_stencil(double p, int N, int nintp, bool sh
         w[3] = 0;
     } else if (nintp == 2) {
         long long iv = (long long)v;           // int(vr)
-        first = (int)(iv % N);                  // mod(ivr - 1 + 1 + N, N)
+        first = wrap_mod(iv, N);                // mod(ivr - 1 + 1 + N, N)
         h = cic_nint ? v - (double)llround(v) : v - (double)iv;
         w[0] = (W)1 - (W)h;
         w[1] = (W)h;
         w[2] = w[3] = 0;
     } else {
         long long iv = llround(v);             // nint(vr)
-        first = (int)((iv - 1) % N);            // mod(ivr - 1 + N, N)
+        first = wrap_mod(iv - 1, N);            // mod(ivr - 1 + N, N)
         w[0] = 1;
         w[1] = w[2] = w[3] = 0;
     }
@@ -72,15 +84,10 @@ __device__ __forceinline__ void axis_stencil(double p, int N, int nintp, bool sh
     if (first < 0 || first >= N) first = 0;
 }
 
-template <class W>
-__device__ __forceinline__ long long to_fixed(W c, double scale) {
-    return __double2ll_rn((double)c * scale);
-}
-
 // ---------------------------------------------------------------- direct ---
-template <class W>
-__global__ void assign_direct_kernel(int N, int nintp, int64_t npart, const double *__restrict__ pos,
-                                     const double *__restrict__ weight, double scale, int interlaced,
+template <class W, int nintp>
+__global__ void assign_direct_kernel(int N, int64_t npart, const double *__restrict__ pos,
+                                     const double *__restrict__ weight, int bits, int interlaced,
                                      unsigned long long *__restrict__ g1, unsigned long long *__restrict__ g2) {
     const size_t NN = (size_t)N * N;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < npart;
@@ -91,18 +98,18 @@ __global__ void assign_direct_kernel(int N, int nintp, int64_t npart, const doub
             int f0, f1, f2;
             W wx[4], wy[4], wz[4];
             const bool shifted = g == 1, cic_nint = !interlaced;
-            axis_stencil<W>(p0, N, nintp, shifted, cic_nint, f0, wx);
-            axis_stencil<W>(p1, N, nintp, shifted, cic_nint, f1, wy);
-            axis_stencil<W>(p2, N, nintp, shifted, cic_nint, f2, wz);
+            axis_stencil<W, nintp>(p0, N, shifted, cic_nint, f0, wx);
+            axis_stencil<W, nintp>(p1, N, shifted, cic_nint, f1, wy);
+            axis_stencil<W, nintp>(p2, N, shifted, cic_nint, f2, wz);
             unsigned long long *grid = g ? g2 : g1;
-            for (int a = 0; a < nintp; a++) {
+            PBI4G_UNROLL for (int a = 0; a < nintp; a++) {
                 int x = f0 + a; x -= (x >= N) ? N : 0;
-                for (int b = 0; b < nintp; b++) {
+                PBI4G_UNROLL for (int b = 0; b < nintp; b++) {
                     int y = f1 + b; y -= (y >= N) ? N : 0;
                     W wxy = wx[a] * wy[b];
-                    for (int c = 0; c < nintp; c++) {
+                    PBI4G_UNROLL for (int c = 0; c < nintp; c++) {
                         int z = f2 + c; z -= (z >= N) ? N : 0;
-                        long long q = to_fixed<W>(wxy * wz[c] * wt, scale);
+                        long long q = to_fixed(weight ? wxy * wz[c] * wt : wxy * wz[c], bits);
                         atomicAdd(grid + (size_t)z * NN + (size_t)y * N + x, (unsigned long long)q);
                     }
                 }
@@ -122,20 +129,22 @@ constexpr int kHalo = 4;                   // 1 cell below + up to 3 above
 constexpr int kAcc = kTile + kHalo;        // 12
 constexpr int kAccCells = kAcc * kAcc * kAcc;  // 1728 x 8 B = 13.8 KB per grid
 
-__device__ __forceinline__ int tile_of(double p, int N, int nintp, int ntile_axis) {
+template <int nintp>
+__device__ __forceinline__ int tile_of(double p, int N, int ntile_axis) {
     int f;
     float w[4];
-    axis_stencil<float>(p, N, nintp, false, false, f, w);
+    axis_stencil<float, nintp>(p, N, false, false, f, w);
     return f / kTile < ntile_axis ? f / kTile : ntile_axis - 1;
 }
 
-__global__ void tile_count_kernel(int N, int nintp, int64_t npart, const double *__restrict__ pos, int nt,
+template <int nintp>
+__global__ void tile_count_kernel(int N, int64_t npart, const double *__restrict__ pos, int nt,
                                   unsigned int *__restrict__ tile_count, unsigned int *__restrict__ ptile) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < npart;
          i += (int64_t)gridDim.x * blockDim.x) {
-        int tx = tile_of(pos[i], N, nintp, nt);
-        int ty = tile_of(pos[npart + i], N, nintp, nt);
-        int tz = tile_of(pos[2 * npart + i], N, nintp, nt);
+        int tx = tile_of<nintp>(pos[i], N, nt);
+        int ty = tile_of<nintp>(pos[npart + i], N, nt);
+        int tz = tile_of<nintp>(pos[2 * npart + i], N, nt);
         unsigned int t = (unsigned)((tz * nt + ty) * nt + tx);
         ptile[i] = t;
         atomicAdd(tile_count + t, 1u);
@@ -184,10 +193,10 @@ __global__ void tile_scatter_kernel(int64_t npart, const unsigned int *__restric
         order[atomicAdd(cursor + ptile[i], 1u)] = (unsigned int)i;
 }
 
-template <class W>
-__global__ void __launch_bounds__(256) assign_tiled_kernel(int N, int nintp, int64_t npart,
+template <class W, int nintp>
+__global__ void __launch_bounds__(256) assign_tiled_kernel(int N, int64_t npart,
                                                            const double *__restrict__ pos,
-                                                           const double *__restrict__ weight, double scale,
+                                                           const double *__restrict__ weight, int bits,
                                                            int interlaced, int nt,
                                                            const unsigned int *__restrict__ start,
                                                            const unsigned int *__restrict__ order,
@@ -212,19 +221,19 @@ __global__ void __launch_bounds__(256) assign_tiled_kernel(int N, int nintp, int
                 int f0, f1, f2;
                 W wx[4], wy[4], wz[4];
                 const bool shifted = g == 1, cic_nint = !interlaced;
-                axis_stencil<W>(p0, N, nintp, shifted, cic_nint, f0, wx);
-                axis_stencil<W>(p1, N, nintp, shifted, cic_nint, f1, wy);
-                axis_stencil<W>(p2, N, nintp, shifted, cic_nint, f2, wz);
+                axis_stencil<W, nintp>(p0, N, shifted, cic_nint, f0, wx);
+                axis_stencil<W, nintp>(p1, N, shifted, cic_nint, f1, wy);
+                axis_stencil<W, nintp>(p2, N, shifted, cic_nint, f2, wz);
                 // local coordinates; a first cell that wrapped below 0 maps to N-1
                 int lx = f0 - ox, ly = f1 - oy, lz = f2 - oz;
                 if (lx < 0) lx += N; if (ly < 0) ly += N; if (lz < 0) lz += N;
                 if (lx >= N) lx -= N; if (ly >= N) ly -= N; if (lz >= N) lz -= N;
                 const bool inside = lx + nintp <= kAcc && ly + nintp <= kAcc && lz + nintp <= kAcc;
-                for (int a = 0; a < nintp; a++)
-                    for (int bb = 0; bb < nintp; bb++) {
+                PBI4G_UNROLL for (int a = 0; a < nintp; a++)
+                    PBI4G_UNROLL for (int bb = 0; bb < nintp; bb++) {
                         W wxy = wx[a] * wy[bb];
-                        for (int c = 0; c < nintp; c++) {
-                            long long q = to_fixed<W>(wxy * wz[c] * wt, scale);
+                        PBI4G_UNROLL for (int c = 0; c < nintp; c++) {
+                            long long q = to_fixed(weight ? wxy * wz[c] * wt : wxy * wz[c], bits);
                             if (inside) {
                                 atomicAdd(&acc[g][((lz + c) * kAcc + (ly + bb)) * kAcc + (lx + a)],
                                           (unsigned long long)q);
@@ -340,26 +349,33 @@ int assign_fixed(AssignWork &wk, int N, int nintp, bool interlaced, bool fp64_we
     PBI4G_CHECK(fixed_point_bits(npart, wmax, &bits));
     *bits_out = bits;
     if (npart == 0) return PBI4G_OK;
-    const double scale = ldexp(1.0, bits);
     const int nt = (N + kTile - 1) / kTile;
     const int ntiles = nt * nt * nt;
     // Tiling pays when tiles hold several particles on average.
     const bool tiled = N >= 2 * kTile && npart >= (int64_t)ntiles * 2;
+    // the kernels are compiled per order: their weights stay in registers
+    auto by_order = [&](auto run) {
+        if (nintp == 1) run(std::integral_constant<int, 1>{});
+        else if (nintp == 2) run(std::integral_constant<int, 2>{});
+        else if (nintp == 3) run(std::integral_constant<int, 3>{});
+        else run(std::integral_constant<int, 4>{});
+    };
     if (!tiled) {
-        if (fp64_weights)
-            assign_direct_kernel<double><<<grid_blocks(npart, 256), 256, 0, st>>>(N, nintp, npart, d_pos, d_weight,
-                                                                                 scale, interlaced, g1, g2);
-        else
-            assign_direct_kernel<float><<<grid_blocks(npart, 256), 256, 0, st>>>(N, nintp, npart, d_pos, d_weight,
-                                                                                scale, interlaced, g1, g2);
+        by_order([&](auto ni) {
+            constexpr int NI = decltype(ni)::value;
+            auto kern = fp64_weights ? assign_direct_kernel<double, NI> : assign_direct_kernel<float, NI>;
+            kern<<<grid_blocks(npart, 256), 256, 0, st>>>(N, npart, d_pos, d_weight, bits, interlaced, g1, g2);
+        });
         PBI4G_LAUNCH_CHECK();
         ++*launches;
         return PBI4G_OK;
     }
     unsigned int *cnt = wk.tile_count.as<unsigned int>();
     PBI4G_CUDA(cudaMemsetAsync(cnt, 0, (size_t)(ntiles + 1) * 4, st));
-    tile_count_kernel<<<grid_blocks(npart, 256), 256, 0, st>>>(N, nintp, npart, d_pos, nt, cnt,
-                                                               wk.ptile.as<unsigned int>());
+    by_order([&](auto ni) {
+        tile_count_kernel<decltype(ni)::value><<<grid_blocks(npart, 256), 256, 0, st>>>(
+            N, npart, d_pos, nt, cnt, wk.ptile.as<unsigned int>());
+    });
     PBI4G_LAUNCH_CHECK();
     tile_scan_kernel<<<1, 1024, 0, st>>>(ntiles, cnt, wk.tile_start.as<unsigned int>(),
                                          wk.tile_cursor.as<unsigned int>());
@@ -369,14 +385,12 @@ int assign_fixed(AssignWork &wk, int N, int nintp, bool interlaced, bool fp64_we
                                                                  wk.order.as<unsigned int>());
     PBI4G_LAUNCH_CHECK();
     const int blocks = ntiles < 152 * 8 ? ntiles : 152 * 8;
-    if (fp64_weights)
-        assign_tiled_kernel<double><<<blocks, 256, 0, st>>>(N, nintp, npart, d_pos, d_weight, scale, interlaced, nt,
-                                                           wk.tile_start.as<unsigned int>(),
-                                                           wk.order.as<unsigned int>(), g1, g2);
-    else
-        assign_tiled_kernel<float><<<blocks, 256, 0, st>>>(N, nintp, npart, d_pos, d_weight, scale, interlaced, nt,
-                                                          wk.tile_start.as<unsigned int>(),
-                                                          wk.order.as<unsigned int>(), g1, g2);
+    by_order([&](auto ni) {
+        constexpr int NI = decltype(ni)::value;
+        auto kern = fp64_weights ? assign_tiled_kernel<double, NI> : assign_tiled_kernel<float, NI>;
+        kern<<<blocks, 256, 0, st>>>(N, npart, d_pos, d_weight, bits, interlaced, nt,
+                                     wk.tile_start.as<unsigned int>(), wk.order.as<unsigned int>(), g1, g2);
+    });
     PBI4G_LAUNCH_CHECK();
     *launches += 4;
     return PBI4G_OK;
