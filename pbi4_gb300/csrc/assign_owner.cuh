@@ -5,7 +5,7 @@
 namespace pbi4g {
 
 struct OwnerWork {
-    DevBuf count, start, cursor, key, rec, sorted, wsorted, wmax;
+    DevBuf count, start, cursor, sorted, wsorted, wmax;
     bool fixed = false;  // a shared scratch: sized once, never reallocated (ensure fails instead)
     int ensure(int N, int64_t npart);
     bool fits(int N, int64_t npart) const;
@@ -14,6 +14,10 @@ struct OwnerWork {
 };
 
 bool owner_supported(int N);
+// Whether a direct (not captured) box of npart particles is assigned by the owner tiles: the
+// supported grids, and other grids from 32 on up to 2^26 particles (their records take 288
+// bytes a particle, where the 64-bit grid in global memory takes 8 a particle and 8 a cell).
+bool owner_direct(int N, int64_t npart);
 
 // The owner kernels read the buffers of their OwnerWork from a device block of
 // kOwnerPtrBytes bytes, which the caller fills from owner_ptrs_host whenever the

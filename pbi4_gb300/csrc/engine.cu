@@ -546,7 +546,14 @@ static int owner_bind(pbi4g_plan *p, int64_t npart) {
 static int density_impl(pbi4g_plan *p, int64_t npart, const double *d_pos, const double *d_weight, const BoxPar *bp) {
     const int N = p->N;
     int bits;
-    if (!p->fp64 && owner_supported(N)) {
+    bool owner = !p->fp64 && (bp ? owner_supported(N) : owner_direct(N, npart));
+    if (owner && !bp && !owner_supported(N) && p->ow_cur->ensure(N, npart) != PBI4G_OK) {
+        // no room for this grid's records: the 64-bit grid in global memory
+        p->ow_cur->release();
+        cudaGetLastError();
+        owner = false;
+    }
+    if (owner) {
         // FP32 grids straight from the owner-computes tiles (fixed-point sums in shared memory);
         // a captured box uses the binding made before the capture
         if (!bp) PBI4G_CHECK(owner_bind(p, npart));
