@@ -177,19 +177,20 @@ __device__ __forceinline__ float sfrac_to_float(long long x) {
 // its fraction, aligned to 64 bits, in which the shifted grid's v - 1/2 (exact) flips the top
 // bit and nint's offset is the two's complement reading.  Each offset takes the single FP32
 // rounding first_and_h gives it, so cells and offsets are bit-identical to it.  v outside
-// [1, 4096) (positions outside [0, 1]) takes first_and_h.
+// [1, N + 2) (positions outside [0, 1]) takes first_and_h.
 __device__ __forceinline__ void first_cells(double p, int N, int nintp, bool interlaced, int &f0, float &h0, int &f1,
                                             float &h1) {
     const double v = __dadd_rn(__dmul_rn((double)N, p), 1.0);  // two roundings, as in assign.cu
     const unsigned hi = (unsigned)__double2hiint(v);
-    if (hi - 0x3FF00000u >= 0x00C00000u) {
+    // (of no use, and not used, where v is outside)
+    const int k = (int)(hi >> 20) - 1023;                            // 2^k <= v < 2^(k+1)
+    const int iv = (int)(((hi & 0xFFFFFu) | 0x100000u) >> ((20 - k) & 31));  // floor(v)
+    if (hi - 0x3FF00000u >= 0x00C00000u || iv > N + 1) {
         first_and_h(p, N, nintp, false, !interlaced, f0, h0);
         if (interlaced) first_and_h(p, N, nintp, true, false, f1, h1);
         else { f1 = f0; h1 = 0.f; }
         return;
     }
-    const int k = (int)(hi >> 20) - 1023;                            // 2^k <= v < 2^(k+1)
-    const int iv = (int)(((hi & 0xFFFFFu) | 0x100000u) >> (20 - k));  // floor(v)
     const unsigned long long fr = (unsigned long long)__double_as_longlong(v) << (12 + k);  // (v - floor(v)) 2^64
     const unsigned long long frs = fr ^ (1ull << 63);                // v - 1/2: the same
     const bool up = (long long)fr < 0;                               // v - floor(v) >= 1/2

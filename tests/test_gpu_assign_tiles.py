@@ -75,3 +75,15 @@ def test_no_room_for_records():
     kw = dict(grid=50, nintp=4, interlacing=True)
     a, b = _delta(pos, None, **kw), _delta(pos, None, fail=1, **kw)
     assert np.abs(_low(a) - _low(b)).max() <= 2 * TOL * abs(a[0, 0, 0])
+
+
+@pytest.mark.parametrize("grid,nintp,interlacing", [(34, 4, True), (64, 4, True), (64, 3, False), (66, 2, True), (208, 1, False)])
+def test_positions_far_outside(grid, nintp, interlacing):
+    pos = _particles(3000, grid, 3)
+    far = np.array([77.7, -3.2, 12.0 + 1 / 3, 2.0, 1.0 + 1.5 / grid, 1.0 + 2.5 / grid, 60.0, -0.5 / grid])
+    rng = np.random.default_rng(4)
+    pos[:, 500:540] = np.where(rng.random((3, 40)) < 0.5, rng.choice(far, (3, 40)), pos[:, 500:540])
+    kw = dict(grid=grid, nintp=nintp, interlacing=interlacing)
+    a, b = _delta(pos, None, **kw), _delta(pos, None, precision="fp64", **kw)
+    # a negative offset (above -1) takes the weights to 4/3 at most
+    assert np.abs(_low(a) - _low(b)).max() <= 4 * TOL * np.abs(_low(b)).max()
