@@ -138,27 +138,27 @@ __device__ __forceinline__ double position(double p, double v, bool shift, doubl
     return q < 1.0 || isnan(q) ? q : 1.0;
 }
 
-template <class T>
+template <class T, bool SHIFT>
 __global__ void __launch_bounds__(kThreads) catalog_positions_kernel(int64_t n, const T *__restrict__ pos,
                                                                     const T *__restrict__ vel, const CatArgs a, T box,
                                                                     double *__restrict__ out) {
-    __shared__ T sp[3 * kTile], sv[3 * kTile];
+    __shared__ T sp[3 * kTile], sv[SHIFT ? 3 * kTile : 1];
     const int t = threadIdx.x;
     const int64_t ntiles = (n + kTile - 1) / kTile;
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int64_t base = tile * kTile;
         const int np = (int)(n - base < kTile ? n - base : kTile), ne = 3 * np;
-        T p[kPer], v[kPer];
+        T p[kPer], v[SHIFT ? kPer : 1];
 #pragma unroll
         for (int j = 0; j < kPer; j++) {
             const int e = t + j * kThreads;
             p[j] = e < ne ? __ldcs(pos + 3 * base + e) : (T)0;
-            v[j] = vel && e < ne ? __ldcs(vel + 3 * base + e) : (T)0;
+            if (SHIFT) v[j] = e < ne ? __ldcs(vel + 3 * base + e) : (T)0;
         }
 #pragma unroll
         for (int j = 0; j < kPer; j++) {
             sp[t + j * kThreads] = p[j];
-            if (vel) sv[t + j * kThreads] = v[j];
+            if (SHIFT) sv[t + j * kThreads] = v[j];
         }
         __syncthreads();
 #pragma unroll
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kThreads) catalog_positions_kernel(int64_t n, 
 #pragma unroll
             for (int d = 0; d < 3; d++)
                 __stcs(out + (size_t)d * n + base + i,
-                       position(sp[3 * i + d], vel ? sv[3 * i + d] : (T)0, vel != nullptr, box, a, d));
+                       position(sp[3 * i + d], SHIFT ? sv[3 * i + d] : (T)0, SHIFT, box, a, d));
         }
         __syncthreads();
     }
@@ -213,14 +213,15 @@ int pbi4g_catalog_positions(int64_t npart, const void *d_pos, const void *d_vel,
         if (!(fabs(c) > 0x1p-60 && fabs(c) < 0x1p60)) a.ch[d] = NAN;
     }
     const int blocks = grid_blocks((size_t)npart, kTile, 152 * 16);
+    auto launch = [&](auto kern, auto box_t) {
+        using T = decltype(box_t);
+        kern<<<blocks, kThreads, 0, st>>>(npart, static_cast<const T *>(d_pos), static_cast<const T *>(d_vel), a, box_t,
+                                          d_out);
+    };
     if (is_double)
-        catalog_positions_kernel<double><<<blocks, kThreads, 0, st>>>(npart, static_cast<const double *>(d_pos),
-                                                                      static_cast<const double *>(d_vel), a, box,
-                                                                      d_out);
+        launch(d_vel ? catalog_positions_kernel<double, true> : catalog_positions_kernel<double, false>, box);
     else
-        catalog_positions_kernel<float><<<blocks, kThreads, 0, st>>>(npart, static_cast<const float *>(d_pos),
-                                                                     static_cast<const float *>(d_vel), a, (float)box,
-                                                                     d_out);
+        launch(d_vel ? catalog_positions_kernel<float, true> : catalog_positions_kernel<float, false>, (float)box);
     PBI4G_LAUNCH_CHECK();
     return PBI4G_OK;
 }
