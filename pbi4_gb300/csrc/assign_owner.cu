@@ -6,18 +6,16 @@
 // are evaluated in FP32 from the FP64 cell offset.  Every contribution
 // (w_x w_y) w_z weight is rounded once to an integer at scale 2^S (|q| < 2^30,
 // 2^-28 resolution for unit weights: far below the FP32 grid's rounding) and
-// summed into 64-bit integers with shared-memory atomics, so the grid is
-// bit-identical for any particle order and schedule.
+// summed exactly with shared-memory atomics, so the grid is bit-identical for any
+// particle order and schedule.
 //
 // 1. count: per particle, the first stencil cell of each grid and the tiles its
 //    stencils touch (1 to 8).
 // 2. scan, then scatter: the particle is prepared again and one 32-byte record
 //    per (particle, touched tile) written in tile order.
-// 3. one CTA per tile, one warp per record: the lanes take distinct stencil
-//    cells of the record's particle (no two lanes of a warp add to the same
-//    cell), keep those inside the tile and add them into the tile's shared
-//    accumulator; the tile is then converted to FP32 and stored.  No global
-//    atomics, no int64 grid, no memset of the grids.
+// 3. one CTA per tile: groups of lanes take the records' stencils column by column and add
+//    them into the tile's shared accumulator, halo included; the tile's own cells are then
+//    converted to FP32 and stored.  No global atomics, no int64 grid, no memset of the grids.
 //
 // Tiles are 16^3 cells on grids that are a multiple of 16 and 10 to 16 cells an
 // axis on others (TileGeom).
@@ -26,9 +24,13 @@
 // positions (2.1e6 particles in 256^3, PCS on two grids): count 37 us (FP64 pipe
 // 67% busy with two operations a coordinate; issue 54%), scatter 75 us (issue 62%).
 // With prepared particles written by the count and read back by the scatter, and
-// the cells from FP64 arithmetic, the two took 154 us.  The tiles are bound by their
-// shared 64-bit atomics: 510 us of 134 M adds at 256^3, 31.5 ms at 10^7 particles in
-// 1024^3 (most of it clearing and storing 262,144 tiles of two grids).
+// the cells from FP64 arithmetic, the two took 154 us.
+// The tiles are bound by instruction issue (74% at 2 10^6 random particles in 256^3, 271 us;
+// 61 instructions a record of two grids) and next by the shared atomics; in dense boxes the
+// other way round.  Of the 483 us before, with 64-bit atomics on the cells inside the tile, the
+// tests of every cell, its branch and coefficients reloaded for want of registers took half.
+// Boxes of few particles are bound by clearing and storing the tiles (512^3: 376 us, 158 of
+// them the grids at HBM rate).
 #include "assign_owner.cuh"
 #include "fixed.cuh"
 
@@ -44,23 +46,30 @@ namespace {
 
 constexpr int kT = 16;                  // tile edge
 constexpr int kTC = kT * kT * kT;       // 4096 cells
-// padded shared layout of a tile's 64-bit sums: cell (x, y, z) at z * kPz + y * kPy + x.
-// A stencil step's lanes are (i, j, l) in [0,4) x [0,4) x [0,2), l = lane / 16; a 64-bit
-// access takes the bank pair 2 (i + 20 j + 16 l) = 2 i + 8 j (mod 32), so each half-warp
-// (one wavefront of 8-byte accesses) touches 16 distinct pairs.
-constexpr int kPy = 20, kPz = 336;
-constexpr int kTCP = kT * kPz;          // 5376 cells per tile array
+// Shared layout of a tile's sums: the tile and the NI cells below and above it that the
+// stencils of its records reach, so that a stencil is added whole, without a test for each
+// cell, and the halo is not stored (the neighbouring tiles have their own records of these
+// particles).  Cell (x, y, z) of the tile is word (z + NI) pitch_z + (y + NI) kPy + x + 4;
+// x has a halo of 4 for every order (rows of 96 bytes, 16-byte aligned in the tile).  Two
+// arrays, arr_words apart.  At order 4 a step's lanes are the columns (i, j) in [0,4) x [0,4)
+// of two items (grids 1 and 2 of one record, or two records): 16 columns take the banks
+// i + 24 j = i + 8 j' (mod 32), which leaves every second group of four banks to the other
+// array (arr_words = 4 mod 8).
+constexpr int kPy = 24;
+__host__ __device__ constexpr int halo_rows(int ni) { return kT + 2 * ni; }
+__host__ __device__ constexpr int pitch_z(int ni) { return kPy * halo_rows(ni); }
+__host__ __device__ constexpr int words(int ni) { return pitch_z(ni) * halo_rows(ni); }
+__host__ __device__ constexpr int arr_words(int ni) { return words(ni) + 4; }
+__host__ __device__ constexpr int origin_word(int ni) { return ni * (pitch_z(ni) + kPy) + 4; }
+constexpr size_t tile_smem(int ni) { return sizeof(unsigned) * (size_t)(arr_words(ni) + words(ni)); }
 constexpr int kThreads = 512;
 
-// One particle's stencil on one grid, relative to one tile (16 bytes): pack =
-// base + kBias | x mask << 13 | y mask << 17 | z mask << 21, with base the
-// padded offset (z kPz + y kPy + x) of the stencil's first cell from the tile
-// origin and bit i of an axis mask set when the stencil's cell i on that axis
-// lies inside the tile (pack 0: no cell inside).  The scatter writes them, so
-// the tile kernel's lanes test one bit pattern and add one offset per cell.
+// One particle's stencil on one grid, relative to one tile (16 bytes): the offsets that set
+// its weights, and in pack the byte offset of its first cell in the tile's shared array
+// (below 2^16) with kOut when a coordinate lies outside [0, 1].
 struct alignas(16) PCell {
-    int pack;
     float h[3];
+    int pack;
 };
 struct alignas(16) PTile {              // a sorted record (particle, tile), both grids (32 bytes)
     PCell g[2];
@@ -76,8 +85,7 @@ struct OwnerPtrs {
     float *wsorted;
 };
 static_assert(sizeof(OwnerPtrs) <= kOwnerPtrBytes, "owner pointer block");
-constexpr int kBias = 2048;             // a stencil with a cell inside starts at [-3, 15] per axis: base + kBias in [977, 7403]
-constexpr int kMX = 13, kMY = 17, kMZ = 21;
+constexpr int kOut = 1 << 16;
 
 // first cell (0-based, in [0,N)) and the offset h that sets the weights
 // t mod N for the cell indices: t is in [-2, 2N) for positions in [0, 1]
@@ -125,14 +133,55 @@ __device__ __forceinline__ float4 axis_poly(int i) {
     }
 }
 
-__device__ __forceinline__ float horner(float4 c, float h) { return fmaf(h, fmaf(h, fmaf(h, c.w, c.z), c.y), c.x); }
+// All weights of an axis: no FP32 rounding makes any of them negative inside the box.
+template <int NI>
+__device__ __forceinline__ void axis_weights(float h, float (&w)[NI]) {
+    if constexpr (NI == 4) {
+        const float u = 1.f - h, h2 = h * h, u2 = u * u;
+        w[0] = u * (1.f / 6.f) * u2;
+        w[1] = fmaf(fmaf(h, 0.5f, -1.f), h2, 2.f / 3.f);
+        w[2] = fmaf(fmaf(u, 0.5f, -1.f), u2, 0.66666663f);  // 2/3 rounded down: the two errors cancel in the sum
+        w[3] = h * (1.f / 6.f) * h2;
+    } else if constexpr (NI == 3) {
+        const float a = 0.5f - h, c = 0.5f + h;
+        w[0] = 0.5f * a * a;
+        w[1] = fmaf(-h, h, 0.75f);
+        w[2] = 0.5f * c * c;
+    } else if constexpr (NI == 2) {
+        w[0] = 1.f - h;
+        w[1] = h;
+    } else {
+        w[0] = 1.f;
+    }
+}
 
-// offset of a stencil's first cell from the tile origin, with the stencils that
-// wrap past the upper grid edge into tile 0 shifted down by N: the lanes'
-// cells are then d + c, inside the tile iff 0 <= d + c < 16 (N >= 32)
+// two float32 in one 64-bit register, and their packed multiply and multiply-add
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 f2(float lo, float hi) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float f2_lo(F2 a) { return __uint_as_float((unsigned)a); }
+__device__ __forceinline__ float f2_hi(F2 a) { return __uint_as_float((unsigned)(a >> 32)); }
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ F2 horner2(const F2 c[4], F2 h) { return fma2(h, fma2(h, fma2(h, c[3], c[2]), c[1]), c[0]); }
+
+// offset of a stencil's first cell from the origin of a tile that the stencils of its
+// particle touch, in [-NI, 16]: the tile and the stencil may lie on either side of the wrap
+// (N >= 32, so the three ranges are apart)
 __device__ __forceinline__ int tile_offset(int f, int o, int N) {
     const int d = f - o;
-    return d >= N - 4 ? d - N : d;
+    return d + (d < -4 ? N : 0) - (d >= N - 4 ? N : 0);
 }
 
 // The tiles of one axis.  Grids that are a multiple of 16 have N / 16 tiles of 16 cells;
@@ -177,8 +226,9 @@ __device__ __forceinline__ float sfrac_to_float(long long x) {
 // its fraction, aligned to 64 bits, in which the shifted grid's v - 1/2 (exact) flips the top
 // bit and nint's offset is the two's complement reading.  Each offset takes the single FP32
 // rounding first_and_h gives it, so cells and offsets are bit-identical to it.  v outside
-// [1, N + 2) (positions outside [0, 1]) takes first_and_h.
-__device__ __forceinline__ void first_cells(double p, int N, int nintp, bool interlaced, int &f0, float &h0, int &f1,
+// [1, N + 2) (positions outside [0, 1]) takes first_and_h (and returns true: its offsets may
+// make negative weights).
+__device__ __forceinline__ bool first_cells(double p, int N, int nintp, bool interlaced, int &f0, float &h0, int &f1,
                                             float &h1) {
     const double v = __dadd_rn(__dmul_rn((double)N, p), 1.0);  // two roundings, as in assign.cu
     const unsigned hi = (unsigned)__double2hiint(v);
@@ -189,7 +239,7 @@ __device__ __forceinline__ void first_cells(double p, int N, int nintp, bool int
         first_and_h(p, N, nintp, false, !interlaced, f0, h0);
         if (interlaced) first_and_h(p, N, nintp, true, false, f1, h1);
         else { f1 = f0; h1 = 0.f; }
-        return;
+        return true;
     }
     const unsigned long long fr = (unsigned long long)__double_as_longlong(v) << (12 + k);  // (v - floor(v)) 2^64
     const unsigned long long frs = fr ^ (1ull << 63);                // v - 1/2: the same
@@ -211,6 +261,7 @@ __device__ __forceinline__ void first_cells(double p, int N, int nintp, bool int
         f1 = cell(iv - 1); h1 = 0.f;
     }
     if (!interlaced) { f1 = f0; h1 = 0.f; }
+    return false;
 }
 
 // One particle: the cells and offsets of both grids, and the lowest first cell per axis
@@ -218,13 +269,19 @@ __device__ __forceinline__ void first_cells(double p, int N, int nintp, bool int
 struct Prep {
     int f[2][3], lo[3];
     float h[2][3];
+    int out;  // kOut when a coordinate lies outside [0, 1]
 };
 __device__ __forceinline__ void prep_particle(const double *__restrict__ pos, int64_t stride, int64_t i, int N,
                                               int nintp, int interlaced, Prep &r) {
+    r.out = 0;
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-        first_cells(__ldg(pos + (size_t)c * stride + i), N, nintp, interlaced != 0, r.f[0][c], r.h[0][c], r.f[1][c],
-                    r.h[1][c]);
+        if (first_cells(__ldg(pos + (size_t)c * stride + i), N, nintp, interlaced != 0, r.f[0][c], r.h[0][c], r.f[1][c],
+                        r.h[1][c])) {
+            r.out = kOut;
+            // never further apart than the tiles' halos hold
+            if (r.f[1][c] != r.f[0][c] && r.f[1][c] != (r.f[0][c] == 0 ? N - 1 : r.f[0][c] - 1)) r.f[1][c] = r.f[0][c];
+        }
         r.lo[c] = (interlaced && r.f[1][c] == (r.f[0][c] == 0 ? N - 1 : r.f[0][c] - 1)) ? r.f[1][c] : r.f[0][c];
     }
 }
@@ -349,17 +406,8 @@ __global__ void owner_scan_kernel(int ntiles, const OwnerPtrs ov, const OwnerPtr
     if (threadIdx.x == 0) start[ntiles] = carry;
 }
 
-// Mask of the stencil's NI cells d .. d + NI - 1 that fall inside a tile of tw cells, d the
-// offset of its first cell from the tile origin on one axis (tile_offset).
-__device__ __forceinline__ unsigned axis_mask(int d, int NI, int tw) {
-    const int lo = max(0, -d), hi = min(NI - 1, tw - 1 - d);
-    return lo <= hi ? ((2u << hi) - 1u) & ~((1u << lo) - 1u) : 0u;
-}
-
 // Scatter: a record per (particle, touched tile).  The positions are read again: preparing
-// them costs less than a 32-byte prepared record written by the count and read back.  Per
-// axis, grid and tile the cell offset and mask are one addend of PCell::pack, so a record's
-// pack is the sum of three.
+// them costs less than a 32-byte prepared record written by the count and read back.
 template <bool IND, bool GEN, bool SMALL>
 __global__ void __launch_bounds__(kSortThreads) owner_scatter_kernel(
     const TileGeom g, int nintp, int interlaced, int64_t npart, int64_t stride, const BoxPar *__restrict__ bp,
@@ -371,6 +419,7 @@ __global__ void __launch_bounds__(kSortThreads) owner_scatter_kernel(
     float *__restrict__ wsorted = weight ? (IND ? op->wsorted : ov.wsorted) : nullptr;
     __shared__ unsigned int place[SMALL ? kSmallTiles : 1];
     const int w = nintp + (interlaced ? 1 : 0);
+    const int pz = pitch_z(nintp), org = 4 * origin_word(nintp);
     const int ntiles = g.nt * g.nt * g.nt;
     int64_t b, e, step;
     block_share(SMALL, bp ? bp->npart : npart, b, e, step);
@@ -400,25 +449,17 @@ __global__ void __launch_bounds__(kSortThreads) owner_scatter_kernel(
         const int two = span_tiles<GEN>(r.lo, w, g, t);
         const unsigned act = __activemask();
         const float wt = weight ? (float)weight[i] : 1.f;
-        int x[3][2][2];  // [axis][tile of the axis][grid]
+        int x[3][2][2];  // byte offset by [axis][tile of the axis][grid]
 #pragma unroll
         for (int c = 0; c < 3; c++)
 #pragma unroll
             for (int k = 0; k < 2; k++) {
                 x[c][k][0] = x[c][k][1] = 0;
                 if (k == 1 && !__any_sync(act, two >> c & 1)) continue;
-                const int cell = c == 0 ? 1 : (c == 1 ? kPy : kPz), msk = c == 0 ? kMX : (c == 1 ? kMY : kMZ);
+                const int cell = 4 * (c == 0 ? 1 : (c == 1 ? kPy : pz));
                 const int o = tile_origin<GEN>(t[c][k], g);
-                const int tw = GEN ? tile_origin<GEN>(t[c][k] + 1, g) - o : kT;
 #pragma unroll
-                for (int gr = 0; gr < 2; gr++) {
-                    if (gr == 1 && !interlaced) continue;
-                    const int d = tile_offset(r.f[gr][c], o, g.N);
-                    // no cell in this tile: no offset either (a grid on the other side of the
-                    // wrap is up to N cells away, beyond what pack's low bits hold)
-                    const unsigned m = axis_mask(d, nintp, tw);
-                    x[c][k][gr] = m ? d * cell + (int)(m << msk) : 0;
-                }
+                for (int gr = 0; gr < 2; gr++) x[c][k][gr] = tile_offset(r.f[gr][c], o, g.N) * cell;
             }
         // slot by slot (as owner_count_kernel counts them)
 #pragma unroll
@@ -443,9 +484,7 @@ __global__ void __launch_bounds__(kSortThreads) owner_scatter_kernel(
                 PTile o;
 #pragma unroll
                 for (int gr = 0; gr < 2; gr++) {
-                    const int pk = kBias + x[0][sl & 1][gr] + x[1][(sl >> 1) & 1][gr] + x[2][sl >> 2][gr];
-                    const bool in = (pk >> kMX & 15) && (pk >> kMY & 15) && (pk >> kMZ & 15);
-                    o.g[gr].pack = in ? pk : 0;
+                    o.g[gr].pack = (org + x[0][sl & 1][gr] + x[1][(sl >> 1) & 1][gr] + x[2][sl >> 2][gr]) | r.out;
 #pragma unroll
                     for (int c = 0; c < 3; c++) o.g[gr].h[c] = r.h[gr][c];
                 }
@@ -456,217 +495,347 @@ __global__ void __launch_bounds__(kSortThreads) owner_scatter_kernel(
     }
 }
 
-// PCS records in columns: a half-warp takes one (particle, grid) pair of a
-// record, lane (j, i) = (l >> 2 & 3, l & 3) of it the z column of cells
-// (i, j, 0..3).  The x and y weights and their product are formed once per
-// column, the z weights per cell, in the same order as the cell mapping,
-// ((w_x w_y) w_z) weight, so every q is the same integer.  Two grids: the
-// halves take grids 0 and 1 of one record; one grid: two records.  Each
-// half-warp's 16 cells of a z step fall on 16 distinct bank pairs (2 i + 8 j).
 // Read-only loads of the sorted records (their pointers come from the pointer
 // block, so the compiler cannot infer that the kernel never writes them).
 __device__ __forceinline__ PCell ld_cell(const PCell *p) {
     const int4 v = __ldg(reinterpret_cast<const int4 *>(p));
     PCell c;
-    c.pack = v.x;
-    c.h[0] = __int_as_float(v.y);
-    c.h[1] = __int_as_float(v.z);
-    c.h[2] = __int_as_float(v.w);
+    c.h[0] = __int_as_float(v.x);
+    c.h[1] = __int_as_float(v.y);
+    c.h[2] = __int_as_float(v.z);
+    c.pack = v.w;
     return c;
 }
-__device__ __forceinline__ PTile ld_tile(const PTile *p) {
-    PTile t;
-    t.g[0] = ld_cell(&p->g[0]);
-    t.g[1] = ld_cell(&p->g[1]);
-    return t;
+
+__device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ float ldexp_bits(int e) { return __int_as_float((127 + e) << 23); }  // 2^e
+__device__ __forceinline__ void red_shared(unsigned a, unsigned v) {
+    asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ unsigned atom_shared(unsigned a, unsigned v) {
+    unsigned old;
+    asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(a), "r"(v) : "memory");
+    return old;
 }
 
-template <int G, bool W, bool GEN>
-__device__ __forceinline__ void pcs_columns(unsigned b, unsigned e, int warp, int nwarps, int lane, float scale, int bits,
-                                            const PTile *__restrict__ sorted, const float *__restrict__ wsorted,
-                                            unsigned long long *acc64) {
-    const int half = lane >> 4, ci = lane & 3, cj = (lane >> 2) & 3;
-    const int g = G == 2 ? half : 0;
-    const float4 px = axis_poly<4>(ci), py = axis_poly<4>(cj);
-    float4 pz[4];
-#pragma unroll
-    for (int l = 0; l < 4; l++) {
-        const float4 zc = axis_poly<4>(l);
-        pz[l] = make_float4(zc.x * scale, zc.y * scale, zc.z * scale, zc.w * scale);
-    }
-    const int need = (1 << (kMX + ci)) | (1 << (kMY + cj));  // the column's x and y cells
-    const int loff = g * kTCP + cj * kPy + ci - kBias;  // the column's cell offset less the bias
-    constexpr int RPW = G == 2 ? 1 : 2;  // records per warp step
-    const unsigned step = (unsigned)(RPW * nwarps), off = G == 2 ? 0u : (unsigned)half;
-    // the next record of the half-warp is loaded while this one is added
-    PCell cn = {};
-    float wn = 1.f;
-    if (b + (unsigned)(RPW * warp) + off < e) {
-        cn = ld_cell(&sorted[b + (unsigned)(RPW * warp) + off].g[g]);
-        if (W) wn = __ldg(&wsorted[b + (unsigned)(RPW * warp) + off]);
-    }
-    for (unsigned k = b + (unsigned)(RPW * warp) + off; k - off < e; k += step) {
-        const PCell c = cn;
-        const float wt = wn;
-        if (k + step < e) {
-            cn = ld_cell(&sorted[k + step].g[g]);
-            if (W) wn = __ldg(&wsorted[k + step]);
+// A tile's sums are kept in 32-bit shared words, whose atomics run at 2.7 times the rate of
+// 64-bit ones (3880 against 1440 lanes a ns over the GPU):
+//  * SHORT: the sum mod 2^32, biased by kSumBias, both grids at once.  No contribution is
+//    below -64 (offsets inside the box make no negative weights but for FP32 rounding), so a
+//    cell's sum is at least -kSumBias and a sum beyond 32 bits loses a positive multiple of
+//    2^32.  The tile's contributions are also summed in 64-bit registers: the cells hold
+//    their true sums exactly when the two totals agree.  If they do not, or a position lay
+//    outside the box, or a particle weight is negative, a second pass (HIGH) sums the
+//    contributions' bits from 16 up: with less than 2^16 records, the sum of the low 16 bits
+//    is what the first pass's sum holds beyond it.
+//    kFree: up to so many records no cell can reach 2^32 (a contribution is at most
+//    2^28 times the largest weight of the stencil), and the totals are not compared.
+//  * SPLIT: one grid at a time, the integer cut into the part above its low L bits and those
+//    bits, neither below -1, whose biased sums fill the two arrays and are checked in the same
+//    way.  GEN takes it for contributions of up to 43 bits, with L <= 22; others take it with
+//    L = 14 for tiles of more records.
+//  * WIDE: one grid at a time as 64-bit sums, low words and high words (array 0 and 1):
+//    the low word's atomic returns the old word, from which follows the carry.
+// The sums are the same integers in every form.  (2 10^6 particles in 256^3, order 4 on two
+// grids: 64-bit words 483 us, SHORT 271; 10^8: 19.9 ms, SHORT 10.7, SPLIT 21.8, WIDE 27.  Where
+// every tile has a cell beyond 16 particles, SHORT and HIGH take 533 against 475 us, and 4.17
+// against 4.12 ms at 2 10^7.)
+constexpr unsigned kSumBias = 1u << 24;
+constexpr unsigned kShortRecords = (1u << 16) - 1, kSplitRecords = 1u << 23;
+constexpr int kAhead = 4;
+__host__ __device__ constexpr unsigned free_records(int ni) { return ni == 4 ? 52u : (ni == 3 ? 36u : 15u); }
+enum Form { SHORT, HIGH, SPLIT, WIDE };
+
+// Add the tile's items: an item is one record's stencil on one grid (NG = 2: both grids in
+// turn, each into its own array; NG = 1: grid g0).  LPI lanes take an item, lane (j, i) of
+// them the z column of cells (i, j, 0 .. NI - 1): the x and y weights and their product are
+// formed once per column, the z weights per cell, in the reference's order
+// ((w_x w_y) w_z) weight.  The scale (2^S; with GEN 2^(S - L) in SPLIT and 1 in WIDE) rides in the
+// product (a power of two: the same bits as scaling at the end), so a contribution rounds
+// straight to an integer below 2^30.  GEN (grids that are not a multiple of 16): every
+// contribution is kept to 2^-bits, the resolution these grids had when their particles were
+// added to a 64-bit grid in global memory.  Returns the sum of the words added and collects
+// the records' pack bits in flags (SHORT, SPLIT).
+template <int NI, int NG, bool W, bool GEN, Form F, class Before>
+__device__ __forceinline__ long long add_items(unsigned b, unsigned e, int g0, float scale, int bits, int lbits,
+                                               const PTile *__restrict__ sorted, const float *__restrict__ wsorted,
+                                               unsigned *acc, int &flags, Before &&before) {
+    constexpr int LPI = NI * NI, IPW = 32 / LPI;
+    constexpr int PZ = 4 * pitch_z(NI), HI = 4 * arr_words(NI);
+    const unsigned sub = (threadIdx.x & 31) / LPI;
+    const int col = (threadIdx.x & 31) % LPI, ci = col % NI, cj = col / NI;
+    const float4 cx = axis_poly<NI>(ci), cy = axis_poly<NI>(cj);
+    const F2 pxy[4] = {f2(cx.x, cy.x), f2(cx.y, cy.y), f2(cx.z, cy.z), f2(cx.w, cy.w)};
+    const bool idle = sub >= IPW;  // (order 3: three items of 9 columns)
+    const unsigned n = (e - b) * NG, step = (blockDim.x >> 5) * IPW;
+    const unsigned t0 = (threadIdx.x >> 5) * IPW;
+    const int g = NG == 2 ? (int)((t0 + sub) & 1u) : g0;  // (step is even)
+    const unsigned base = smem_addr(acc) + 4u * (unsigned)((NG == 2 ? g * arr_words(NI) : 0) + cj * kPy + ci);
+    long long tot = 0;
+    auto fetch = [&](unsigned t, PCell &c, float &wt) {
+        t += sub;
+        if (t < n && !idle) {
+            c = ld_cell(&sorted[b + t / NG].g[g]);
+            if (W) wt = __ldg(&wsorted[b + t / NG]);
         }
-        // k >= e (the second record of a one-grid step past the end): pack 0
-        const int pk = k < e ? c.pack : 0;
-        const bool okxy = (pk & need) == need;
-        const float wxy = horner(px, c.h[0]) * horner(py, c.h[1]);
-        unsigned long long *col = acc64 + (loff + (pk & ((1 << kMX) - 1)));
+    };
+    auto add = [&](unsigned t, const PCell &c, float wt) {
+        if ((IPW > NG && t + sub >= n) || idle) return;
+        const F2 wxwy = horner2(pxy, f2(c.h[0], c.h[1]));  // w_x and w_y, each rounded as by single FMAs
+        const float wxy = f2_lo(wxwy) * f2_hi(wxwy) * scale;
+        float wz[NI];
+        axis_weights<NI>(c.h[2], wz);
+        const unsigned cell = base + (unsigned)(c.pack & (kOut - 1));
+        if (F == SHORT || F == SPLIT) {
+            flags |= c.pack;
+            if (W) flags |= wt >= 0.f ? 0 : kOut;
+        }
+        int part = 0;
 #pragma unroll
-        for (int l = 0; l < 4; l++) {
-            float wv = wxy * horner(pz[l], c.h[2]);
+        for (int l = 0; l < NI; l++) {
+            float wv = wxy * wz[l];
             if (W) wv *= wt;
-            const long long q = GEN ? to_fixed(wv, bits) : (long long)__float2int_rn(wv);
-            if (okxy && (pk >> (kMZ + l) & 1)) atomicAdd(col + l * kPz, (unsigned long long)q);
+            if constexpr (F == SHORT) {
+                const int q = __float2int_rn(wv);
+                red_shared(cell + l * PZ, (unsigned)q);
+                part += q;
+            } else if constexpr (F == HIGH) {
+                red_shared(cell + l * PZ, (unsigned)(__float2int_rn(wv) >> 16));
+            } else if constexpr (F == SPLIT) {
+                int hi, lo;
+                if constexpr (GEN) {
+                    // floor(wv) and the rest, rounded at 2^-L: below 2^22 both, so they are
+                    // read from the low bits of sums with 1.5 2^23
+                    const float m = 12582912.f, f = __fadd_rd(wv, m);
+                    hi = __float_as_int(f) - 0x4B400000;
+                    lo = __float_as_int(fmaf(wv - (f - m), ldexp_bits(lbits), m)) - 0x4B400000;
+                } else {
+                    const int q = __float2int_rn(wv);
+                    hi = q >> lbits;
+                    lo = q & ((1 << lbits) - 1);
+                }
+                red_shared(cell + l * PZ, (unsigned)lo);
+                red_shared(cell + l * PZ + HI, (unsigned)hi);
+                part += hi + lo;
+            } else {
+                const long long q = GEN ? to_fixed(wv, bits) : (long long)__float2int_rn(wv);
+                const unsigned old = atom_shared(cell + l * PZ, (unsigned)q);
+                const unsigned hi = (unsigned)(q >> 32) + (old + (unsigned)q < old ? 1u : 0u);
+                if (hi) red_shared(cell + l * PZ + HI, hi);
+            }
+        }
+        if (F == SHORT || F == SPLIT) tot += part;
+    };
+    // kAhead records of a warp in flight
+    PCell c[kAhead] = {};
+    float wt[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; k++) {
+        wt[k] = 1.f;
+        fetch(t0 + k * step, c[k], wt[k]);
+    }
+    before();
+    for (unsigned t = t0; t < n; t += kAhead * step) {
+#pragma unroll
+        for (int k = 0; k < kAhead; k++) {
+            if (t + k * step >= n) break;
+            add(t + k * step, c[k], wt[k]);
+            fetch(t + (k + kAhead) * step, c[k], wt[k]);
         }
     }
+    return tot;
 }
 
-// Tile kernel, specialised on the stencil width NI (1..4), the number of
-// grids G (2 when interlaced) and the presence of particle weights W: below
-// PCS a warp takes one record (particle, tile) and its lanes take the
-// G * NI^3 (grid, cell) pairs, so the cell indices and the weight polynomials
-// fold to constants and shifts; PCS takes the column mapping above.  The
-// fixed-point scale 2^S rides in the z polynomial (a power of two: the
-// products are the same bits as scaling at the end).
-// GEN (grids that are not a multiple of 16): tiles of 10 to 16 cells an axis, and every
-// contribution kept to 2^-bits as one 64-bit integer (scale is then 1), the resolution
-// these grids had when their particles were added to a 64-bit grid in global memory.
+// Tile kernel, specialised on the stencil width NI (1..4), the number of grids G (2 when
+// interlaced) and the presence of particle weights W.  A single CIC grid takes its offset
+// from the nearest cell, which makes weights of both signs: it has the WIDE form only.
+// lbits: L of the SPLIT form (negative: the contributions have more bits than it holds), and
+// split_free its kFree.
 template <int NI, int G, bool W, bool IND, bool GEN>
 __global__ void __launch_bounds__(kThreads, 2) owner_tile_kernel(const TileGeom g, const OwnerPtrs ov,
                                                                const OwnerPtrs *__restrict__ op, float scale,
-                                                               int bits, float inv_scale, float *__restrict__ out1,
-                                                               float *__restrict__ out2) {
-    constexpr int NC = NI * NI * NI;
-    extern __shared__ unsigned long long acc64[];  // [G][kTCP]
+                                                               int bits, int lbits, unsigned split_free,
+                                                               float inv_scale, float *__restrict__ out1, float *__restrict__ out2) {
+    constexpr bool kPositive = !(NI == 2 && G == 1), kShort = kPositive && !GEN;
+    constexpr int PZ = pitch_z(NI), ARR = arr_words(NI), ORG = origin_word(NI);
+    extern __shared__ __align__(16) unsigned acc[];  // arr_words + words
     const int N = g.N, nt = g.nt, ntiles = nt * nt * nt;
     const unsigned int *__restrict__ start = IND ? op->start : ov.start;
     const PTile *__restrict__ sorted = IND ? op->sorted : ov.sorted;
     const float *__restrict__ wsorted = W ? (IND ? op->wsorted : ov.wsorted) : nullptr;
     unsigned int *next_tile = (IND ? op->count : ov.count) + ntiles + 1;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    __shared__ int s_tile;
+    __shared__ int s_bad[2][3];  // [tile parity][grid, or 2 for both]
+    __shared__ unsigned s_tile[2], s_b[2], s_e[2];
+    __shared__ unsigned long long s_chk[2][3];
+    uint4 *acc4 = reinterpret_cast<uint4 *>(acc);
     // tiles are handed out dynamically (their particle loads differ by orders of
-    // magnitude in clustered boxes); the counter is zeroed before the launch
-    for (;;) {
-        if (threadIdx.x == 0) s_tile = (int)atomicAdd(next_tile, 1u);
+    // magnitude in clustered boxes); the counter is zeroed before the launch.  A tile is drawn
+    // and its records are fetched into L2 while the one before it is done
+    auto draw = [&](int slot) {
+        const unsigned t = atomicAdd(next_tile, 1u);
+        s_tile[slot] = t;
+        if (t < (unsigned)ntiles) {
+            const unsigned tb = __ldg(&start[t]), te = __ldg(&start[t + 1]);
+            s_b[slot] = tb;
+            s_e[slot] = te;
+            if (te > tb)
+                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(sorted + tb),
+                             "r"((unsigned)sizeof(PTile) * min(te - tb, kShortRecords))
+                             : "memory");
+        }
+    };
+    if (threadIdx.x == 0) draw(0);
+    for (int par = 0;; par ^= 1) {
+        if (threadIdx.x == 0) {
+#pragma unroll
+            for (int k = 0; k < 3; k++) {  // (the other tile's may still be read)
+                s_chk[par][k] = 0ull;
+                s_bad[par][k] = 0;
+            }
+        }
         __syncthreads();
-        const int tile = s_tile;
-        if (tile >= ntiles) break;
-        const int tx = tile % nt, ty = (tile / nt) % nt, tz = tile / (nt * nt);
+        const unsigned tile = s_tile[par];
+        if (tile >= (unsigned)ntiles) break;
+        const unsigned b = s_b[par], e = s_e[par];
+        if (threadIdx.x == 0) draw(par ^ 1);
+        const int tx = (int)tile % nt, ty = ((int)tile / nt) % nt, tz = (int)tile / (nt * nt);
         const int ox = tile_origin<GEN>(tx, g), oy = tile_origin<GEN>(ty, g), oz = tile_origin<GEN>(tz, g);
-        for (int c = threadIdx.x; c < G * kTCP; c += blockDim.x) acc64[c] = 0ull;
-        __syncthreads();
-        const unsigned b = __ldg(&start[tile]), e = __ldg(&start[tile + 1]);
-        if constexpr (NI == 4) {
-            pcs_columns<G, W, GEN>(b, e, warp, nwarps, lane, scale, bits, sorted, wsorted, acc64);
-        } else {
-            // per-lane stencil cells of one grid: NIT steps of 32 cells; the (i, j, l)
-            // of a lane, its cell offset, its bit pattern and its weight polynomials
-            // are the same for every record
-            constexpr int NIT = (NC + 31) / 32;
-            int need[NIT], loff[NIT];
-            float4 px[NIT], py[NIT], pz[NIT];
-#pragma unroll
-            for (int it = 0; it < NIT; it++) {
-                const int c = it * 32 + lane;
-                const int ci = c % NI, cj = (c / NI) % NI, cl = c < NC ? c / (NI * NI) : 0;
-                // no cell for this lane at this step: a bit no pack has
-                need[it] = c < NC ? (1 << (kMX + ci)) | (1 << (kMY + cj)) | (1 << (kMZ + cl)) : (1 << 30);
-                loff[it] = cl * kPz + cj * kPy + ci - kBias;
-                px[it] = axis_poly<NI>(ci);
-                py[it] = axis_poly<NI>(cj);
-                const float4 zc = axis_poly<NI>(cl);
-                pz[it] = make_float4(zc.x * scale, zc.y * scale, zc.z * scale, zc.w * scale);
+        auto clear = [&](int nwords, unsigned v) {
+            for (int c = threadIdx.x; c < nwords / 4; c += blockDim.x) acc4[c] = make_uint4(v, v, v, v);
+            __syncthreads();
+        };
+        // the totals' difference, into s_chk; every word in use was cleared to the bias
+        auto compare = [&](long long chk, int nwords, int gr) {
+            for (int c = threadIdx.x; c < nwords / 4; c += blockDim.x) {
+                const uint4 v = acc4[c];
+                chk -= (long long)v.x + v.y + v.z + v.w - 4ll * kSumBias;
             }
-            // the next record of the warp is loaded while this one is added
-            PTile rn;
-            float wn = 1.f;
-            if (b + warp < e) {
-                rn = ld_tile(&sorted[b + warp]);
-                if (W) wn = __ldg(&wsorted[b + warp]);
+            for (int o = 16; o; o >>= 1) chk += __shfl_xor_sync(0xffffffffu, chk, o);
+            if ((threadIdx.x & 31) == 0) atomicAdd(&s_chk[par][gr], (unsigned long long)chk);
+        };
+        if constexpr (kShort) {
+            if (e - b <= kShortRecords) {
+                constexpr int NW = (G == 2 ? ARR : 0) + words(NI);
+                const bool few = e - b <= free_records(NI);
+                // the tile's cells in fours, f(words of the accumulator, place in the grid)
+                auto cells = [&](auto &&f) {
+                    for (int c = threadIdx.x; c < G * kTC / 4; c += blockDim.x) {
+                        const int gr = c / (kTC / 4), x = c % 4 * 4, y = c / 4 % kT, z = c / (4 * kT) % kT;
+                        f(acc4[(gr * ARR + ORG + z * PZ + y * kPy + x) / 4],
+                          reinterpret_cast<float4 *>((gr ? out2 : out1) + ((size_t)(oz + z) * N + (oy + y)) * N + ox + x));
+                    }
+                };
+                int flags = 0;
+                const long long tot =
+                    add_items<NI, G, W, false, SHORT>(b, e, 0, scale, bits, 0, sorted, wsorted, acc, flags, [&] {
+                        if (!few) {
+                            clear(NW, kSumBias);
+                            return;
+                        }
+                        cells([](uint4 &v, float4 *) { v = make_uint4(kSumBias, kSumBias, kSumBias, kSumBias); });
+                        __syncthreads();
+                    });
+                __syncthreads();
+                if (!few) compare(tot, NW, 2);
+                if (flags & kOut) s_bad[par][2] = 1;
+                cells([&](uint4 &v, float4 *o) {
+                    auto value = [&](unsigned s) {  // the sum, which ranges from -2^24 to beyond 2^31
+                        const unsigned d = s - kSumBias;
+                        return (s >= kSumBias ? __uint2float_rn(d) : __int2float_rn((int)d)) * inv_scale;
+                    };
+                    *o = make_float4(value(v.x), value(v.y), value(v.z), value(v.w));
+                });
+                __syncthreads();
+                if (s_chk[par][2] == 0ull && !s_bad[par][2]) continue;
+                // the first pass's sums wait in the grid
+                cells([&](uint4 &v, float4 *o) { *reinterpret_cast<uint4 *>(o) = v; });
+                __syncthreads();
+                add_items<NI, G, W, false, HIGH>(b, e, 0, scale, bits, 0, sorted, wsorted, acc, flags,
+                                                 [&] { clear(NW, 0u); });
+                __syncthreads();
+                cells([&](uint4 &v, float4 *o) {
+                    const uint4 low = *reinterpret_cast<const uint4 *>(o);
+                    auto value = [&](unsigned l, unsigned h) {
+                        const long long s = (long long)(int)h * 65536;
+                        return sfrac_to_float(s + (unsigned)(l - kSumBias - (unsigned)s)) * inv_scale *
+                               18446744073709551616.0f;  // 2^64
+                    };
+                    *o = make_float4(value(low.x, v.x), value(low.y, v.y), value(low.z, v.z), value(low.w, v.w));
+                });
+                __syncthreads();
+                continue;
             }
-            for (unsigned k = b + warp; k < e; k += nwarps) {
-                const PTile r = rn;
-                const float wt = wn;
-                if (k + nwarps < e) {
-                    rn = ld_tile(&sorted[k + nwarps]);
-                    if (W) wn = __ldg(&wsorted[k + nwarps]);
-                }
-                int cell[G][NIT];
-                long long q[G][NIT];
-                bool ok[G][NIT];
-#pragma unroll
-                for (int gr = 0; gr < G; gr++) {
-                    const int pk = r.g[gr].pack;
-                    const float hx = r.g[gr].h[0], hy = r.g[gr].h[1], hz = r.g[gr].h[2];
-#pragma unroll
-                    for (int it = 0; it < NIT; it++) {
-                        ok[gr][it] = (pk & need[it]) == need[it];
-                        // the reference's product order: ((w_x w_y) w_z) weight; wv * 2^S is exact in
-                        // FP32 (a power-of-two scale) and |wv| 2^S < 2^30, so q is one 32-bit integer
-                        float wv = horner(px[it], hx) * horner(py[it], hy) * horner(pz[it], hz);
-                        if (W) wv *= wt;
-                        q[gr][it] = GEN ? to_fixed(wv, bits) : (long long)__float2int_rn(wv);
-                        cell[gr][it] = (pk & ((1 << kMX) - 1)) + loff[it];
+        }
+        const int wx = GEN ? tile_origin<GEN>(tx + 1, g) - ox : kT, wy = GEN ? tile_origin<GEN>(ty + 1, g) - oy : kT,
+                  wz = GEN ? tile_origin<GEN>(tz + 1, g) - oz : kT;
+        const float s64 = inv_scale * 18446744073709551616.0f;  // 2^(64 - bits)
+        auto store = [&](int gr, auto &&sum) {
+            for (int c = threadIdx.x; c < kTC; c += blockDim.x) {
+                const int x = c % kT, y = (c / kT) % kT, z = c / (kT * kT);
+                if (GEN && (x >= wx || y >= wy || z >= wz)) continue;
+                const int pc = ORG + z * PZ + y * kPy + x;
+                (gr ? out2 : out1)[((size_t)(oz + z) * N + (oy + y)) * N + (ox + x)] =
+                    sfrac_to_float(sum(acc[pc], acc[pc + ARR])) * s64;
+            }
+            __syncthreads();
+        };
+        constexpr int NW = ARR + words(NI);
+        for (int gr = 0; gr < G; gr++) {
+            if constexpr (kPositive) {
+                if (lbits >= 0 && e - b <= kSplitRecords) {
+                    int flags = 0;
+                    const long long tot = add_items<NI, 1, W, GEN, SPLIT>(
+                        b, e, gr, GEN ? scale * ldexp_bits(-lbits) : scale, bits, lbits, sorted, wsorted, acc, flags,
+                        [&] { clear(NW, kSumBias); });
+                    __syncthreads();
+                    if (e - b > split_free) compare(tot, NW, gr);
+                    if (flags & kOut) s_bad[par][gr] = 1;
+                    __syncthreads();
+                    if (s_chk[par][gr] == 0ull && !s_bad[par][gr]) {
+                        store(gr, [&](unsigned lo, unsigned hi) {
+                            return ((long long)hi - kSumBias) * (1ll << lbits) + ((long long)lo - kSumBias);
+                        });
+                        continue;
                     }
                 }
-                // 64-bit fixed-point adds of the sign-extended q (exact mod 2^64)
-#pragma unroll
-                for (int gr = 0; gr < G; gr++)
-#pragma unroll
-                    for (int it = 0; it < NIT; it++)
-                        if (ok[gr][it])
-                            atomicAdd(acc64 + gr * kTCP + cell[gr][it], (unsigned long long)q[gr][it]);
             }
+            int flags = 0;
+            add_items<NI, 1, W, GEN, WIDE>(b, e, gr, GEN ? 1.f : scale, bits, 0, sorted, wsorted, acc, flags,
+                                           [&] { clear(NW, 0u); });
+            __syncthreads();
+            store(gr, [](unsigned lo, unsigned hi) { return (long long)((unsigned long long)hi << 32 | lo); });
         }
-        __syncthreads();
-        for (int c = threadIdx.x; c < G * kTC; c += blockDim.x) {
-            const int gr = c / kTC, cc = c % kTC;
-            const int x = cc % kT, y = (cc / kT) % kT, z = cc / (kT * kT);
-            if (GEN && (x >= tile_origin<GEN>(tx + 1, g) - ox || y >= tile_origin<GEN>(ty + 1, g) - oy ||
-                        z >= tile_origin<GEN>(tz + 1, g) - oz))
-                continue;
-            const int pc = z * kPz + y * kPy + x;
-            const long long v = (long long)acc64[gr * kTCP + pc];
-            float *out = gr ? out2 : out1;
-            out[((size_t)(oz + z) * N + (oy + y)) * N + (ox + x)] = (float)v * inv_scale;
-        }
-        __syncthreads();
     }
 }
 
 template <int NI, int G, bool W, bool IND, bool GEN>
-static int launch_tile_w(const TileGeom &g, const OwnerPtrs &ov, const OwnerPtrs *op, int bits, float *out1,
+static int launch_tile_w(const TileGeom &g, const OwnerPtrs &ov, const OwnerPtrs *op, int bits, int lbits, float *out1,
                          float *out2, cudaStream_t st) {
-    const size_t smem = sizeof(unsigned long long) * G * kTCP;
     auto kern = owner_tile_kernel<NI, G, W, IND, GEN>;
+    const size_t smem = tile_smem(NI);
     PBI4G_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int ntiles = g.nt * g.nt * g.nt;
     int per_sm = 0;
     PBI4G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem));
     const int grid = std::min(ntiles, 152 * std::max(1, per_sm));
-    kern<<<grid, kThreads, smem, st>>>(g, ov, op, GEN ? 1.0f : ldexpf(1.0f, bits), bits, ldexpf(1.0f, -bits), out1,
-                                       out2);
+    // parts are at most 2^lbits and 2^21 (GEN) or 2^(28 - lbits)
+    const unsigned split_free = lbits < 0 ? 0u : 0xFE000000u >> std::max(lbits, GEN ? 21 : 28 - lbits);
+    kern<<<grid, kThreads, smem, st>>>(g, ov, op, ldexpf(1.0f, bits), bits, lbits, split_free,
+                                        ldexpf(1.0f, -bits), out1, out2);
     PBI4G_LAUNCH_CHECK();
     return PBI4G_OK;
 }
 
 template <int NI, int G>
 static int launch_tile(const TileGeom &g, const OwnerPtrs &ov, const OwnerPtrs *op, bool weighted, int bits,
-                       float *out1, float *out2, cudaStream_t st) {
+                       int lbits, float *out1, float *out2, cudaStream_t st) {
     // the captured form takes no weights and only grids that are multiples of 16
-    if (op) return launch_tile_w<NI, G, false, true, false>(g, ov, op, bits, out1, out2, st);
+    if (op) return launch_tile_w<NI, G, false, true, false>(g, ov, op, bits, lbits, out1, out2, st);
     if (g.N % kT)
-        return weighted ? launch_tile_w<NI, G, true, false, true>(g, ov, op, bits, out1, out2, st)
-                        : launch_tile_w<NI, G, false, false, true>(g, ov, op, bits, out1, out2, st);
-    return weighted ? launch_tile_w<NI, G, true, false, false>(g, ov, op, bits, out1, out2, st)
-                    : launch_tile_w<NI, G, false, false, false>(g, ov, op, bits, out1, out2, st);
+        return weighted ? launch_tile_w<NI, G, true, false, true>(g, ov, op, bits, lbits, out1, out2, st)
+                        : launch_tile_w<NI, G, false, false, true>(g, ov, op, bits, lbits, out1, out2, st);
+    return weighted ? launch_tile_w<NI, G, true, false, false>(g, ov, op, bits, lbits, out1, out2, st)
+                    : launch_tile_w<NI, G, false, false, false>(g, ov, op, bits, lbits, out1, out2, st);
 }
 
 // zero the tile counts and the tile counter (through the pointer block)
@@ -782,6 +951,9 @@ int assign_owner(OwnerWork &wk, const void *d_ptrs, int N, int nintp, bool inter
         bits = std::min(bits, (int)floor(30.0 - log2(4.0 * (wmax > 0 ? wmax : 1.0))));
         if (bits < 8) return set_error(PBI4G_ERR_RANGE, "assign: particle weights up to %g", wmax);
     }
+    // other grids: 2^-bits in two parts, the upper one below 2^21 for the largest weight
+    const int hbits = std::min(bits, (int)floor(21.0 - log2(wmax > 0 ? wmax : 1.0)));
+    const int lbits = !gen ? std::min(bits, 14) : (bits - hbits <= 22 ? bits - hbits : -1);
     const int nt = (N + kT - 1) / kT, ntiles = nt * nt * nt;
     const TileGeom geo = {N, nt, 1.0f / (float)N, 1.0f / (float)nt};
     // few tiles: a block counts its share in shared memory, over about two blocks an SM
@@ -821,14 +993,14 @@ int assign_owner(OwnerWork &wk, const void *d_ptrs, int N, int nintp, bool inter
     pf.begin(tile_stage, st);
     int rc = PBI4G_OK;
     switch (nintp * 2 + (interlaced ? 1 : 0)) {
-        case 2: rc = launch_tile<1, 1>(geo, ov, op, wt, bits, out, o2, st); break;
-        case 3: rc = launch_tile<1, 2>(geo, ov, op, wt, bits, out, o2, st); break;
-        case 4: rc = launch_tile<2, 1>(geo, ov, op, wt, bits, out, o2, st); break;
-        case 5: rc = launch_tile<2, 2>(geo, ov, op, wt, bits, out, o2, st); break;
-        case 6: rc = launch_tile<3, 1>(geo, ov, op, wt, bits, out, o2, st); break;
-        case 7: rc = launch_tile<3, 2>(geo, ov, op, wt, bits, out, o2, st); break;
-        case 8: rc = launch_tile<4, 1>(geo, ov, op, wt, bits, out, o2, st); break;
-        default: rc = launch_tile<4, 2>(geo, ov, op, wt, bits, out, o2, st); break;
+        case 2: rc = launch_tile<1, 1>(geo, ov, op, wt, bits, lbits, out, o2, st); break;
+        case 3: rc = launch_tile<1, 2>(geo, ov, op, wt, bits, lbits, out, o2, st); break;
+        case 4: rc = launch_tile<2, 1>(geo, ov, op, wt, bits, lbits, out, o2, st); break;
+        case 5: rc = launch_tile<2, 2>(geo, ov, op, wt, bits, lbits, out, o2, st); break;
+        case 6: rc = launch_tile<3, 1>(geo, ov, op, wt, bits, lbits, out, o2, st); break;
+        case 7: rc = launch_tile<3, 2>(geo, ov, op, wt, bits, lbits, out, o2, st); break;
+        case 8: rc = launch_tile<4, 1>(geo, ov, op, wt, bits, lbits, out, o2, st); break;
+        default: rc = launch_tile<4, 2>(geo, ov, op, wt, bits, lbits, out, o2, st); break;
     }
     pf.end(st);
     PBI4G_CHECK(rc);

@@ -56,7 +56,10 @@ def _low(d):
     (32, 4, True, False, 700), (34, 4, True, False, 3001), (34, 1, False, True, 3001), (34, 3, True, True, 2000),
     (46, 2, False, False, 4000), (48, 2, True, True, 1), (50, 4, False, True, 5000), (62, 2, True, False, 9),
     (66, 1, True, False, 6000), (100, 3, False, False, 20000), (126, 4, True, True, 30000), (194, 4, True, False, 40000),
-    (202, 3, True, True, 30000), (208, 2, False, False, 40000)])
+    (202, 3, True, True, 30000), (208, 2, False, False, 40000), (208, 4, True, False, 200000), (64, 1, True, False, 30000),
+    (64, 2, True, True, 30000), (64, 3, False, True, 30000), (96, 3, True, False, 9000), (96, 4, False, False, 9000),
+    (32, 2, True, False, 400000), (32, 4, True, True, 150000), (50, 4, True, False, 200000), (98, 3, False, True, 400000),
+    (66, 1, True, True, 300000), (34, 2, True, False, 200000), (124, 4, True, True, 300000)])
 def test_tiles_vs_global_grid(grid, nintp, interlacing, weights, npart):
     pos = _particles(max(npart, 8), grid, grid + nintp)[:, :npart].copy()
     w = np.random.default_rng(grid).uniform(-0.5, 2.0, npart) if weights else None
