@@ -896,7 +896,8 @@ void OwnerWork::release() {
 
 size_t OwnerWork::footprint(int N, int64_t npart) {
     const size_t nt = (size_t)((N + kT - 1) / kT);
-    return 3 * (nt * nt * nt + 2) * 4 + (size_t)npart * 8 * (sizeof(PTile) + 4) + 64;
+    // (32 bytes a particle more than ensure takes: callers have their budgets from this size)
+    return 3 * (nt * nt * nt + 2) * 4 + (size_t)npart * (32 + 8 * (sizeof(PTile) + 4)) + 64;
 }
 
 void owner_ptrs_host(const OwnerWork &wk, unsigned char (&block)[kOwnerPtrBytes]) {
