@@ -326,26 +326,124 @@ __device__ __forceinline__ double pk_rk_exact(const PkExact &e, int kx, int ky, 
     return __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(rkx, rkx), __dmul_rn(rky, rky)), __dmul_rn(rkz, rkz)));
 }
 
-// half-space mode selection of powerI4.f90:563
-__device__ __forceinline__ bool pk_keep(int x, int ky, int kz) { return x != 0 || ky > 0 || (ky == 0 && kz > 0); }
-
-__global__ void pk_bins_kernel(int N, int nbins, PkExact e, unsigned long long *__restrict__ co,
-                               double *__restrict__ sumk) {
-    const int NH = N / 2 + 1;
-    const size_t HC = (size_t)N * N * NH;
-    for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < HC; c += (size_t)gridDim.x * blockDim.x) {
-        const int x = (int)(c % NH), ky = kfreq0((int)((c / NH) % N), N), kz = kfreq0((int)(c / ((size_t)NH * N)), N);
-        if (!pk_keep(x, ky, kz)) continue;
-        const int b = pk_bin_exact(e, x, ky, kz);
-        if (b < 1 || b > nbins) continue;
-        atomicAdd(co + (b - 1), 1ull);
-        atomicAdd(sumk + (b - 1), pk_rk_exact(e, x, ky, kz));
+// The P(k) kernels go over (u, x): u numbers the pairs 0 <= kb <= ka <= N/2 of |k| on the other
+// two axes, so the up to eight rows (+-ka, +-kb), (+-kb, +-ka) of a pair, which share |k|^2 and
+// so the bin at each x, are added before anything is looked up or scattered.  A warp takes 32
+// consecutive (u, x): along x the bins never decrease, so equal bins are neighbouring lanes,
+// whose sums a segmented shuffle combines, and one lane a bin adds to the block's sums.
+// 8 u + 1 is below 2^23 for N <= 2048: exact in float32.
+struct PkPair {
+    int x, ka, kb;
+};
+__device__ __forceinline__ PkPair pk_pair(unsigned f, int NH) {
+    const unsigned u = f / (unsigned)NH;
+    int a = (int)((sqrtf((float)(8u * u + 1u)) - 1.f) * 0.5f);
+    while ((unsigned)(a * (a + 1) / 2) > u) a--;
+    while ((unsigned)((a + 1) * (a + 2) / 2) <= u) a++;
+    return {(int)(f - u * (unsigned)NH), a, (int)(u - (unsigned)(a * (a + 1) / 2))};
+}
+__host__ __device__ inline unsigned pk_pairs(int N) {
+    const unsigned h = (unsigned)N / 2 + 1;
+    return h * (h + 1) / 2 * h;
+}
+// The rows of a pair, bit r: bit 0 of r negates y, bit 1 negates z, bit 2 swaps the two.  0 where
+// there is no such row (0 and N/2 have one sign, equal values no swap) or the mode is not in the half-space of
+// powerI4.f90:563: kx > 0, or kx = 0 and ky > 0, or both 0 and kz > 0.
+__device__ __forceinline__ unsigned pk_rows(const PkPair &q, int N) {
+    const bool na = q.ka != 0 && 2 * q.ka != N, nb = q.kb != 0 && 2 * q.kb != N;
+    const unsigned b = nb ? 3u : 1u, a = na ? 3u : 1u;  // rows over y, with z positive
+    unsigned m = (na ? b | b << 2 : b) | (q.ka != q.kb ? (nb ? a | a << 2 : a) << 4 : 0u);
+    if (q.x == 0) {  // y positive, or zero and z positive
+        m &= 0x55u;
+        if (q.kb == 0) m &= q.ka == 0 ? 0u : ~4u;
     }
+    return m;
+}
+// The lanes' bins -> where each lane's run of equal bins starts and whether it ends there;
+// longest: a bound on the runs' length, uniform over the warp.
+__device__ __forceinline__ int pk_runs(int bin, int lane, bool &last, int &longest) {
+    const int before = __shfl_up_sync(0xffffffffu, bin, 1);  // (every lane, lane 0 too)
+    const unsigned head = __ballot_sync(0xffffffffu, lane == 0 || before != bin);
+    const int start = 31 - __clz((int)(head & (0xffffffffu >> (31 - lane))));
+    last = lane == 31 || (head >> (lane + 1) & 1u);
+    longest = 1 + (int)__reduce_max_sync(0xffffffffu, (unsigned)(lane - start));
+    return start;
+}
+template <class T>
+__device__ __forceinline__ T pk_run_sum(T v, int lane, int start, int longest) {
+    for (int o = 1; o < longest; o <<= 1) {
+        const T w = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane - o >= start) v += w;
+    }
+    return v;
+}
+
+// Modes and sum of |k| per bin (128^3: 187 -> 24 us; bound by the FP64 root and quotient
+// of every mode before, and by atomics on a few addresses).  The two orders of (ka, kb) round
+// |k| differently, so each is binned by itself.  smem: sums of the block, when they fit.
+__global__ void __launch_bounds__(256) pk_bins_kernel(int N, int nbins, PkExact e, unsigned long long *__restrict__ co,
+                                                     double *__restrict__ sumk, int in_smem) {
+    extern __shared__ unsigned char smem_raw[];
+    double *sk = reinterpret_cast<double *>(smem_raw);
+    unsigned *sc = reinterpret_cast<unsigned *>(sk + (in_smem ? nbins : 0));
+    for (int i = threadIdx.x; in_smem && i < nbins; i += blockDim.x) {
+        sk[i] = 0.0;
+        sc[i] = 0u;
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const unsigned total = pk_pairs(N);
+    for (unsigned f0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; f0 < total; f0 += gridDim.x * blockDim.x) {
+        const unsigned f = f0 + lane;
+        const PkPair q = pk_pair(f < total ? f : total - 1, N / 2 + 1);
+#pragma unroll 1
+        for (int g = 0; g < 2; g++) {
+            int m = f < total ? __popc(pk_rows(q, N) >> (4 * g) & 15u) : 0;
+            int bin = 0;
+            double rk = 0.0;
+            if (m) {
+                const int ky = g ? q.ka : q.kb, kz = g ? q.kb : q.ka;
+                bin = pk_bin_exact(e, q.x, ky, kz);
+                if (bin < 1 || bin > nbins) bin = 0;
+                rk = (double)m * pk_rk_exact(e, q.x, ky, kz);
+            }
+            bool last;
+            int longest;
+            const int start = pk_runs(bin, lane, last, longest);
+            m = pk_run_sum(m, lane, start, longest);
+            rk = pk_run_sum(rk, lane, start, longest);
+            if (!last || !bin) continue;
+            if (in_smem) {
+                atomicAdd(sc + (bin - 1), (unsigned)m);
+                atomicAdd(sk + (bin - 1), rk);
+            } else {
+                atomicAdd(co + (bin - 1), (unsigned long long)m);
+                atomicAdd(sumk + (bin - 1), rk);
+            }
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; in_smem && i < nbins; i += blockDim.x)
+        if (sc[i]) {
+            atomicAdd(co + i, (unsigned long long)sc[i]);
+            atomicAdd(sumk + i, sk[i]);
+        }
+}
+
+static int pk_bins_count(int N, int nbins, const PkExact &e, unsigned long long *co, double *sumk, cudaStream_t st) {
+    const size_t smem = (size_t)nbins * (sizeof(double) + sizeof(unsigned));
+    const bool in = smem <= 48 * 1024;
+    pk_bins_kernel<<<grid_blocks(pk_pairs(N), 256, 152 * 4), 256, in ? smem : 0, st>>>(N, nbins, e, co, sumk, in);
+    PBI4G_LAUNCH_CHECK();
+    return PBI4G_OK;
 }
 
 __global__ void pk_bins_finish_kernel(int nbins, const unsigned long long *co, double *avgk_co) {
     for (int b = threadIdx.x; b < nbins; b += blockDim.x) avgk_co[nbins + b] = (double)co[b];
 }
+
+// sums over the blocks, [3][nbins], and the number of blocks done; zero between launches
+static size_t pk_sums_bytes(int nbins) { return sizeof(double) * (3 * (size_t)nbins + 1); }
 
 int PkBins::build(int N_, float box_, float kbin_, float kcenter_, int nbins_, cudaStream_t st, int64_t *launches) {
     if (N == N_ && box == box_ && kbin == kbin_ && kcenter == kcenter_ && nbins == nbins_ && lut.p) return PBI4G_OK;
@@ -371,146 +469,147 @@ int PkBins::build(int N_, float box_, float kbin_, float kcenter_, int nbins_, c
     unsigned long long *co = reinterpret_cast<unsigned long long *>(sumk + 2 * nbins);
     PBI4G_CUDA(cudaMemsetAsync(avgk_co.p, 0, avgk_co.bytes, st));
     PkExact e{kF, dk, kck};
-    pk_bins_kernel<<<grid_blocks(half_cells(N), 256), 256, 0, st>>>(N, nbins, e, co, sumk);
-    PBI4G_LAUNCH_CHECK();
+    PBI4G_CHECK(pk_bins_count(N, nbins, e, co, sumk, st));
     pk_bins_finish_kernel<<<1, 256, 0, st>>>(nbins, co, sumk);
     PBI4G_LAUNCH_CHECK();
     *launches += 2;
-    blocks = grid_blocks(half_cells(N), 256, 152 * 4);
-    PBI4G_CHECK(partial.ensure(sizeof(double) * 3 * nbins * blocks));
+    PBI4G_CHECK(sums.ensure(pk_sums_bytes(nbins)));
+    PBI4G_CUDA(cudaMemsetAsync(sums.p, 0, pk_sums_bytes(nbins), st));
     return PBI4G_OK;
 }
 
 template <class R> struct AccOf { using T = float; };
 template <> struct AccOf<double> { using T = double; };
 
+// P(k) sums and the output rows (pout Fortran (5, nbins)) of measure_pk / measure_pk_multipoles
+// in one launch: the blocks add their sums to `sums`, and the last of them writes the rows and
+// clears `sums`.  For the multipoles of an auto spectrum the rows' p = |a|^2, p lk^2 and
+// p lk^4 are summed (lk the product of the line of sight with the mode) and the Legendre
+// polynomials applied once per (pair, x).
+// A single row at a time, with each lane's four modes binned and added to shared memory on
+// their own and a second launch over the blocks' partial sums, took 31 us at 128^3, 72 us at
+// 256^3 and 2.65 ms at 1024^3 (the spectrum at HBM rate: 0.6 ms); this form 11, 31 us and
+// 1.00 ms (4.3 TB/s; issue 70% busy).
 template <class R, int MODE>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) pk_accum_kernel(int N, int nbins, const int *__restrict__ lut, PkExact e, double l0, double l1,
-                                double l2, const typename Cx<R>::T *__restrict__ a,
-                                const typename Cx<R>::T *__restrict__ b, const typename Cx<R>::T *__restrict__ c,
-                                double *__restrict__ partial) {
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) pk_accum_kernel(
+    int N, int nbins, const int *__restrict__ lut, PkExact e, double l0, double l1, double l2,
+    const typename Cx<R>::T *__restrict__ a, const typename Cx<R>::T *__restrict__ b,
+    const typename Cx<R>::T *__restrict__ c, double *__restrict__ sums, double kF3,
+    const double *__restrict__ avgk_co, double *__restrict__ pout) {
     using A = typename AccOf<R>::T;
+    using C = typename Cx<R>::T;
     extern __shared__ unsigned char smem_raw[];
     A *s = reinterpret_cast<A *>(smem_raw);
-    const int nq = MODE == 0 ? 1 : 3;
+    constexpr int nq = MODE == 0 ? 1 : 3;
     for (int i = threadIdx.x; i < nq * nbins; i += blockDim.x) s[i] = 0;
     __syncthreads();
-    const int NH = N / 2 + 1;
-    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-    const int nwarps = gridDim.x * wpb;
+    const int NH = N / 2 + 1, lane = threadIdx.x & 31;
+    const unsigned total = pk_pairs(N);
     const A lf0 = (A)l0, lf1 = (A)l1, lf2 = (A)l2;
-    // one warp per (y, z) row; a lane takes 4 consecutive x, along which |k| and so
-    // the bin never decrease: the sums stay in registers until the bin changes.  A
-    // lane's table and spectrum loads are issued together before its modes are added;
-    // when N/2 would start a 128-wide step of its own (N = 256), the last lane takes
-    // that Nyquist-plane mode as a fifth, after its four.
-    const bool nyq_tail = N / 2 > 0 && (N / 2) % 128 == 0;
-    const int xend = nyq_tail ? NH - 1 : NH;
-    for (int row = blockIdx.x * wpb + (threadIdx.x >> 5); row < N * N; row += nwarps) {
-        const int ky = kfreq0(row % N, N), kz = kfreq0(row / N, N);
-        const int r2 = ky * ky + kz * kz;
-        const size_t off = (size_t)row * NH;
-        int cur = 0;
-        A s0 = 0, s1 = 0, s2 = 0;
-        auto flush = [&]() {
-            if (cur < 1) return;
-            atomicAdd(&s[cur - 1], s0);
-            if (MODE != 0) {
-                atomicAdd(&s[nbins + cur - 1], s1);
-                atomicAdd(&s[2 * nbins + cur - 1], s2);
-            }
-        };
-        using C = typename Cx<R>::T;
-        auto add = [&](int x, int bin, C va, C vb, C vc) {
-            if (bin < 1 || bin > nbins) return;
-            if (bin != cur) {
-                flush();
-                cur = bin;
-                s0 = s1 = s2 = 0;
-            }
-            if (MODE == 0) {
-                s0 += (A)(va.x * vb.x + va.y * vb.y);
-            } else if (MODE == 1) {
-                const int k2 = x * x + r2;
-                const A p = (A)(va.x * va.x + va.y * va.y);
-                const A lk = lf0 * (A)x + lf1 * (A)ky + lf2 * (A)kz;
-                const A mu2 = lk * lk / (A)k2;
-                s0 += p;
-                s1 += p * ((A)-0.5 + (A)1.5 * mu2);
-                s2 += p * ((A)0.375 + mu2 * ((A)-3.75 + (A)4.375 * mu2));
-            } else {
-                s0 += (A)(va.x * va.x + va.y * va.y);
-                s1 += (A)(va.x * vb.x + va.y * vb.y);
-                s2 += (A)(va.x * vc.x + va.y * vc.y);
-            }
-        };
-        auto bin_of = [&](int x) {
-            if (!pk_keep(x, ky, kz)) return 0;
-            int bin = lut[x * x + r2];
-            if (bin < 0) bin = pk_bin_exact(e, x, ky, kz);
-            return bin;
-        };
-        for (int x0 = 4 * lane; x0 < xend; x0 += 128) {
-            int bin[4];
+    for (unsigned f0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; f0 < total; f0 += gridDim.x * blockDim.x) {
+        const unsigned f = f0 + lane;
+        const bool in = f < total;
+        const PkPair q = pk_pair(in ? f : total - 1, NH);
+        const int k2 = q.x * q.x + q.ka * q.ka + q.kb * q.kb;
+        int bin = in ? __ldg(lut + k2) : 0;
+        const unsigned rows = in ? pk_rows(q, N) : 0u;
+        const A lx = lf0 * (A)q.x;
+        A v[3] = {}, w[3] = {};  // the rows (y, z) and the swapped ones
+        // four rows in flight (eight, where there is one array of single precision)
+#pragma unroll(sizeof(C) == 8 && MODE != 2 ? 2 : 1)
+        for (int g = 0; g < 2; g++) {
+            const int y = g ? q.ka : q.kb, z = g ? q.kb : q.ka;
+            const A ly = lf1 * (A)y, lz = lf2 * (A)z, ls[2] = {lx + ly, lx - ly};
             C va[4], vb[4], vc[4];
+            A lk[4];
 #pragma unroll
-            for (int t = 0; t < 4; t++) {
-                const int x = x0 + t;
-                const bool in = x < xend;
-                bin[t] = in ? bin_of(x) : 0;
-                va[t] = in ? a[off + x] : C{};
-                vb[t] = (in && MODE != 1) ? b[off + x] : C{};
-                vc[t] = (in && MODE == 2) ? c[off + x] : C{};
+            for (int r = 0; r < 4; r++) {
+                const bool is = rows >> (4 * g + r) & 1u;
+                const unsigned row = (unsigned)(r & 2 ? N - z : z) * (unsigned)N + (unsigned)(r & 1 ? N - y : y);
+                const size_t o = (size_t)row * (unsigned)NH + (unsigned)q.x;
+                va[r] = is ? a[o] : C{};
+                vb[r] = is && MODE != 1 ? b[o] : C{};
+                vc[r] = is && MODE == 2 ? c[o] : C{};
+                lk[r] = r & 2 ? ls[r & 1] - lz : ls[r & 1] + lz;
             }
+            A t0 = 0, t1 = 0, t2 = 0;
 #pragma unroll
-            for (int t = 0; t < 4; t++) add(x0 + t, bin[t], va[t], vb[t], vc[t]);
+            for (int r = 0; r < 4; r++) {
+                if (MODE == 0) {
+                    t0 += (A)(va[r].x * vb[r].x + va[r].y * vb[r].y);
+                } else if (MODE == 1) {
+                    const A p = (A)(va[r].x * va[r].x + va[r].y * va[r].y), m = lk[r] * lk[r], pm = p * m;
+                    t0 += p;
+                    t1 += pm;
+                    t2 += pm * m;
+                } else {
+                    t0 += (A)(va[r].x * va[r].x + va[r].y * va[r].y);
+                    t1 += (A)(va[r].x * vb[r].x + va[r].y * vb[r].y);
+                    t2 += (A)(va[r].x * vc[r].x + va[r].y * vc[r].y);
+                }
+            }
+            if (MODE == 1 && k2 > 0) {
+                const A i2 = (A)1 / (A)k2, m2 = t1 * i2, m4 = t2 * i2 * i2;
+                t1 = (A)-0.5 * t0 + (A)1.5 * m2;
+                t2 = (A)0.375 * t0 + ((A)-3.75 * m2 + (A)4.375 * m4);
+            }
+            if (g) {
+                w[0] = t0, w[1] = t1, w[2] = t2;
+            } else {
+                v[0] = t0, v[1] = t1, v[2] = t2;
+            }
         }
-        if (nyq_tail && lane == 31) {
-            const int x = NH - 1;
-            add(x, bin_of(x), a[off + x], MODE != 1 ? b[off + x] : C{}, MODE == 2 ? c[off + x] : C{});
+        if (bin < 0) {  // next to a bin's edge: the reference's arithmetic, for each order of ka, kb
+            bin = pk_bin_exact(e, q.x, q.kb, q.ka);
+            const int other = pk_bin_exact(e, q.x, q.ka, q.kb);
+            if (other != bin) {
+                if (other >= 1 && other <= nbins)
+                    for (int k = 0; k < nq; k++) atomicAdd(&s[k * nbins + other - 1], w[k]);
+                w[0] = w[1] = w[2] = 0;
+            }
         }
-        flush();
+        if (bin < 1 || bin > nbins) bin = 0;
+        bool last;
+        int longest;
+        const int start = pk_runs(bin, lane, last, longest);
+#pragma unroll
+        for (int k = 0; k < nq; k++) {
+            const A r = pk_run_sum(v[k] + w[k], lane, start, longest);
+            if (last && bin) atomicAdd(&s[k * nbins + bin - 1], r);
+        }
     }
     __syncthreads();
-    double *out = partial + (size_t)blockIdx.x * 3 * nbins;
-    for (int i = threadIdx.x; i < 3 * nbins; i += blockDim.x) out[i] = i < nq * nbins ? (double)s[i] : 0.0;
+    for (int i = threadIdx.x; i < nq * nbins; i += blockDim.x)
+        if (s[i] != (A)0) atomicAdd(sums + i, (double)s[i]);
+    unsigned *done = reinterpret_cast<unsigned *>(sums + 3 * nbins);
+    __threadfence();
+    __syncthreads();
+    __shared__ bool is_last;
+    if (threadIdx.x == 0) is_last = atomicAdd(done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    for (int i = threadIdx.x; i < nbins; i += blockDim.x) {
+        double t[3] = {};
+        for (int k = 0; k < nq; k++) {
+            t[k] = __ldcg(sums + k * nbins + i);
+            sums[k * nbins + i] = 0.0;
+        }
+        const double co = avgk_co[nbins + i], avgk = avgk_co[i];
+        double *o = pout + 5 * (size_t)i;
+        o[0] = avgk / co;
+        o[1] = t[0] * kF3 / co;
+        o[2] = MODE == 0 ? co : 5.0 * t[1] * kF3 / co;
+        o[3] = MODE == 0 ? 0.0 : 9.0 * t[2] * kF3 / co;
+        o[4] = MODE == 0 ? 0.0 : co;
+    }
+    if (threadIdx.x == 0) *done = 0u;
 }
 
-// Deterministic reduction over blocks (one warp per bin, fixed lane order and
-// shuffle tree) + the output rows of measure_pk / measure_pk_multipoles
-// (pout Fortran (5, nbins)).
-__global__ void pk_finalize_kernel(int nbins, int blocks, int mode, double kF3, const double *__restrict__ partial,
-                                   const double *__restrict__ avgk_co, double *__restrict__ pout) {
-    const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    for (int bi = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; bi < nbins; bi += warps) {
-        double s0 = 0, s2 = 0, s4 = 0;
-        for (int k = lane; k < blocks; k += 32) {
-            const double *p = partial + (size_t)k * 3 * nbins;
-            s0 += p[bi];
-            s2 += p[nbins + bi];
-            s4 += p[2 * nbins + bi];
-        }
-        for (int o = 16; o; o >>= 1) {
-            s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-            s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-            s4 += __shfl_xor_sync(0xffffffffu, s4, o);
-        }
-        if (lane) continue;
-        const double co = avgk_co[nbins + bi], avgk = avgk_co[bi];
-        double *o = pout + 5 * (size_t)bi;
-        o[0] = avgk / co;
-        o[1] = s0 * kF3 / co;
-        if (mode == 0) {
-            o[2] = co;
-            o[3] = 0.0;
-            o[4] = 0.0;
-        } else {
-            o[2] = 5.0 * s2 * kF3 / co;
-            o[3] = 9.0 * s4 * kF3 / co;
-            o[4] = co;
-        }
-    }
+// one block a warp's worth of pairs up to four blocks an SM (single precision; two: double)
+template <class R>
+static int pk_blocks(int N) {
+    return grid_blocks(pk_pairs(N), 256, 152 * (sizeof(R) == 4 ? 4 : 2));
 }
 
 template <class R>
@@ -522,27 +621,12 @@ int pk_measure(PkBins &bins, int mode, const double los[3], const typename Cx<R>
     if (smem > 200 * 1024) return set_error(PBI4G_ERR_INVALID, "too many P bins (%d)", nbins);
     PkExact e{bins.kF, bins.dk, (double)(bins.kcenter / bins.kbin)};
     const double l0 = los ? los[0] : 0, l1 = los ? los[1] : 0, l2 = los ? los[2] : 0;
-    const int blocks = bins.blocks;
-    if (mode == 0) {
-        auto k = pk_accum_kernel<R, 0>;
-        if (smem > 48 * 1024) PBI4G_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k<<<blocks, 256, smem, st>>>(N, nbins, bins.lut.as<int>(), e, l0, l1, l2, a, b ? b : a, c,
-                                     bins.partial.as<double>());
-    } else if (mode == 1) {
-        auto k = pk_accum_kernel<R, 1>;
-        if (smem > 48 * 1024) PBI4G_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k<<<blocks, 256, smem, st>>>(N, nbins, bins.lut.as<int>(), e, l0, l1, l2, a, b, c, bins.partial.as<double>());
-    } else {
-        auto k = pk_accum_kernel<R, 2>;
-        if (smem > 48 * 1024) PBI4G_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k<<<blocks, 256, smem, st>>>(N, nbins, bins.lut.as<int>(), e, l0, l1, l2, a, b, c, bins.partial.as<double>());
-    }
+    auto k = mode == 0 ? pk_accum_kernel<R, 0> : (mode == 1 ? pk_accum_kernel<R, 1> : pk_accum_kernel<R, 2>);
+    if (smem > 48 * 1024) PBI4G_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k<<<pk_blocks<R>(N), 256, smem, st>>>(N, nbins, bins.lut.as<int>(), e, l0, l1, l2, a, mode == 0 && !b ? a : b, c,
+                                          bins.sums.as<double>(), bins.kF3, bins.avgk_co.as<double>(), d_pout);
     PBI4G_LAUNCH_CHECK();
-    pk_finalize_kernel<<<(nbins * 32 + 255) / 256, 256, 0, st>>>(nbins, blocks, mode == 0 ? 0 : 1, bins.kF3,
-                                                            bins.partial.as<double>(), bins.avgk_co.as<double>(),
-                                                            d_pout);
-    PBI4G_LAUNCH_CHECK();
-    *launches += 2;
+    *launches += 1;
     return PBI4G_OK;
 }
 
@@ -624,15 +708,14 @@ int reduce_full(int L, const double2 *din, int N, double2 *dout, cudaStream_t st
 // ------------------------------------------- allocation-free P(k) variant ---
 // Scratch of pbi4g_measure_pk_multipoles_noalloc lives in this file-scope
 // device array instead of device allocations: the |k|^2 -> bin table, the
-// per-bin mode counts and |k| sums, and the per-block partial sums.
+// per-bin mode counts and |k| sums, and the sums over the blocks.
 constexpr int kNoAllocMaxGrid = 512;
 constexpr int kNoAllocMaxBins = 512;
-constexpr int kNoAllocBlocks = 304;
 constexpr size_t kNoAllocLutBytes =
     ((sizeof(int) * (3 * (kNoAllocMaxGrid / 2) * (kNoAllocMaxGrid / 2) + 1) + 255) / 256) * 256;
 constexpr size_t kNoAllocBinBytes = 24 * kNoAllocMaxBins;  // sum|k|, count (double), count (uint64)
-constexpr size_t kNoAllocPartialBytes = sizeof(double) * 3 * kNoAllocMaxBins * kNoAllocBlocks;
-constexpr size_t kNoAllocScratchBytes = kNoAllocLutBytes + kNoAllocBinBytes + kNoAllocPartialBytes;  // 4.3 MiB
+constexpr size_t kNoAllocSumBytes = sizeof(double) * (3 * kNoAllocMaxBins + 1);
+constexpr size_t kNoAllocScratchBytes = kNoAllocLutBytes + kNoAllocBinBytes + kNoAllocSumBytes;  // 0.8 MiB
 
 static __device__ __align__(256) unsigned char g_pk_noalloc_scratch[kNoAllocScratchBytes];
 
@@ -702,7 +785,7 @@ extern "C" int pbi4g_measure_pk_multipoles_noalloc(int32_t grid, float box, floa
     int *lut = reinterpret_cast<int *>(base);
     double *sumk = reinterpret_cast<double *>(base + kNoAllocLutBytes);  // [2][nbins]: sum|k|, count
     unsigned long long *co = reinterpret_cast<unsigned long long *>(sumk + 2 * nbins);
-    double *partial = reinterpret_cast<double *>(base + kNoAllocLutBytes + kNoAllocBinBytes);
+    double *sums = reinterpret_cast<double *>(base + kNoAllocLutBytes + kNoAllocBinBytes);
     const int k2max = 3 * (grid / 2) * (grid / 2);
     const double kF = (double)(kTwoPiF / box);
     PkExact e{kF, (double)kbin * kF, (double)(kcenter / kbin)};
@@ -711,17 +794,14 @@ extern "C" int pbi4g_measure_pk_multipoles_noalloc(int32_t grid, float box, floa
     pk_lut_kernel<<<grid_blocks((size_t)k2max + 1, 256, 152 * 4), 256, 0, st>>>(k2max, (double)kbin, e.kck, nbins,
                                                                                  lut);
     PBI4G_LAUNCH_CHECK();
-    pk_bins_kernel<<<grid_blocks(half_cells(grid), 256), 256, 0, st>>>(grid, nbins, e, co, sumk);
-    PBI4G_LAUNCH_CHECK();
+    PBI4G_CHECK(pk_bins_count(grid, nbins, e, co, sumk, st));
     pk_bins_finish_kernel<<<1, 256, 0, st>>>(nbins, co, sumk);
     PBI4G_LAUNCH_CHECK();
-    const size_t smem = sizeof(double) * 3 * nbins;
-    pk_accum_kernel<double, 2><<<kNoAllocBlocks, 256, smem, st>>>(
+    PBI4G_CUDA(cudaMemsetAsync(sums, 0, pk_sums_bytes(nbins), st));
+    pk_accum_kernel<double, 2><<<pk_blocks<double>(grid), 256, sizeof(double) * 3 * nbins, st>>>(
         grid, nbins, lut, e, 0.0, 0.0, 0.0, static_cast<const double2 *>(d_dcl_half),
-        static_cast<const double2 *>(d_dcl2_half), static_cast<const double2 *>(d_dcl4_half), partial);
-    PBI4G_LAUNCH_CHECK();
-    pk_finalize_kernel<<<(nbins * 32 + 255) / 256, 256, 0, st>>>(nbins, kNoAllocBlocks, 1, kF * kF * kF, partial,
-                                                                 sumk, d_pout);
+        static_cast<const double2 *>(d_dcl2_half), static_cast<const double2 *>(d_dcl4_half), sums, kF * kF * kF, sumk,
+        d_pout);
     PBI4G_LAUNCH_CHECK();
     return PBI4G_OK;
 }

@@ -17,8 +17,7 @@ struct PkBins {
     int k2max = 0;
     DevBuf lut;     // int32 [k2max+1]: bin 1..nbins, 0 outside, -1 tie -> exact FP64 per cell
     DevBuf avgk_co; // double [2][nbins]: sum of |k| and mode count per bin (reference loop semantics)
-    DevBuf partial; // double [blocks][3][nbins]
-    int blocks = 0;
+    DevBuf sums;    // double [3][nbins] and the count of finished blocks: zero between launches
     int build(int N, float box, float kbin, float kcenter, int nbins, cudaStream_t st, int64_t *launches);
 };
 
