@@ -25,11 +25,11 @@
 // 67% busy with two operations a coordinate; issue 54%), scatter 75 us (issue 62%).
 // With prepared particles written by the count and read back by the scatter, and
 // the cells from FP64 arithmetic, the two took 154 us.
-// The tiles are bound by instruction issue (74% at 2 10^6 random particles in 256^3, 271 us;
-// 61 instructions a record of two grids) and next by the shared atomics; in dense boxes the
+// The tiles are bound by instruction issue (67% at 2 10^6 random particles in 256^3, 258 us;
+// 54 instructions a record of two grids) and next by the shared atomics; in dense boxes the
 // other way round.  Of the 483 us before, with 64-bit atomics on the cells inside the tile, the
 // tests of every cell, its branch and coefficients reloaded for want of registers took half.
-// Boxes of few particles are bound by clearing and storing the tiles (512^3: 376 us, 158 of
+// Boxes of few particles are bound by clearing and storing the tiles (512^3: 393 us, 158 of
 // them the grids at HBM rate).
 #include "assign_owner.cuh"
 #include "fixed.cuh"
@@ -133,28 +133,6 @@ __device__ __forceinline__ float4 axis_poly(int i) {
     }
 }
 
-// All weights of an axis: no FP32 rounding makes any of them negative inside the box.
-template <int NI>
-__device__ __forceinline__ void axis_weights(float h, float (&w)[NI]) {
-    if constexpr (NI == 4) {
-        const float u = 1.f - h, h2 = h * h, u2 = u * u;
-        w[0] = u * (1.f / 6.f) * u2;
-        w[1] = fmaf(fmaf(h, 0.5f, -1.f), h2, 2.f / 3.f);
-        w[2] = fmaf(fmaf(u, 0.5f, -1.f), u2, 0.66666663f);  // 2/3 rounded down: the two errors cancel in the sum
-        w[3] = h * (1.f / 6.f) * h2;
-    } else if constexpr (NI == 3) {
-        const float a = 0.5f - h, c = 0.5f + h;
-        w[0] = 0.5f * a * a;
-        w[1] = fmaf(-h, h, 0.75f);
-        w[2] = 0.5f * c * c;
-    } else if constexpr (NI == 2) {
-        w[0] = 1.f - h;
-        w[1] = h;
-    } else {
-        w[0] = 1.f;
-    }
-}
-
 // two float32 in one 64-bit register, and their packed multiply and multiply-add
 using F2 = unsigned long long;
 __device__ __forceinline__ F2 f2(float lo, float hi) {
@@ -175,6 +153,34 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
     return r;
 }
 __device__ __forceinline__ F2 horner2(const F2 c[4], F2 h) { return fma2(h, fma2(h, fma2(h, c[3], c[2]), c[1]), c[0]); }
+
+// s times all weights of an axis, by pairs (every operation rounds as the single one does): no
+// FP32 rounding makes any of them negative inside the box.
+template <int NI>
+__device__ __forceinline__ void axis_products(float s, float h, float (&w)[NI]) {
+    const F2 ss = f2(s, s);
+    if constexpr (NI == 4) {
+        const F2 hu = f2(h, 1.f - h), sq = mul2(hu, hu);
+        const F2 outer = mul2(ss, mul2(mul2(hu, f2(1.f / 6.f, 1.f / 6.f)), sq));  // w3, w0
+        // 2/3 rounded up and down: the two errors cancel in the sum
+        const F2 inner = mul2(ss, fma2(fma2(hu, f2(0.5f, 0.5f), f2(-1.f, -1.f)), sq, f2(2.f / 3.f, 0.66666663f)));
+        w[0] = f2_hi(outer);
+        w[1] = f2_lo(inner);
+        w[2] = f2_hi(inner);
+        w[3] = f2_lo(outer);
+    } else if constexpr (NI == 3) {
+        const float a = 0.5f - h, c = 0.5f + h;
+        const F2 ac = f2(a, c), outer = mul2(ss, mul2(mul2(f2(0.5f, 0.5f), ac), ac));
+        w[0] = f2_lo(outer);
+        w[1] = s * fmaf(-h, h, 0.75f);
+        w[2] = f2_hi(outer);
+    } else if constexpr (NI == 2) {
+        w[0] = s * (1.f - h);
+        w[1] = s * h;
+    } else {
+        w[0] = s;
+    }
+}
 
 // offset of a stencil's first cell from the origin of a tile that the stencils of its
 // particle touch, in [-NI, 16]: the tile and the stencil may lie on either side of the wrap
@@ -537,8 +543,8 @@ __device__ __forceinline__ unsigned atom_shared(unsigned a, unsigned v) {
 //  * WIDE: one grid at a time as 64-bit sums, low words and high words (array 0 and 1):
 //    the low word's atomic returns the old word, from which follows the carry.
 // The sums are the same integers in every form.  (2 10^6 particles in 256^3, order 4 on two
-// grids: 64-bit words 483 us, SHORT 271; 10^8: 19.9 ms, SHORT 10.7, SPLIT 21.8, WIDE 27.  Where
-// every tile has a cell beyond 16 particles, SHORT and HIGH take 533 against 475 us, and 4.17
+// grids: 64-bit words 483 us, SHORT 258; 10^8: 19.9 ms, SHORT 9.3.  Where
+// every tile has a cell beyond 16 particles, SHORT and HIGH take 516 against 475 us, and 3.83
 // against 4.12 ms at 2 10^7.)
 constexpr unsigned kSumBias = 1u << 24;
 constexpr unsigned kShortRecords = (1u << 16) - 1, kSplitRecords = 1u << 23;
@@ -572,19 +578,19 @@ __device__ __forceinline__ long long add_items(unsigned b, unsigned e, int g0, f
     const int g = NG == 2 ? (int)((t0 + sub) & 1u) : g0;  // (step is even)
     const unsigned base = smem_addr(acc) + 4u * (unsigned)((NG == 2 ? g * arr_words(NI) : 0) + cj * kPy + ci);
     long long tot = 0;
-    auto fetch = [&](unsigned t, PCell &c, float &wt) {
+    auto fetch = [&](unsigned t, PCell &c, float &wt, bool all) {
         t += sub;
-        if (t < n && !idle) {
+        if (all || (t < n && !idle)) {
             c = ld_cell(&sorted[b + t / NG].g[g]);
             if (W) wt = __ldg(&wsorted[b + t / NG]);
         }
     };
-    auto add = [&](unsigned t, const PCell &c, float wt) {
-        if ((IPW > NG && t + sub >= n) || idle) return;
+    auto add = [&](const PCell &c, float wt, bool is) {
+        if (IPW > NG && (!is || idle)) return;
         const F2 wxwy = horner2(pxy, f2(c.h[0], c.h[1]));  // w_x and w_y, each rounded as by single FMAs
         const float wxy = f2_lo(wxwy) * f2_hi(wxwy) * scale;
-        float wz[NI];
-        axis_weights<NI>(c.h[2], wz);
+        float w[NI];
+        axis_products<NI>(wxy, c.h[2], w);
         const unsigned cell = base + (unsigned)(c.pack & (kOut - 1));
         if (F == SHORT || F == SPLIT) {
             flags |= c.pack;
@@ -593,8 +599,7 @@ __device__ __forceinline__ long long add_items(unsigned b, unsigned e, int g0, f
         int part = 0;
 #pragma unroll
         for (int l = 0; l < NI; l++) {
-            float wv = wxy * wz[l];
-            if (W) wv *= wt;
+            const float wv = W ? w[l] * wt : w[l];
             if constexpr (F == SHORT) {
                 const int q = __float2int_rn(wv);
                 red_shared(cell + l * PZ, (unsigned)q);
@@ -632,15 +637,23 @@ __device__ __forceinline__ long long add_items(unsigned b, unsigned e, int g0, f
 #pragma unroll
     for (int k = 0; k < kAhead; k++) {
         wt[k] = 1.f;
-        fetch(t0 + k * step, c[k], wt[k]);
+        fetch(t0 + k * step, c[k], wt[k], false);
     }
     before();
-    for (unsigned t = t0; t < n; t += kAhead * step) {
+    unsigned t = t0;
+    const unsigned round = kAhead * step;
+    for (; t < n && n - t >= 2 * round; t += round)  // (no test of the bounds until the end)
+#pragma unroll
+        for (int k = 0; k < kAhead; k++) {
+            add(c[k], wt[k], true);
+            fetch(t + (k + kAhead) * step, c[k], wt[k], true);
+        }
+    for (; t < n; t += round) {
 #pragma unroll
         for (int k = 0; k < kAhead; k++) {
             if (t + k * step >= n) break;
-            add(t + k * step, c[k], wt[k]);
-            fetch(t + (k + kAhead) * step, c[k], wt[k]);
+            add(c[k], wt[k], t + k * step + sub < n);
+            fetch(t + (k + kAhead) * step, c[k], wt[k], false);
         }
     }
     return tot;

@@ -61,7 +61,8 @@ template <bool R20>
 __device__ __forceinline__ void run_dit(const fftd::FftDesc &fd, float2 *buf, const int2 *ent, const float2 *tw,
                                         int warp, int nw, int lane) {
     for (int s = fd.nst - 1; s >= 0; s--) {
-        const int R = fd.rad[s], ls = fd.ls[s], nbf = fd.n / R;
+        const int R = fd.rad[s], ls = fd.ls[s];
+        const int nbf = (s + 1 < fd.nst ? fd.eoff[s + 1] : fd.nent) - fd.eoff[s];  // n / R
         const int2 *e = ent + fd.eoff[s];
         if (R20 && R == 20) {
             for (int j = warp; j < nbf; j += nw) fftd::dit_butterfly<20>(buf, kP, lane, e[j].x, ls, e[j].y, tw);
