@@ -549,7 +549,8 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) pk_accum_kernel(
                 }
             }
             if (MODE == 1 && k2 > 0) {
-                const A i2 = (A)1 / (A)k2, m2 = t1 * i2, m4 = t2 * i2 * i2;
+                // divided, not multiplied by 1 / k2, whose rounding all modes of this k2 would share
+                const A m2 = t1 / (A)k2, m4 = t2 / (A)k2 / (A)k2;
                 t1 = (A)-0.5 * t0 + (A)1.5 * m2;
                 t2 = (A)0.375 * t0 + ((A)-3.75 * m2 + (A)4.375 * m4);
             }
