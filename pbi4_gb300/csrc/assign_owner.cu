@@ -83,6 +83,7 @@ struct OwnerPtrs {
     unsigned int *count, *start, *cursor;  // count: [ntiles + 2], the last two the tile counter
     PTile *sorted;
     float *wsorted;
+    unsigned int *place;  // few tiles: the first place of each counting block's records, by block and tile
 };
 static_assert(sizeof(OwnerPtrs) <= kOwnerPtrBytes, "owner pointer block");
 constexpr int kOut = 1 << 16;
@@ -312,7 +313,7 @@ __device__ __forceinline__ int span_tiles(const int lo[3], int w, const TileGeom
 // tile's count once.  Particles in random order otherwise queue on a few addresses
 // (100,000 of them on 64 tiles: 31 us for the count alone).
 constexpr int kSmallTiles = 2048;
-constexpr int kSortThreads = 256;
+constexpr int kSortThreads = 256, kSmallThreads = 512, kSmallBlocks = 304;
 
 // particles [b, e) of this block (small grids: a contiguous share; else all, strided by the grid)
 __device__ __forceinline__ void block_share(bool small, int64_t n, int64_t &b, int64_t &e, int64_t &step) {
@@ -328,7 +329,7 @@ __device__ __forceinline__ void block_share(bool small, int64_t n, int64_t &b, i
 }
 
 template <bool IND, bool GEN, bool SMALL>
-__global__ void __launch_bounds__(kSortThreads) owner_count_kernel(const TileGeom g, int nintp, int interlaced,
+__global__ void __launch_bounds__(SMALL ? kSmallThreads : kSortThreads) owner_count_kernel(const TileGeom g, int nintp, int interlaced,
                                                                   int64_t npart, int64_t stride,
                                                                   const BoxPar *__restrict__ bp,
                                                                   const double *__restrict__ pos_arg,
@@ -370,8 +371,9 @@ __global__ void __launch_bounds__(kSortThreads) owner_count_kernel(const TileGeo
     }
     if (SMALL) {
         __syncthreads();
+        unsigned int *__restrict__ place = (IND ? op->place : ov.place) + (size_t)blockIdx.x * ntiles;
         for (int t = threadIdx.x; t < ntiles; t += blockDim.x)
-            if (hist[t]) atomicAdd(count + t, hist[t]);
+            if (hist[t]) place[t] = atomicAdd(count + t, hist[t]);  // (from the tile's start)
     }
 }
 
@@ -415,7 +417,7 @@ __global__ void owner_scan_kernel(int ntiles, const OwnerPtrs ov, const OwnerPtr
 // Scatter: a record per (particle, touched tile).  The positions are read again: preparing
 // them costs less than a 32-byte prepared record written by the count and read back.
 template <bool IND, bool GEN, bool SMALL>
-__global__ void __launch_bounds__(kSortThreads) owner_scatter_kernel(
+__global__ void __launch_bounds__(SMALL ? kSmallThreads : kSortThreads) owner_scatter_kernel(
     const TileGeom g, int nintp, int interlaced, int64_t npart, int64_t stride, const BoxPar *__restrict__ bp,
     const double *__restrict__ pos_arg, const OwnerPtrs ov, const OwnerPtrs *__restrict__ op,
     const double *__restrict__ weight) {
@@ -430,22 +432,10 @@ __global__ void __launch_bounds__(kSortThreads) owner_scatter_kernel(
     int64_t b, e, step;
     block_share(SMALL, bp ? bp->npart : npart, b, e, step);
     if (SMALL) {
-        // the block's records per tile, then a range of places for them: one global atomic a tile
-        for (int t = threadIdx.x; t < ntiles; t += blockDim.x) place[t] = 0u;
-        __syncthreads();
-        for (int64_t i = b + threadIdx.x; i < e; i += step) {
-            Prep r;
-            prep_particle(pos, stride, i, g.N, nintp, interlaced, r);
-            int t[3][2];
-            const int two = span_tiles<GEN>(r.lo, w, g, t);
-#pragma unroll
-            for (int sl = 0; sl < 8; sl++)
-                if ((sl & ~two) == 0)
-                    atomicAdd(place + (t[2][sl >> 2] * g.nt + t[1][(sl >> 1) & 1]) * g.nt + t[0][sl & 1], 1u);
-        }
-        __syncthreads();
-        for (int t = threadIdx.x; t < ntiles; t += blockDim.x)
-            if (place[t]) place[t] = atomicAdd(cursor + t, place[t]);
+        // the block's places of each tile: the particles are those it counted
+        const unsigned int *__restrict__ first = (IND ? op->place : ov.place) + (size_t)blockIdx.x * ntiles;
+        const unsigned int *__restrict__ start = IND ? op->start : ov.start;
+        for (int t = threadIdx.x; t < ntiles; t += blockDim.x) place[t] = start[t] + first[t];
         __syncthreads();
     }
     for (int64_t i = b + threadIdx.x; i < e; i += step) {
@@ -876,12 +866,16 @@ bool owner_direct(int N, int64_t npart) {
     return owner_supported(N) || (N >= 2 * kT && N <= 2048 && npart <= ((int64_t)1 << 26));
 }
 
+// (whatever the grid: a shared scratch of a large grid also serves plans of few tiles)
+static constexpr size_t kPlaceBytes = sizeof(unsigned) * (size_t)kSmallBlocks * kSmallTiles;  // 2.5 MB
+
 bool OwnerWork::fits(int N, int64_t npart) const {
     const int nt = (N + kT - 1) / kT;
     const size_t ntiles = (size_t)nt * nt * nt;
     const size_t n = (size_t)(npart > 0 ? npart : 1);
     return count.p && count.bytes >= (ntiles + 2) * 4 && start.bytes >= (ntiles + 1) * 4 &&
-           cursor.bytes >= (ntiles + 1) * 4 && sorted.bytes >= 8 * n * sizeof(PTile) && wsorted.bytes >= 8 * n * 4 && wmax.bytes >= 8;
+           cursor.bytes >= (ntiles + 1) * 4 && sorted.bytes >= 8 * n * sizeof(PTile) && wsorted.bytes >= 8 * n * 4 && wmax.bytes >= 8 &&
+           place.bytes >= kPlaceBytes;
 }
 
 int OwnerWork::ensure(int N, int64_t npart) {
@@ -900,11 +894,12 @@ int OwnerWork::ensure(int N, int64_t npart) {
     PBI4G_CHECK(sorted.ensure(8 * n * sizeof(PTile)));
     PBI4G_CHECK(wsorted.ensure(8 * n * 4));
     PBI4G_CHECK(wmax.ensure(8));
+    PBI4G_CHECK(place.ensure(kPlaceBytes));
     return PBI4G_OK;
 }
 
 void OwnerWork::release() {
-    for (DevBuf *b : {&count, &start, &cursor, &sorted, &wsorted, &wmax}) b->release();
+    for (DevBuf *b : {&count, &start, &cursor, &sorted, &wsorted, &wmax, &place}) b->release();
 }
 
 size_t OwnerWork::footprint(int N, int64_t npart) {
@@ -920,6 +915,7 @@ void owner_ptrs_host(const OwnerWork &wk, unsigned char (&block)[kOwnerPtrBytes]
     o.cursor = wk.cursor.as<unsigned int>();
     o.sorted = static_cast<PTile *>(wk.sorted.p);
     o.wsorted = wk.wsorted.as<float>();
+    o.place = wk.place.as<unsigned int>();
     memset(block, 0, kOwnerPtrBytes);
     memcpy(block, &o, sizeof(o));
 }
@@ -972,18 +968,19 @@ int assign_owner(OwnerWork &wk, const void *d_ptrs, int N, int nintp, bool inter
     const TileGeom geo = {N, nt, 1.0f / (float)N, 1.0f / (float)nt};
     // few tiles: a block counts its share in shared memory, over about two blocks an SM
     const bool small = ntiles <= kSmallTiles;
-    const int blocks = small ? (int)std::min<int64_t>(152 * 2, (npart + kSortThreads - 1) / kSortThreads)
-                             : grid_blocks(npart, kSortThreads);
+    const int threads = small ? kSmallThreads : kSortThreads;
+    const int blocks = small ? (int)std::min<int64_t>(kSmallBlocks, (npart + threads - 1) / threads)
+                             : grid_blocks(npart, threads);
     pf.begin(sort_stage, st);
     // counts and the tile counter
     auto sort = [&](auto ind, auto general, auto few) -> int {
         constexpr bool IND = decltype(ind)::value, GEN = decltype(general)::value, SM = decltype(few)::value;
-        owner_count_kernel<IND, GEN, SM><<<blocks, kSortThreads, 0, st>>>(geo, nintp, interlaced, npart, stride, bp,
+        owner_count_kernel<IND, GEN, SM><<<blocks, threads, 0, st>>>(geo, nintp, interlaced, npart, stride, bp,
                                                                          d_pos, ov, op);
         PBI4G_LAUNCH_CHECK();
         owner_scan_kernel<IND><<<1, 1024, 0, st>>>(ntiles, ov, op);
         PBI4G_LAUNCH_CHECK();
-        owner_scatter_kernel<IND, GEN, SM><<<blocks, kSortThreads, 0, st>>>(geo, nintp, interlaced, npart, stride, bp,
+        owner_scatter_kernel<IND, GEN, SM><<<blocks, threads, 0, st>>>(geo, nintp, interlaced, npart, stride, bp,
                                                                            d_pos, ov, op, d_weight);
         return PBI4G_OK;
     };

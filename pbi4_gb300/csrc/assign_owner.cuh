@@ -5,7 +5,7 @@
 namespace pbi4g {
 
 struct OwnerWork {
-    DevBuf count, start, cursor, sorted, wsorted, wmax;
+    DevBuf count, start, cursor, sorted, wsorted, wmax, place;
     bool fixed = false;  // a shared scratch: sized once, never reallocated (ensure fails instead)
     int ensure(int N, int64_t npart);
     bool fits(int N, int64_t npart) const;
