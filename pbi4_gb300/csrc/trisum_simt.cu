@@ -247,33 +247,43 @@ __global__ void __launch_bounds__(Shape<T, S>::threads, Shape<T, S>::ctas) trisu
     }
 }
 
-// S[slot] (+)= sum over the partial results: 32 slots a block, the partials dealt to
-// its 32 warps and their sums added in warp order (a fixed order for every launch).
-// One thread a slot took 52 us for 86 slots x 304 partials, all of it load latency.
+// S[slot] (+)= sum over the partial results: SL slots a block, the partials dealt to its
+// 1024 / SL groups of lanes and the groups' sums added in order (a fixed order for every
+// launch).  The loads' latency is all of it (one thread a slot took 52 us for 86 slots x 304
+// partials), so few slots take more groups: 86 slots x 1376 partials take 16.6 us with 32 slots a
+// block, 8.0 with 8.
+template <int SL>
 __global__ void __launch_bounds__(1024) reduce_partial_kernel(int nslots, int nparts,
                                                               const double *__restrict__ partial,
                                                               double *__restrict__ S, int accumulate) {
-    __shared__ double sh[32][33];
-    const int lane = threadIdx.x, w = threadIdx.y, s = blockIdx.x * 32 + lane;
+    constexpr int G = 1024 / SL;
+    __shared__ double sh[G][SL + 1];
+    const int i = threadIdx.x % SL, g = threadIdx.x / SL, s = blockIdx.x * SL + i;
     double v = 0;
     if (s < nslots) {
 #pragma unroll 8
-        for (int k = w; k < nparts; k += 32) v += partial[(size_t)k * nslots + s];
+        for (int k = g; k < nparts; k += G) v += partial[(size_t)k * nslots + s];
     }
-    sh[w][lane] = v;
+    sh[g][i] = v;
     __syncthreads();
-    if (w == 0 && s < nslots) {
+    if (threadIdx.x < 32 * SL) {  // a warp a slot
+        const int lane = threadIdx.x & 31, t = threadIdx.x >> 5;
         double r = 0;
 #pragma unroll
-        for (int k = 0; k < 32; k++) r += sh[k][lane];
-        S[s] = accumulate ? S[s] + r : r;
+        for (int k = 0; k < G / 32; k++) r += sh[k * 32 + lane][t];
+        for (int o = 16; o; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+        const int d = blockIdx.x * SL + t;
+        if (lane == 0 && d < nslots) S[d] = accumulate ? S[d] + r : r;
     }
 }
 
 }  // namespace
 
 int reduce_partials(int nslots, int nparts, const double *partial, double *S, bool accumulate, cudaStream_t st) {
-    reduce_partial_kernel<<<(nslots + 31) / 32, dim3(32, 32), 0, st>>>(nslots, nparts, partial, S, accumulate ? 1 : 0);
+    if (nslots <= 8 * 152)  // one round of blocks over the SMs
+        reduce_partial_kernel<8><<<(nslots + 7) / 8, 1024, 0, st>>>(nslots, nparts, partial, S, accumulate ? 1 : 0);
+    else
+        reduce_partial_kernel<32><<<(nslots + 31) / 32, 1024, 0, st>>>(nslots, nparts, partial, S, accumulate ? 1 : 0);
     PBI4G_LAUNCH_CHECK();
     return PBI4G_OK;
 }
