@@ -66,31 +66,35 @@ int Shells::build(int N_, float kbin_, float kcenter_, int nb_, int iopen_, int 
     const int h = N / 2;
     k2max = 3 * h * h;
     lut_h.assign(k2max + 1, 0);
+    int k2top = -1;  // the largest |k|^2 of a shell
     for (int k2 = 0; k2 <= k2max; k2++) {
         // idist = nint(dsqrt(di*di+dj*dj+dl*dl)/kbin - kcenter/kbin - tiny) + 1
         // (bispectrumI4.f90:73); di^2+dj^2+dl^2 is exact, so idist depends on k2 only.
         long long b = llround(sqrt((double)k2) / (double)kbin - kck - (double)FLT_MIN) + 1;
-        lut_h[k2] = (b >= 1 && b <= nb) ? (int)b : 0;
+        if (b > nb) break;  // (it never decreases)
+        if (b < 1) continue;
+        lut_h[k2] = (int)b;
+        k2top = k2;
     }
-    // full-grid modes per shell: multiplicity of |k_axis| = d is 1 for d in {0, N/2}, else 2
-    nmodes.assign(nb, 0);
-    for (int dz = 0; dz <= h; dz++)
-        for (int dy = 0; dy <= h; dy++)
-            for (int dx = 0; dx <= h; dx++) {
-                int b = lut_h[dx * dx + dy * dy + dz * dz];
-                if (!b) continue;
-                int m = (dx == 0 || dx == h ? 1 : 2) * (dy == 0 || dy == h ? 1 : 2) * (dz == 0 || dz == h ? 1 : 2);
-                nmodes[b - 1] += m;
-            }
     // Map grid: every shell mode has |k_axis| <= kmax, so the per-axis sum of
     // three of them lies in [-3 kmax, 3 kmax].  On any grid Nm > 3 kmax the
     // condition q1+q2+q3 = 0 (mod Nm) holds only for exact triangles; when
     // 3 kmax < N the reference's N grid has no aliased triangles either, and the
     // sum over x of three maps on the Nm grid equals the reference's sum times
     // (Nm/N)^3.  Otherwise the maps stay on the N grid.
-    kmax = 0;
-    for (int k2 = 0; k2 <= k2max; k2++)
-        if (lut_h[k2]) kmax = std::max(kmax, (int)floor(sqrt((double)k2)));
+    kmax = k2top > 0 ? (int)floor(sqrt((double)k2top)) : 0;
+    // full-grid modes per shell: multiplicity of |k_axis| = d is 1 for d in {0, N/2}, else 2.
+    // Only the sphere up to k2top holds any (a walk over the whole octant took 0.3 ms at 128^3).
+    nmodes.assign(nb, 0);
+    const int top = std::min(h, kmax);
+    auto mult = [&](int d) { return d == 0 || d == h ? 1 : 2; };
+    for (int dz = 0; dz <= top; dz++)
+        for (int dy = 0; dy <= top && dy * dy + dz * dz <= k2top; dy++)
+            for (int dx = 0; dx <= top && dx * dx + dy * dy + dz * dz <= k2top; dx++) {
+                int b = lut_h[dx * dx + dy * dy + dz * dz];
+                if (!b) continue;
+                nmodes[b - 1] += mult(dx) * mult(dy) * mult(dz);
+            }
     Nm = map_grid_for_kmax(N, kmax);
     ishift = (int)(kcenter / kbin) + (iopen ? 1 : 0);  // bispectrumI4.f90:38-42
     tri.clear();

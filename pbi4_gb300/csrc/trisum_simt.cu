@@ -30,8 +30,6 @@
 // the products in shared memory and 44% of their entries triangles.  FP64 at 96^3 points
 // and 10 shells: 1.4 ms against 6.7 ms, at the FP64 pipe's rate (0.5 TFMA/s).
 #include <algorithm>
-#include <map>
-#include <set>
 #include <vector>
 
 #include "bispec.cuh"
@@ -311,23 +309,28 @@ int TriPlan::build(const Shells &sh, int nsets_, int cross, bool dbl, int qoff) 
     nslots = (int)(sh.itot * nsets);
     nrows = cross ? 2 * nb : qoff + nsets * nb;
     // entries (f, g, q shell) -> triangle
-    std::vector<std::map<std::pair<int, int>, int>> ent(nb);
+    using Entry = std::pair<std::pair<int, int>, int>;
+    std::vector<std::vector<Entry>> ent(nb);  // by factor map f, sorted by (g, q shell)
     const int q0set = cross ? cross * nb : qoff;
     for (int64_t m = 0; m < sh.itot; m++) {
         const int l = sh.tri[3 * m], j = sh.tri[3 * m + 1], i = sh.tri[3 * m + 2];
-        if (!cross) ent[j - 1][{i - 1, l - 1}] = (int)m;
-        else ent[l - 1][{j - 1, i - 1}] = (int)m;
+        if (!cross) ent[j - 1].push_back({{i - 1, l - 1}, (int)m});
+        else ent[l - 1].push_back({{j - 1, i - 1}, (int)m});
     }
+    for (auto &e : ent) std::sort(e.begin(), e.end());
     // Cover the entries of one run of factor maps with G x Q windows: strips of Q (or G)
     // columns from the first uncovered one, each cut into windows from its last row down;
     // by columns or by rows, whichever needs fewer windows.
-    using Cells = std::set<std::pair<int, int>>;  // (column, row)
-    auto cover = [](const Cells &cells, int R, int C) {
+    using Cells = std::vector<std::pair<int, int>>;  // (column, row), sorted
+    std::vector<int> rows;
+    auto cover = [&rows](Cells &cells, int R, int C) {
+        std::sort(cells.begin(), cells.end());
         std::vector<std::pair<int, int>> w;  // (first column, first row)
         for (auto it = cells.begin(); it != cells.end();) {
             const int c0 = it->first;
-            std::set<int> rows;
-            for (; it != cells.end() && it->first < c0 + C; ++it) rows.insert(it->second);
+            rows.clear();
+            for (; it != cells.end() && it->first < c0 + C; ++it) rows.push_back(it->second);
+            std::sort(rows.begin(), rows.end());
             int lo = 1 << 30;  // first row of the last window
             for (auto r = rows.rbegin(); r != rows.rend(); ++r)
                 if (*r < lo) {
@@ -343,8 +346,8 @@ int TriPlan::build(const Shells &sh, int nsets_, int cross, bool dbl, int qoff) 
             Cells qg, gq;
             for (int f = f0; f < std::min(f1, nb); f++)
                 for (auto &kv : ent[f]) {
-                    qg.insert({kv.first.second, kv.first.first});
-                    gq.insert(kv.first);
+                    qg.push_back({kv.first.second, kv.first.first});
+                    gq.push_back(kv.first);
                 }
             const auto a = cover(qg, tg, tq), b = cover(gq, tq, tg);
             if (a.size() <= b.size())
@@ -372,8 +375,10 @@ int TriPlan::build(const Shells &sh, int nsets_, int cross, bool dbl, int qoff) 
             if (f >= std::min(nb, tl[t].w)) continue;
             for (int p = 0; p < tg; p++)
                 for (int b = 0; b < tq; b++) {
-                    auto it = ent[f].find({tl[t].y + p, tl[t].z + b});
-                    if (it == ent[f].end() || it->second < 0) continue;
+                    const std::pair<int, int> gq(tl[t].y + p, tl[t].z + b);
+                    auto it = std::lower_bound(ent[f].begin(), ent[f].end(), gq,
+                                               [](const Entry &e, const std::pair<int, int> &k) { return e.first < k; });
+                    if (it == ent[f].end() || it->first != gq || it->second < 0) continue;
                     for (int s = 0; s < nsets; s++)
                         st[(size_t)t * E + ((s * tq + b) * tf + x) * tg + p] = it->second * nsets + s;
                     it->second = -1;  // windows may overlap: each triangle belongs to one tile
