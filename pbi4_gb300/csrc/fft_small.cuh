@@ -25,6 +25,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -237,7 +238,7 @@ struct FftPlan {
 
     // false when n has a prime factor above 7 (or needs too many stages).  Radices
     // are taken greedily from {10, 8, 4, 2, 3, 5, 7}; with allow20 the factorisation
-    // that starts with 20 is used instead when it has fewer stages (each stage is a
+    // that begins with 20 is used instead when it has fewer stages (each stage is a
     // round trip of every point through shared memory).
     bool build(int n, bool allow20 = false) {
         auto factor = [&](bool with20, FftDesc &o) {
@@ -261,6 +262,9 @@ struct FftPlan {
         FftDesc alt;
         if (!factor(false, d)) return false;
         if (allow20 && factor(true, alt) && alt.nst < d.nst) d = alt;
+        // the largest radix last: the first to run, without twiddles, and where the kernels
+        // read it from global memory the one with the most loads in flight
+        std::reverse(d.rad, d.rad + d.nst);
         ent.clear();
         int L = n;
         for (int s = 0; s < d.nst; s++) {

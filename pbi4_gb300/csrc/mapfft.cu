@@ -34,22 +34,18 @@ constexpr int kThreads = 256;
 #ifndef PBI4G_XPASS_MINB
 #define PBI4G_XPASS_MINB 4
 #endif
-// column loads the y pass keeps in flight per thread (8: 8% faster than 1 at 256^3)
-#ifndef PBI4G_YPASS_BATCH
-#define PBI4G_YPASS_BATCH 8
-#endif
 
 __device__ __forceinline__ float2 czero() { return make_float2(0.f, 0.f); }
 
 // copy the packed plan tables (twiddles | entries | positions) into shared memory
 __device__ __forceinline__ void load_tables(const unsigned char *__restrict__ tab, const fftd::FftDesc &fd,
-                                            float2 *tw, int2 *ent, int *perm) {
+                                            float2 *tw, int2 *ent, int *perm) {  // (perm: may be null)
     const float2 *t = reinterpret_cast<const float2 *>(tab);
     const int2 *e = reinterpret_cast<const int2 *>(t + fd.n);
     const int *p = reinterpret_cast<const int *>(e + fd.nent);
     for (int i = threadIdx.x; i < fd.n; i += blockDim.x) {
         tw[i] = t[i];
-        perm[i] = p[i];
+        if (perm) perm[i] = p[i];
     }
     for (int i = threadIdx.x; i < fd.nent; i += blockDim.x) ent[i] = e[i];
 }
@@ -59,8 +55,8 @@ __device__ __forceinline__ void load_tables(const unsigned char *__restrict__ ta
 // R20: the plan may hold radix-20 stages (plans built with allow20)
 template <bool R20>
 __device__ __forceinline__ void run_dit(const fftd::FftDesc &fd, float2 *buf, const int2 *ent, const float2 *tw,
-                                        int warp, int nw, int lane) {
-    for (int s = fd.nst - 1; s >= 0; s--) {
+                                        int warp, int nw, int lane, int from) {
+    for (int s = from; s >= 0; s--) {
         const int R = fd.rad[s], ls = fd.ls[s];
         const int nbf = (s + 1 < fd.nst ? fd.eoff[s + 1] : fd.nent) - fd.eoff[s];  // n / R
         const int2 *e = ent + fd.eoff[s];
@@ -94,6 +90,53 @@ __device__ __forceinline__ void run_dit(const fftd::FftDesc &fd, float2 *buf, co
         }
         __syncthreads();
     }
+}
+
+// The first of those stages straight from its inputs: butterfly j holds the points j R + r, whose
+// inputs are load(i0[j] + r n / R), and has no twiddles (its Ls is 1).  The points then make
+// one round trip through shared memory less than when they are placed there first, with a
+// barrier and a table look-up less (at 256^3, 42 shells x 3 sets: x pass 1027 -> 968 us, y pass
+// 317 -> 243; the z pass, whose inputs take most of its work, gained nothing at 256^3).
+template <int R, class Load>
+__device__ __forceinline__ void first_butterflies(float2 *buf, const int *i0, int nbf, int warp, int nw, int lane,
+                                                  Load &&load) {
+    for (int j = warp; j < nbf; j += nw) {
+        const int i = i0[j];
+        float2 v[fftd::kMaxRadix];
+#pragma unroll
+        for (int r = 0; r < R; r++) v[r] = load(i + r * nbf);
+        fftd::dft_small<R>(v);
+        float2 *o = buf + j * (R * kP) + lane;
+#pragma unroll
+        for (int q = 0; q < R; q++) o[q * kP] = v[q];
+    }
+}
+template <bool R20, class Load>
+__device__ __forceinline__ void first_stage(const fftd::FftDesc &fd, float2 *buf, const int *i0, int warp, int nw,
+                                            int lane, Load &&load) {
+    const int s = fd.nst - 1, nbf = fd.nent - fd.eoff[s];
+    if (R20 && fd.rad[s] == 20) {
+        first_butterflies<20>(buf, i0, nbf, warp, nw, lane, load);
+    } else {
+        switch (fd.rad[s]) {
+            case 10: first_butterflies<10>(buf, i0, nbf, warp, nw, lane, load); break;
+            case 8: first_butterflies<8>(buf, i0, nbf, warp, nw, lane, load); break;
+            case 4: first_butterflies<4>(buf, i0, nbf, warp, nw, lane, load); break;
+            case 2: first_butterflies<2>(buf, i0, nbf, warp, nw, lane, load); break;
+            case 3: first_butterflies<3>(buf, i0, nbf, warp, nw, lane, load); break;
+            case 5: first_butterflies<5>(buf, i0, nbf, warp, nw, lane, load); break;
+            default: first_butterflies<7>(buf, i0, nbf, warp, nw, lane, load); break;
+        }
+    }
+    __syncthreads();
+}
+// the input of each first butterfly's point 0, in place of the positions
+__device__ __forceinline__ void first_inputs(const fftd::FftDesc &fd, const unsigned char *__restrict__ tab, int *i0) {
+    const int *p = reinterpret_cast<const int *>(reinterpret_cast<const int2 *>(reinterpret_cast<const float2 *>(tab) + fd.n) +
+                                                 fd.nent);
+    const int R = fd.rad[fd.nst - 1];
+    for (int i = threadIdx.x; i < fd.n; i += blockDim.x)
+        if (p[i] % R == 0) i0[p[i] / R] = i;
 }
 
 size_t table_smem(const fftd::FftDesc &fd) {
@@ -181,7 +224,7 @@ __global__ void __launch_bounds__(kThreads, PBI4G_ZPASS_MINB) map_zpass_kernel(c
             if (lane == 0 && pw != 0.0) atomicAdd(&spow[s * nb + b - 1], pw);
         }
         __syncthreads();
-        run_dit<true>(fd, buf, ent, tw, warp, nw, lane);
+        run_dit<true>(fd, buf, ent, tw, warp, nw, lane, fd.nst - 1);
         // column c0 + l -> T[tbase + (c0 + l) Nm + z], z along the lanes
         for (int l = warp; l < 32; l += nw) {
             if (c0 + l >= mi.ncol) break;
@@ -219,9 +262,10 @@ __global__ void __launch_bounds__(kThreads, PBI4G_YPASS_MINB) map_ypass_kernel(c
     const int Nm = a.Nm;
     float2 *tw = reinterpret_cast<float2 *>(ysm);
     int2 *ent = reinterpret_cast<int2 *>(tw + fd.n);
-    int *perm = reinterpret_cast<int *>(ent + fd.nent);
-    float2 *buf = reinterpret_cast<float2 *>(perm + fd.n);
-    load_tables(a.tab, fd, tw, ent, perm);
+    int *i0 = reinterpret_cast<int *>(ent + fd.nent);
+    float2 *buf = reinterpret_cast<float2 *>(i0 + fd.n);
+    load_tables(a.tab, fd, tw, ent, nullptr);
+    first_inputs(fd, a.tab, i0);
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int ntiles = (a.nflat + 31) / 32;
@@ -235,22 +279,11 @@ __global__ void __launch_bounds__(kThreads, PBI4G_YPASS_MINB) map_ypass_kernel(c
         const int kx = g - mi.kxc;
         const int2 rc = valid ? a.kxr[mi.kx0 + kx] : make_int2(-1, 0);  // (r, first column)
         const float2 *in = a.T + mi.tbase + (size_t)(rc.y + rc.x) * Nm + z;  // column ky = 0
-        // PBI4G_YPASS_BATCH column loads in flight per thread before their shared stores
-        for (int i0 = warp; i0 < Nm; i0 += PBI4G_YPASS_BATCH * nw) {
-            float2 v[PBI4G_YPASS_BATCH];
-#pragma unroll
-            for (int u = 0; u < PBI4G_YPASS_BATCH; u++) {
-                const int i = i0 + u * nw, ky = kfreq0(i, Nm);
-                v[u] = (i < Nm && ky >= -rc.x && ky <= rc.x) ? __ldcs(in + (ptrdiff_t)ky * Nm) : czero();
-            }
-#pragma unroll
-            for (int u = 0; u < PBI4G_YPASS_BATCH; u++) {
-                const int i = i0 + u * nw;
-                if (i < Nm) buf[perm[i] * kP + lane] = v[u];
-            }
-        }
-        __syncthreads();
-        run_dit<true>(fd, buf, ent, tw, warp, nw, lane);
+        first_stage<true>(fd, buf, i0, warp, nw, lane, [&](int i) {
+            const int ky = kfreq0(i, Nm);
+            return ky >= -rc.x && ky <= rc.x ? __ldcs(in + (ptrdiff_t)ky * Nm) : czero();
+        });
+        run_dit<true>(fd, buf, ent, tw, warp, nw, lane, fd.nst - 2);
         for (int l = warp; l < 32; l += nw) {
             if (t0 + l >= a.nflat) break;
             float2 *o = a.U + (size_t)(t0 + l) * Nm;
@@ -351,8 +384,8 @@ __device__ __forceinline__ void store_planes(const XArgs &a, const float2 *buf, 
 // x pass: tile = (map m, 32 consecutive rows (z, y)).  With M = Nm / 2,
 // Z[k] = (X[k] + conj X[M-k]) + i (X[k] - conj X[M-k]) e^{2 pi i k / Nm} and
 // z = IDFT_M(Z) give the C2R output x[2j] = Re z[j], x[2j+1] = Im z[j].  The
-// raw coefficients (kx < kxmax) stay in their own buffer while the pairs
-// (k, M - k) are formed into the permuted positions of the FFT buffer.  PF:
+// raw coefficients (kx < kxmax) stay in their own buffer, from which the first
+// butterflies form their Z[k].  PF:
 // coefficient rows a warp prefetches into registers for the next tile
 // (kxmax <= PF * warps).
 template <int PF>
@@ -362,11 +395,12 @@ __global__ void __launch_bounds__(kThreads, PF <= 9 ? PBI4G_XPASS_MINB : 2) map_
     const int Nm = a.Nm, M = fd.n, KX = a.kxmax;
     float2 *tw = reinterpret_cast<float2 *>(xsm);
     int2 *ent = reinterpret_cast<int2 *>(tw + fd.n);
-    int *perm = reinterpret_cast<int *>(ent + fd.nent);
-    float2 *xt = reinterpret_cast<float2 *>(perm + fd.n);  // [Nm]
+    int *i0 = reinterpret_cast<int *>(ent + fd.nent);
+    float2 *xt = reinterpret_cast<float2 *>(i0 + fd.n);    // [Nm]
     float2 *xr = xt + Nm;                                  // [KX][kP] raw coefficients
     float2 *buf = xr + (size_t)KX * kP;                    // [M][kP]
-    load_tables(a.tab, fd, tw, ent, perm);
+    load_tables(a.tab, fd, tw, ent, nullptr);
+    first_inputs(fd, a.tab, i0);
     for (int i = threadIdx.x; i < Nm; i += blockDim.x) xt[i] = a.xtw[i];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int row_hi = a.row_lo + a.nrows, tpm = (a.nrows + 31) / 32, ntiles = tpm * a.count;
@@ -406,25 +440,17 @@ __global__ void __launch_bounds__(kThreads, PF <= 9 ? PBI4G_XPASS_MINB : 2) map_
         }
         if (tile + (int)gridDim.x < ntiles) fetch(mn, a.row_lo + rn * 32);
         __syncthreads();
-        for (int k = warp; k <= M / 2; k += nw) {
-            const int kc = M - k;
-            if (k >= kxn && kc >= kxn) {  // X[k] = X[M - k] = 0 (k is warp-uniform)
-                buf[perm[k] * kP + lane] = czero();
-                if (k > 0 && kc != k) buf[perm[kc] * kP + lane] = czero();
-                continue;
-            }
-            const float2 xk = k < kxn ? xr[k * kP + lane] : czero();
-            const float2 xc = (k > 0 && kc < kxn) ? xr[kc * kP + lane] : czero();  // X[M - k]
-            const float2 ck = make_float2(xc.x, -xc.y), cc = make_float2(xk.x, -xk.y);
-            const float2 o1 = fftd::cmul(fftd::csub(xk, ck), xt[k]);
-            buf[perm[k] * kP + lane] = fftd::cadd_i(fftd::cadd(xk, ck), o1);
-            if (k > 0 && kc != k) {
-                const float2 o2 = fftd::cmul(fftd::csub(xc, cc), xt[kc]);
-                buf[perm[kc] * kP + lane] = fftd::cadd_i(fftd::cadd(xc, cc), o2);
-            }
-        }
-        __syncthreads();
-        run_dit<false>(fd, buf, ent, tw, warp, nw, lane);
+        first_stage<false>(fd, buf, i0, warp, nw, lane, [&](int k) {
+            const int kc = M - k;  // (k is warp-uniform, and so are both tests)
+            const bool hk = k < kxn, hc = k > 0 && kc < kxn;
+            if (!hk && !hc) return czero();
+            const float2 xk = hk ? xr[k * kP + lane] : czero();
+            const float2 xc = hc ? xr[kc * kP + lane] : czero();  // X[M - k]
+            const float2 ck = make_float2(xc.x, -xc.y);
+            const float2 o = fftd::cmul(fftd::csub(xk, ck), xt[k]);
+            return fftd::cadd_i(fftd::cadd(xk, ck), o);
+        });
+        run_dit<false>(fd, buf, ent, tw, warp, nw, lane, fd.nst - 2);
         if (a.oform < 0) {
             // dense FP32 maps: one warp per row, x[2j], x[2j+1] = z[j]
             for (int l = warp; l < nrows; l += nw) {
