@@ -155,26 +155,26 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
 }
 __device__ __forceinline__ F2 horner2(const F2 c[4], F2 h) { return fma2(h, fma2(h, fma2(h, c[3], c[2]), c[1]), c[0]); }
 
-// s times all weights of an axis, by pairs (every operation rounds as the single one does): no
-// FP32 rounding makes any of them negative inside the box.
+// s times all weights of an axis, by pairs: axis_poly's cubics, every operation rounded as the
+// single one is, so the three axes err alike (forms of their own for z, though closer to the
+// weights, showed as a quadrupole).
 template <int NI>
 __device__ __forceinline__ void axis_products(float s, float h, float (&w)[NI]) {
-    const F2 ss = f2(s, s);
+    const F2 ss = f2(s, s), hh = f2(h, h);
     if constexpr (NI == 4) {
-        const F2 hu = f2(h, 1.f - h), sq = mul2(hu, hu);
-        const F2 outer = mul2(ss, mul2(mul2(hu, f2(1.f / 6.f, 1.f / 6.f)), sq));  // w3, w0
-        // 2/3 rounded up and down: the two errors cancel in the sum
-        const F2 inner = mul2(ss, fma2(fma2(hu, f2(0.5f, 0.5f), f2(-1.f, -1.f)), sq, f2(2.f / 3.f, 0.66666663f)));
-        w[0] = f2_hi(outer);
-        w[1] = f2_lo(inner);
-        w[2] = f2_hi(inner);
-        w[3] = f2_lo(outer);
+        const F2 w02 = fma2(hh, fma2(hh, fma2(hh, f2(-1.f / 6.f, -0.5f), f2(0.5f, 0.5f)), f2(-0.5f, 0.5f)),
+                            f2(1.f / 6.f, 1.f / 6.f));
+        const F2 w13 = fma2(hh, mul2(hh, fma2(hh, f2(0.5f, 1.f / 6.f), f2(-1.f, 0.f))), f2(2.f / 3.f, 0.f));
+        const F2 p02 = mul2(ss, w02), p13 = mul2(ss, w13);
+        w[0] = f2_lo(p02);
+        w[1] = f2_lo(p13);
+        w[2] = f2_hi(p02);
+        w[3] = f2_hi(p13);
     } else if constexpr (NI == 3) {
-        const float a = 0.5f - h, c = 0.5f + h;
-        const F2 ac = f2(a, c), outer = mul2(ss, mul2(mul2(f2(0.5f, 0.5f), ac), ac));
-        w[0] = f2_lo(outer);
+        const F2 p02 = mul2(ss, fma2(hh, fma2(hh, f2(0.5f, 0.5f), f2(-0.5f, 0.5f)), f2(0.125f, 0.125f)));
+        w[0] = f2_lo(p02);
         w[1] = s * fmaf(-h, h, 0.75f);
-        w[2] = f2_hi(outer);
+        w[2] = f2_hi(p02);
     } else if constexpr (NI == 2) {
         w[0] = s * (1.f - h);
         w[1] = s * h;
