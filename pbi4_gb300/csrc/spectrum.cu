@@ -478,9 +478,6 @@ int PkBins::build(int N_, float box_, float kbin_, float kcenter_, int nbins_, c
     return PBI4G_OK;
 }
 
-template <class R> struct AccOf { using T = float; };
-template <> struct AccOf<double> { using T = double; };
-
 // P(k) sums and the output rows (pout Fortran (5, nbins)) of measure_pk / measure_pk_multipoles
 // in one launch: the blocks add their sums to `sums`, and the last of them writes the rows and
 // clears `sums`.  For the multipoles of an auto spectrum the rows' p = |a|^2, p lk^2 and
@@ -490,16 +487,16 @@ template <> struct AccOf<double> { using T = double; };
 // their own and a second launch over the blocks' partial sums, took 31 us at 128^3, 72 us at
 // 256^3 and 2.65 ms at 1024^3 (the spectrum at HBM rate: 0.6 ms); this form 11, 31 us and
 // 1.00 ms (4.3 TB/s; issue 70% busy).
-template <class R, int MODE>
+template <class R, int MODE, class S>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) pk_accum_kernel(
     int N, int nbins, const int *__restrict__ lut, PkExact e, double l0, double l1, double l2,
     const typename Cx<R>::T *__restrict__ a, const typename Cx<R>::T *__restrict__ b,
     const typename Cx<R>::T *__restrict__ c, double *__restrict__ sums, double kF3,
     const double *__restrict__ avgk_co, double *__restrict__ pout) {
-    using A = typename AccOf<R>::T;
+    using A = R;
     using C = typename Cx<R>::T;
     extern __shared__ unsigned char smem_raw[];
-    A *s = reinterpret_cast<A *>(smem_raw);
+    S *s = reinterpret_cast<S *>(smem_raw);
     constexpr int nq = MODE == 0 ? 1 : 3;
     for (int i = threadIdx.x; i < nq * nbins; i += blockDim.x) s[i] = 0;
     __syncthreads();
@@ -513,7 +510,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) pk_accum_kernel(
         const int k2 = q.x * q.x + q.ka * q.ka + q.kb * q.kb;
         int bin = in ? __ldg(lut + k2) : 0;
         const unsigned rows = in ? pk_rows(q, N) : 0u;
-        const A lx = lf0 * (A)q.x;
+        const A lx = lf0 * (A)q.x, kk = (A)(k2 > 0 ? k2 : 1), ik = (A)1 / kk;
         A v[3] = {}, w[3] = {};  // the rows (y, z) and the swapped ones
         // four rows in flight (eight, where there is one array of single precision)
 #pragma unroll(sizeof(C) == 8 && MODE != 2 ? 2 : 1)
@@ -538,21 +535,17 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) pk_accum_kernel(
                 if (MODE == 0) {
                     t0 += (A)(va[r].x * vb[r].x + va[r].y * vb[r].y);
                 } else if (MODE == 1) {
-                    const A p = (A)(va[r].x * va[r].x + va[r].y * va[r].y), m = lk[r] * lk[r], pm = p * m;
+                    const A p = (A)(va[r].x * va[r].x + va[r].y * va[r].y), m = lk[r] * lk[r], m0 = m * ik;
+                    // the quotient m / k^2: ik's rounding, which all modes of one k^2 share, corrected
+                    const A mu2 = fma(fma(-m0, kk, m), ik, m0);
                     t0 += p;
-                    t1 += pm;
-                    t2 += pm * m;
+                    t1 += p * ((A)-0.5 + (A)1.5 * mu2);
+                    t2 += p * ((A)0.375 + mu2 * ((A)-3.75 + (A)4.375 * mu2));
                 } else {
                     t0 += (A)(va[r].x * va[r].x + va[r].y * va[r].y);
                     t1 += (A)(va[r].x * vb[r].x + va[r].y * vb[r].y);
                     t2 += (A)(va[r].x * vc[r].x + va[r].y * vc[r].y);
                 }
-            }
-            if (MODE == 1 && k2 > 0) {
-                // divided, not multiplied by 1 / k2, whose rounding all modes of this k2 would share
-                const A m2 = t1 / (A)k2, m4 = t2 / (A)k2 / (A)k2;
-                t1 = (A)-0.5 * t0 + (A)1.5 * m2;
-                t2 = (A)0.375 * t0 + ((A)-3.75 * m2 + (A)4.375 * m4);
             }
             if (g) {
                 w[0] = t0, w[1] = t1, w[2] = t2;
@@ -565,7 +558,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) pk_accum_kernel(
             const int other = pk_bin_exact(e, q.x, q.ka, q.kb);
             if (other != bin) {
                 if (other >= 1 && other <= nbins)
-                    for (int k = 0; k < nq; k++) atomicAdd(&s[k * nbins + other - 1], w[k]);
+                    for (int k = 0; k < nq; k++) atomicAdd(&s[k * nbins + other - 1], (S)w[k]);
                 w[0] = w[1] = w[2] = 0;
             }
         }
@@ -576,12 +569,12 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) pk_accum_kernel(
 #pragma unroll
         for (int k = 0; k < nq; k++) {
             const A r = pk_run_sum(v[k] + w[k], lane, start, longest);
-            if (last && bin) atomicAdd(&s[k * nbins + bin - 1], r);
+            if (last && bin) atomicAdd(&s[k * nbins + bin - 1], (S)r);
         }
     }
     __syncthreads();
     for (int i = threadIdx.x; i < nq * nbins; i += blockDim.x)
-        if (s[i] != (A)0) atomicAdd(sums + i, (double)s[i]);
+        if (s[i] != (S)0) atomicAdd(sums + i, (double)s[i]);
     unsigned *done = reinterpret_cast<unsigned *>(sums + 3 * nbins);
     __threadfence();
     __syncthreads();
@@ -616,13 +609,19 @@ static int pk_blocks(int N) {
 template <class R>
 int pk_measure(PkBins &bins, int mode, const double los[3], const typename Cx<R>::T *a, const typename Cx<R>::T *b,
                const typename Cx<R>::T *c, double *d_pout, cudaStream_t st, int64_t *launches) {
-    using A = typename AccOf<R>::T;
     const int nbins = bins.nbins, N = bins.N;
-    const size_t smem = sizeof(A) * (mode == 0 ? 1 : 3) * nbins;
-    if (smem > 200 * 1024) return set_error(PBI4G_ERR_INVALID, "too many P bins (%d)", nbins);
+    const size_t n = (mode == 0 ? 1 : 3) * (size_t)nbins;
+    constexpr size_t kMax = 200 * 1024;
+    if (sizeof(R) * n > kMax) return set_error(PBI4G_ERR_INVALID, "too many P bins (%d)", nbins);
+    const bool wide = sizeof(double) * n <= kMax;
+    const size_t smem = (wide ? sizeof(double) : sizeof(R)) * n;
     PkExact e{bins.kF, bins.dk, (double)(bins.kcenter / bins.kbin)};
     const double l0 = los ? los[0] : 0, l1 = los ? los[1] : 0, l2 = los ? los[2] : 0;
-    auto k = mode == 0 ? pk_accum_kernel<R, 0> : (mode == 1 ? pk_accum_kernel<R, 1> : pk_accum_kernel<R, 2>);
+    auto pick = [&](auto acc) {
+        using S = decltype(acc);
+        return mode == 0 ? pk_accum_kernel<R, 0, S> : (mode == 1 ? pk_accum_kernel<R, 1, S> : pk_accum_kernel<R, 2, S>);
+    };
+    auto k = wide ? pick(double()) : pick(R());
     if (smem > 48 * 1024) PBI4G_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k<<<pk_blocks<R>(N), 256, smem, st>>>(N, nbins, bins.lut.as<int>(), e, l0, l1, l2, a, mode == 0 && !b ? a : b, c,
                                           bins.sums.as<double>(), bins.kF3, bins.avgk_co.as<double>(), d_pout);
@@ -799,7 +798,7 @@ extern "C" int pbi4g_measure_pk_multipoles_noalloc(int32_t grid, float box, floa
     pk_bins_finish_kernel<<<1, 256, 0, st>>>(nbins, co, sumk);
     PBI4G_LAUNCH_CHECK();
     PBI4G_CUDA(cudaMemsetAsync(sums, 0, pk_sums_bytes(nbins), st));
-    pk_accum_kernel<double, 2><<<pk_blocks<double>(grid), 256, sizeof(double) * 3 * nbins, st>>>(
+    pk_accum_kernel<double, 2, double><<<pk_blocks<double>(grid), 256, sizeof(double) * 3 * nbins, st>>>(
         grid, nbins, lut, e, 0.0, 0.0, 0.0, static_cast<const double2 *>(d_dcl_half),
         static_cast<const double2 *>(d_dcl2_half), static_cast<const double2 *>(d_dcl4_half), sums, kF * kF * kF, sumk,
         d_pout);
