@@ -7,7 +7,7 @@ FP32 forms: Tz, Uy complex elements of the pruned transform's z-column and
   assign          FP32 forms (the owner-tile kernel): 32 R Np (R = records per particle,
                   (1 + (w-1)/16)^3 for a stencil w = nintp (+1 interlaced) wide) read + 4 G N^3
                   (FP32 grid write); FP64 form: 24 Np (float64 xyz read) + 8 G N^3 (int64)
-  assign_sort     FP32 forms' counting sort: 24 Np (xyz) + 64 Np (record write, read) + 32 R Np
+  assign_sort     FP32 forms' counting sort: 48 Np (xyz, by the count and the scatter) + 32 R Np
   grid_convert    8 G N^3 read + 4 G N^3 write (FP64 form only)
   fcomb           8 G H read + 8 H write
   pk_binning      8 H read
@@ -54,7 +54,8 @@ def traffic_table():
 
 
 # the source files each stage's kernels are built from (pbi4_gb300/csrc)
-SOURCES = {"assign": ("assign_owner.cu", "assign_owner.cuh"), "assign_sort": ("assign_owner.cu", "assign_owner.cuh"),
+SOURCES = {"assign": ("assign_owner.cu", "assign_owner.cuh", "fixed.cuh"),
+           "assign_sort": ("assign_owner.cu", "assign_owner.cuh"),
            "fcomb": ("spectrum.cu",), "pk_binning": ("spectrum.cu",),
            "shell_maps_z": ("mapfft.cu", "fft_small.cuh"), "shell_maps_y": ("mapfft.cu", "fft_small.cuh"),
            "shell_maps_x": ("mapfft.cu", "fft_small.cuh"), "triangle_sums": ("trisum_tm.cu", "tc_ptx.cuh")}
@@ -99,7 +100,7 @@ def stage_work(cfg, npart, map_grid=None, nmaps=None, map_work=None):
     work = {
         "assign": ("hbm", (24 * npart + gbytes * G * N ** 3) if cfg.precision == "fp64"
                    else (32 * R * npart + 4 * G * N ** 3)),
-        "assign_sort": ("hbm", 24 * npart + 64 * npart + 32 * R * npart),
+        "assign_sort": ("hbm", 48 * npart + 32 * R * npart),
         "grid_convert": ("hbm", 12 * G * N ** 3),
         "fcomb": ("hbm", 8 * G * H + 8 * H),
         "pk_binning": ("hbm", 8 * H),
