@@ -485,9 +485,9 @@ int PkBins::build(int N_, float box_, float kbin_, float kcenter_, int nbins_, c
 // polynomials applied once per (pair, x).
 // A single row at a time, with each lane's four modes binned and added to shared memory on
 // their own and a second launch over the blocks' partial sums, took 31 us at 128^3, 72 us at
-// 256^3 and 2.65 ms at 1024^3 (the spectrum at HBM rate: 0.6 ms); this form 11, 31 us and
-// 1.00 ms (4.3 TB/s; issue 70% busy).
-template <class R, int MODE, class S>
+// 256^3 and 2.65 ms at 1024^3 (the spectrum at HBM rate: 0.6 ms); this form 11, 32 us and
+// 1.04 ms (4.1 TB/s; issue 70% busy).
+template <class R, int MODE>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) pk_accum_kernel(
     int N, int nbins, const int *__restrict__ lut, PkExact e, double l0, double l1, double l2,
     const typename Cx<R>::T *__restrict__ a, const typename Cx<R>::T *__restrict__ b,
@@ -496,7 +496,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) pk_accum_kernel(
     using A = R;
     using C = typename Cx<R>::T;
     extern __shared__ unsigned char smem_raw[];
-    S *s = reinterpret_cast<S *>(smem_raw);
+    A *s = reinterpret_cast<A *>(smem_raw);
     constexpr int nq = MODE == 0 ? 1 : 3;
     for (int i = threadIdx.x; i < nq * nbins; i += blockDim.x) s[i] = 0;
     __syncthreads();
@@ -558,7 +558,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) pk_accum_kernel(
             const int other = pk_bin_exact(e, q.x, q.ka, q.kb);
             if (other != bin) {
                 if (other >= 1 && other <= nbins)
-                    for (int k = 0; k < nq; k++) atomicAdd(&s[k * nbins + other - 1], (S)w[k]);
+                    for (int k = 0; k < nq; k++) atomicAdd(&s[k * nbins + other - 1], w[k]);
                 w[0] = w[1] = w[2] = 0;
             }
         }
@@ -569,12 +569,12 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) pk_accum_kernel(
 #pragma unroll
         for (int k = 0; k < nq; k++) {
             const A r = pk_run_sum(v[k] + w[k], lane, start, longest);
-            if (last && bin) atomicAdd(&s[k * nbins + bin - 1], (S)r);
+            if (last && bin) atomicAdd(&s[k * nbins + bin - 1], r);
         }
     }
     __syncthreads();
     for (int i = threadIdx.x; i < nq * nbins; i += blockDim.x)
-        if (s[i] != (S)0) atomicAdd(sums + i, (double)s[i]);
+        if (s[i] != (A)0) atomicAdd(sums + i, (double)s[i]);
     unsigned *done = reinterpret_cast<unsigned *>(sums + 3 * nbins);
     __threadfence();
     __syncthreads();
@@ -610,18 +610,11 @@ template <class R>
 int pk_measure(PkBins &bins, int mode, const double los[3], const typename Cx<R>::T *a, const typename Cx<R>::T *b,
                const typename Cx<R>::T *c, double *d_pout, cudaStream_t st, int64_t *launches) {
     const int nbins = bins.nbins, N = bins.N;
-    const size_t n = (mode == 0 ? 1 : 3) * (size_t)nbins;
-    constexpr size_t kMax = 200 * 1024;
-    if (sizeof(R) * n > kMax) return set_error(PBI4G_ERR_INVALID, "too many P bins (%d)", nbins);
-    const bool wide = sizeof(double) * n <= kMax;
-    const size_t smem = (wide ? sizeof(double) : sizeof(R)) * n;
+    const size_t smem = sizeof(R) * (mode == 0 ? 1 : 3) * nbins;
+    if (smem > 200 * 1024) return set_error(PBI4G_ERR_INVALID, "too many P bins (%d)", nbins);
     PkExact e{bins.kF, bins.dk, (double)(bins.kcenter / bins.kbin)};
     const double l0 = los ? los[0] : 0, l1 = los ? los[1] : 0, l2 = los ? los[2] : 0;
-    auto pick = [&](auto acc) {
-        using S = decltype(acc);
-        return mode == 0 ? pk_accum_kernel<R, 0, S> : (mode == 1 ? pk_accum_kernel<R, 1, S> : pk_accum_kernel<R, 2, S>);
-    };
-    auto k = wide ? pick(double()) : pick(R());
+    auto k = mode == 0 ? pk_accum_kernel<R, 0> : (mode == 1 ? pk_accum_kernel<R, 1> : pk_accum_kernel<R, 2>);
     if (smem > 48 * 1024) PBI4G_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k<<<pk_blocks<R>(N), 256, smem, st>>>(N, nbins, bins.lut.as<int>(), e, l0, l1, l2, a, mode == 0 && !b ? a : b, c,
                                           bins.sums.as<double>(), bins.kF3, bins.avgk_co.as<double>(), d_pout);
@@ -798,7 +791,7 @@ extern "C" int pbi4g_measure_pk_multipoles_noalloc(int32_t grid, float box, floa
     pk_bins_finish_kernel<<<1, 256, 0, st>>>(nbins, co, sumk);
     PBI4G_LAUNCH_CHECK();
     PBI4G_CUDA(cudaMemsetAsync(sums, 0, pk_sums_bytes(nbins), st));
-    pk_accum_kernel<double, 2, double><<<pk_blocks<double>(grid), 256, sizeof(double) * 3 * nbins, st>>>(
+    pk_accum_kernel<double, 2><<<pk_blocks<double>(grid), 256, sizeof(double) * 3 * nbins, st>>>(
         grid, nbins, lut, e, 0.0, 0.0, 0.0, static_cast<const double2 *>(d_dcl_half),
         static_cast<const double2 *>(d_dcl2_half), static_cast<const double2 *>(d_dcl4_half), sums, kF * kF * kF, sumk,
         d_pout);
