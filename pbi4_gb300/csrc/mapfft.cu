@@ -95,7 +95,7 @@ __device__ __forceinline__ void run_dit(const fftd::FftDesc &fd, float2 *buf, co
 // The first of those stages straight from its inputs: butterfly j holds the points j R + r, whose
 // inputs are load(i0[j] + r n / R), and has no twiddles (its Ls is 1).  The points then make
 // one round trip through shared memory less than when they are placed there first, with a
-// barrier and a table look-up less (at 256^3, 42 shells x 3 sets: x pass 1027 -> 968 us, y pass
+// barrier and a table look-up less (at 256^3, 21 shells x 3 sets: x pass 1027 -> 968 us, y pass
 // 317 -> 243; the z pass, whose inputs take most of its work, gained nothing at 256^3).
 template <int R, class Load>
 __device__ __forceinline__ void first_butterflies(float2 *buf, const int *i0, int nbf, int warp, int nw, int lane,
