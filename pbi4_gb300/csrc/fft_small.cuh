@@ -25,7 +25,6 @@
 
 #include <cuda_runtime.h>
 
-#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -262,9 +261,6 @@ struct FftPlan {
         FftDesc alt;
         if (!factor(false, d)) return false;
         if (allow20 && factor(true, alt) && alt.nst < d.nst) d = alt;
-        // the largest radix last: the first to run, without twiddles, and where the kernels
-        // read it from global memory the one with the most loads in flight
-        std::reverse(d.rad, d.rad + d.nst);
         ent.clear();
         int L = n;
         for (int s = 0; s < d.nst; s++) {

@@ -96,19 +96,28 @@ __device__ __forceinline__ void run_dit(const fftd::FftDesc &fd, float2 *buf, co
 // inputs are load(i0[j] + r n / R), and has no twiddles (its Ls is 1).  The points then make
 // one round trip through shared memory less than when they are placed there first, with a
 // barrier and a table look-up less (at 256^3, 21 shells x 3 sets: x pass 1027 -> 968 us, y pass
-// 317 -> 243; the z pass, whose inputs take most of its work, gained nothing at 256^3).
+// 317 -> 244; the z pass, whose inputs take most of its work, gained nothing at 256^3).
 template <int R, class Load>
 __device__ __forceinline__ void first_butterflies(float2 *buf, const int *i0, int nbf, int warp, int nw, int lane,
                                                   Load &&load) {
-    for (int j = warp; j < nbf; j += nw) {
-        const int i = i0[j];
-        float2 v[fftd::kMaxRadix];
+    constexpr int B = R >= 7 ? 1 : 8 / R;  // small radices: about eight loads in flight
+    for (int j0 = warp; j0 < nbf; j0 += B * nw) {
+        float2 v[B][fftd::kMaxRadix];
 #pragma unroll
-        for (int r = 0; r < R; r++) v[r] = load(i + r * nbf);
-        fftd::dft_small<R>(v);
-        float2 *o = buf + j * (R * kP) + lane;
+        for (int b = 0; b < B; b++) {
+            const int j = j0 + b * nw, i = j < nbf ? i0[j] : 0;
 #pragma unroll
-        for (int q = 0; q < R; q++) o[q * kP] = v[q];
+            for (int r = 0; r < R; r++) v[b][r] = j < nbf ? load(i + r * nbf) : czero();
+        }
+#pragma unroll
+        for (int b = 0; b < B; b++) {
+            const int j = j0 + b * nw;
+            if (j >= nbf) break;
+            fftd::dft_small<R>(v[b]);
+            float2 *o = buf + j * (R * kP) + lane;
+#pragma unroll
+            for (int q = 0; q < R; q++) o[q * kP] = v[b][q];
+        }
     }
 }
 template <bool R20, class Load>
