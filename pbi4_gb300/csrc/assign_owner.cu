@@ -116,15 +116,12 @@ __device__ __forceinline__ void first_and_h(double p, int N, int nintp, bool shi
 // w3 = h^3/6 and w2 = 1 - w0 - w1 - w3; TSC w0 = (1/2 - h)^2 / 2, w1 = 3/4 - h^2,
 // w2 = 1 - w0 - w1; CIC 1 - h, h.  Each lane's stencil indices are fixed, so it
 // picks its coefficients once and evaluates three FMAs per weight.
-// GEN: the constant 1/6 rounded down, so that the weights sum to 1 within 2e-10 (rounded to
-// nearest 3e-8 more), as these grids' did when w2 was formed as 1 - w0 - w1 - w3.
-template <bool GEN> constexpr float kSixth = GEN ? 0.16666665f : 1.f / 6.f;
-template <int NI, bool GEN>
+template <int NI>
 __device__ __forceinline__ float4 axis_poly(int i) {
     if constexpr (NI == 4) {
-        return i == 0 ? make_float4(kSixth<GEN>, -0.5f, 0.5f, -1.f / 6.f)
+        return i == 0 ? make_float4(1.f / 6.f, -0.5f, 0.5f, -1.f / 6.f)
              : i == 1 ? make_float4(2.f / 3.f, 0.f, -1.f, 0.5f)
-             : i == 2 ? make_float4(kSixth<GEN>, 0.5f, 0.5f, -0.5f)
+             : i == 2 ? make_float4(1.f / 6.f, 0.5f, 0.5f, -0.5f)
                       : make_float4(0.f, 0.f, 0.f, 1.f / 6.f);
     } else if constexpr (NI == 3) {
         return i == 0 ? make_float4(0.125f, -0.5f, 0.5f, 0.f)
@@ -158,15 +155,49 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
 }
 __device__ __forceinline__ F2 horner2(const F2 c[4], F2 h) { return fma2(h, fma2(h, fma2(h, c[3], c[2]), c[1]), c[0]); }
 
+// x / 6 rounded to nearest (Markstein's correction of the product with the rounded reciprocal)
+__device__ __forceinline__ float sixth(float x) {
+    const float c = 1.f / 6.f, q = x * c;
+    return fmaf(fmaf(-q, 6.f, x), c, q);
+}
+// All weights of an axis in the forms of axis_stencil (assign.cu), for GEN: the weights that
+// these grids had in the 64-bit grid in global memory, whose rounding the other forms' is not.
+template <int NI>
+__device__ __forceinline__ void axis_direct(float h, float (&w)[NI]) {
+    if constexpr (NI == 4) {
+        const float h2 = h * h;
+        w[0] = sixth((1.f - h) * (1.f - h) * (1.f - h));
+        w[1] = 4.f / 6.f + (0.5f * h - 1.f) * h2;
+        w[3] = sixth(h2 * h);
+        w[2] = 1.f - w[0] - w[1] - w[3];
+    } else if constexpr (NI == 3) {
+        w[0] = 0.5f * (0.5f - h) * (0.5f - h);
+        w[1] = 0.75f - h * h;
+        w[2] = 1.f - w[0] - w[1];
+    } else if constexpr (NI == 2) {
+        w[0] = 1.f - h;
+        w[1] = h;
+    } else {
+        w[0] = 1.f;
+    }
+}
+template <int NI>
+__device__ __forceinline__ float pick_weight(const float (&w)[NI], int i) {
+    float r = w[0];
+#pragma unroll
+    for (int k = 1; k < NI; k++) r = i == k ? w[k] : r;
+    return r;
+}
+
 // s times all weights of an axis, by pairs: axis_poly's cubics, every operation rounded as the
 // single one is, so the three axes err alike (forms of their own for z, though closer to the
 // weights, showed as a quadrupole).
-template <int NI, bool GEN>
+template <int NI>
 __device__ __forceinline__ void axis_products(float s, float h, float (&w)[NI]) {
     const F2 ss = f2(s, s), hh = f2(h, h);
     if constexpr (NI == 4) {
         const F2 w02 = fma2(hh, fma2(hh, fma2(hh, f2(-1.f / 6.f, -0.5f), f2(0.5f, 0.5f)), f2(-0.5f, 0.5f)),
-                            f2(kSixth<GEN>, kSixth<GEN>));
+                            f2(1.f / 6.f, 1.f / 6.f));
         const F2 w13 = fma2(hh, mul2(hh, fma2(hh, f2(0.5f, 1.f / 6.f), f2(-1.f, 0.f))), f2(2.f / 3.f, 0.f));
         const F2 p02 = mul2(ss, w02), p13 = mul2(ss, w13);
         w[0] = f2_lo(p02);
@@ -563,7 +594,7 @@ __device__ __forceinline__ long long add_items(unsigned b, unsigned e, int g0, f
     constexpr int PZ = 4 * pitch_z(NI), HI = 4 * arr_words(NI);
     const unsigned sub = (threadIdx.x & 31) / LPI;
     const int col = (threadIdx.x & 31) % LPI, ci = col % NI, cj = col / NI;
-    const float4 cx = axis_poly<NI, GEN>(ci), cy = axis_poly<NI, GEN>(cj);
+    const float4 cx = axis_poly<NI>(ci), cy = axis_poly<NI>(cj);
     const F2 pxy[4] = {f2(cx.x, cy.x), f2(cx.y, cy.y), f2(cx.z, cy.z), f2(cx.w, cy.w)};
     const bool idle = sub >= IPW;  // (order 3: three items of 9 columns)
     const unsigned n = (e - b) * NG, step = (blockDim.x >> 5) * IPW;
@@ -580,10 +611,19 @@ __device__ __forceinline__ long long add_items(unsigned b, unsigned e, int g0, f
     };
     auto add = [&](const PCell &c, float wt, bool is) {
         if (IPW > NG && (!is || idle)) return;
-        const F2 wxwy = horner2(pxy, f2(c.h[0], c.h[1]));  // w_x and w_y, each rounded as by single FMAs
-        const float wxy = f2_lo(wxwy) * f2_hi(wxwy) * scale;
         float w[NI];
-        axis_products<NI, GEN>(wxy, c.h[2], w);
+        if constexpr (GEN) {
+            float wx[NI], wy[NI];
+            axis_direct<NI>(c.h[0], wx);
+            axis_direct<NI>(c.h[1], wy);
+            axis_direct<NI>(c.h[2], w);
+            const float wxy = pick_weight<NI>(wx, ci) * pick_weight<NI>(wy, cj) * scale;
+#pragma unroll
+            for (int l = 0; l < NI; l++) w[l] *= wxy;
+        } else {
+            const F2 wxwy = horner2(pxy, f2(c.h[0], c.h[1]));  // w_x and w_y, each rounded as by single FMAs
+            axis_products<NI>(f2_lo(wxwy) * f2_hi(wxwy) * scale, c.h[2], w);
+        }
         const unsigned cell = base + (unsigned)(c.pack & (kOut - 1));
         if (F == SHORT || F == SPLIT) {
             flags |= c.pack;
