@@ -49,7 +49,6 @@ struct TriPlan {
     DevBuf tiles;        // int4 [ntiles]: (first f, first g, first q of set 0, unused)
     DevBuf slots;        // int [ntiles][nsets][tq][tf][tg]: output slot or -1
     DevBuf groups;       // int2 [ngroups]: tiles [x, y)
-    DevBuf run;          // FP64 running sums of the FP32 form, one column per thread
     // qoff: added to the map index of every non-cross q (a second copy of the maps)
     int build(const Shells &sh, int nsets, int cross, bool fp64, int qoff = 0);
 };

@@ -31,6 +31,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "widen.cuh"
 
 namespace pbi4g {
 
@@ -110,20 +111,6 @@ __device__ __forceinline__ float shift_f32(float p, float v, const CatArgs &a, i
     const float room = h - 0x1p-42f * (fabsf(s) + fabsf(th));
     if (fabsf(r) > 0x1p-60f && fabsf(r) < 0x1p100f && fabsf(off) < room) return r;
     return shift_ref<float>(p, v, a, d);
-}
-
-// float32 -> float64 in integer arithmetic (conversions run at the FP64 pipe's rate)
-__device__ __forceinline__ double widen(float q) {
-    const unsigned u = __float_as_uint(q);
-    unsigned m = u & 0x7fffffffu;
-    long long bias = 896;
-    if (m < 0x00800000u) {  // zero or subnormal: scaled into the normal range, exactly
-        m = __float_as_uint(fabsf(q) * 0x1p64f);
-        bias = m ? 896 - 64 : 0;
-    } else if (m >= 0x7f800000u) {  // inf, NaN: exponent 2047
-        bias = 2047 - 255;
-    }
-    return __longlong_as_double(((long long)(u >> 31) << 63) | (((long long)m << 29) + (bias << 52)));
 }
 
 // one component: shift, wrap, scale, clip

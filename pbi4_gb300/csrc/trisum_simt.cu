@@ -15,30 +15,30 @@
 //
 // Points are the contiguous axis of the maps in memory and in shared memory: the FP32
 // products and sums are packed pairs of neighbouring points (one packed instruction does
-// two FMAs), with no transposition.  Each accumulator half adds at most 32 products
-// before it is folded into a second-level FP32 sum in shared memory, and that one after
-// 32 folds into an FP64 sum in global memory: its rounding error grows as sqrt(32 + 32)
-// per point, that of one 64-point FP32 chunk under a compensated sum.
+// two FMAs), with no transposition.  Each accumulator half adds at most 32 products (a
+// stage) before it is folded into a Kahan-compensated FP32 sum in shared memory.  (Shell
+// maps are smooth, so a thread's stages add up coherently and a plain FP32 sum of them rounds
+// by more than the stages do: 4 times as much after 32.)  What a fold rounds off is where the
+// accumulator begins the next stage, so the compensation takes no room.
 //
 // What bounds it: the FP32 FMA pipe, and the shared loads next.  A shared load moves 128
 // bytes of registers a cycle however many lanes share an address, so a tile is chosen by
 // both: a 4-point step of a 2 x 4 x 2 tile at S = 3 takes 224 FMA-pipe cycles a scheduler
 // and 192 load cycles an SM for 4 warps (4 x 4 x 1: 208 and 272).  Packed and scalar FMAs
-// reach 34 TFMA/s here with three distinct operands; this kernel runs 22.4 TFMA/s of
+// reach 34 TFMA/s here with three distinct operands; this kernel runs 23.7 TFMA/s of
 // them at the 256^3 box (21 shells, 3 sets), 83% in lanes that hold a tile and 68% of
-// those triangles: 2.55 ms, against 25.3 ms for 4 x 8 tiles of a pairs x maps matrix with
+// those triangles: 2.41 ms, against 25.3 ms for 4 x 8 tiles of a pairs x maps matrix with
 // the products in shared memory and 44% of their entries triangles.  FP64 at 96^3 points
 // and 10 shells: 1.4 ms against 6.7 ms, at the FP64 pipe's rate (0.5 TFMA/s).
 #include <algorithm>
 #include <vector>
 
 #include "bispec.cuh"
+#include "widen.cuh"
 
 namespace pbi4g {
 
 namespace {
-
-constexpr int kFoldPoints = 2048;  // points of a thread between folds into the FP64 sum
 
 // Tile shapes F x G x Q.  FP32: 48 packed accumulators at S = 3, 32 at S = 1.  FP64:
 // 1 x 2 x 2, since its pipe is 64 times slower than the FP32 one and only the work
@@ -76,7 +76,6 @@ template <class T> struct TriArgs {
     const int2 *groups;
     const int *slots;
     double *partial;       // [ksplit * reps][nslots]
-    double *run;           // FP32: [grid][TP TQ S][threads]
 };
 
 __device__ __forceinline__ void cp_async16(void *dst, const void *src, bool valid) {
@@ -142,26 +141,10 @@ __global__ void __launch_bounds__(Shape<T, S>::threads, Shape<T, S>::ctas) trisu
     }
     if (FP32)
         for (int e = 0; e < E / 4; e++) mid_s[(size_t)e * nthr] = make_float4(0.f, 0.f, 0.f, 0.f);
-    double *run = FP32 ? a.run + (size_t)blockIdx.x * E * nthr + tid : nullptr;
-    bool flushed = false;
-    auto flush = [&]() {  // the second-level FP32 sums into the FP64 ones
-#pragma unroll 2
-        for (int e = 0; e < E / 4; e++) {
-            const float4 m = mid_s[(size_t)e * nthr];
-            double *r = run + (size_t)4 * e * nthr;
-            const float v[4] = {m.x, m.y, m.z, m.w};
-#pragma unroll
-            for (int c = 0; c < 4; c++) r[(size_t)c * nthr] = (flushed ? r[(size_t)c * nthr] : 0.0) + (double)v[c];
-            mid_s[(size_t)e * nthr] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        flushed = true;
-    };
 
     const int rowoff = rep * a.sub;
     const int fo = tile.x * pitch + rowoff, go = tile.y * pitch + rowoff, qo = tile.z * pitch + rowoff;
     const int so = a.setrows * pitch;
-    const int folds = kFoldPoints / a.sub;
-    int nfold = 0;
     for (int i = 0; i < a.nstages - 1; i++) issue(i);
     for (int i = 0; i < n; i++) {
         if (a.nstages == 4) asm volatile("cp.async.wait_group 2;" ::: "memory");
@@ -206,24 +189,28 @@ __global__ void __launch_bounds__(Shape<T, S>::threads, Shape<T, S>::ctas) trisu
             }
         }
         if constexpr (FP32) {
+            // m + c, and c - ((m + c) - m) into the accumulator
+            auto fold = [&](float2 m, P &a0, P &a1) {
+                const float2 c = make_float2(PK::sum(a0), PK::sum(a1)), t = __fadd2_rn(m, c);
+                const float2 d = __fadd2_rn(t, make_float2(-m.x, -m.y));
+                const float2 r = __fadd2_rn(c, make_float2(-d.x, -d.y));
+                a0 = make_float2(r.x, 0.f);
+                a1 = make_float2(r.y, 0.f);
+                return t;
+            };
 #pragma unroll
             for (int e = 0; e < E / 4; e++) {
-                float4 m = mid_s[(size_t)e * nthr];
-                m.x += PK::sum(acc[4 * e]);
-                m.y += PK::sum(acc[4 * e + 1]);
-                m.z += PK::sum(acc[4 * e + 2]);
-                m.w += PK::sum(acc[4 * e + 3]);
-                mid_s[(size_t)e * nthr] = m;
+                const float4 m = mid_s[(size_t)e * nthr];
+                const float2 lo = fold(make_float2(m.x, m.y), acc[4 * e], acc[4 * e + 1]);
+                const float2 hi = fold(make_float2(m.z, m.w), acc[4 * e + 2], acc[4 * e + 3]);
+                mid_s[(size_t)e * nthr] = make_float4(lo.x, lo.y, hi.x, hi.y);
             }
         } else {
 #pragma unroll
-            for (int e = 0; e < E; e++) mid_d[e] += acc[e];
-        }
-#pragma unroll
-        for (int e = 0; e < E; e++) acc[e] = PK::zero();
-        if (FP32 && ++nfold == folds) {
-            flush();
-            nfold = 0;
+            for (int e = 0; e < E; e++) {
+                mid_d[e] += acc[e];
+                acc[e] = PK::zero();
+            }
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -236,8 +223,9 @@ __global__ void __launch_bounds__(Shape<T, S>::threads, Shape<T, S>::ctas) trisu
         if (slot < 0) continue;
         double v;
         if constexpr (FP32) {
-            v = (double)reinterpret_cast<const float *>(mid_s + (size_t)(e / 4) * nthr)[e % 4];
-            if (flushed) v += run[(size_t)e * nthr];
+            // (one conversion on the FP64 pipe, not two: its rate shows in small boxes; sums of the
+            // 64^3 box of 86 triangles 34 us, 39 with two)
+            v = (double)reinterpret_cast<const float *>(mid_s + (size_t)(e / 4) * nthr)[e % 4] + widen(acc[e].x);
         } else {
             v = mid_d[e];
         }
@@ -464,11 +452,6 @@ static int launch_trisum(TriPlan &tp, TriArgs<T> &a, DevBuf &partial, double *So
     const int grid = tp.ngroups * a.ksplit, nparts = a.ksplit * a.reps;
     PBI4G_CHECK(partial.ensure(sizeof(double) * (size_t)nparts * tp.nslots));
     a.partial = partial.as<double>();
-    a.run = nullptr;
-    if (sizeof(T) == 4) {
-        PBI4G_CHECK(tp.run.ensure(sizeof(double) * (size_t)grid * E * threads));
-        a.run = tp.run.as<double>();
-    }
     kern<<<grid, threads, smem, st>>>(a);
     PBI4G_LAUNCH_CHECK();
     PBI4G_CHECK(reduce_partials(tp.nslots, nparts, partial.as<double>(), Sout, accumulate, st));
