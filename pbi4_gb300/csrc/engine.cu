@@ -105,15 +105,17 @@ int BkEngine::run(const typename Cx<R>::T *const src[3], const int fac[3], const
     const size_t HC = half_cells(N);
     const int nm = nmaps();
     const bool fp64 = sizeof(R) == 8;
-    if (tp_nsets != nsets || tp_cross != cross || tp_fp64 != (int)fp64) {
-        PBI4G_CHECK(tp.build(sh, cross ? 1 : nsets, cross, fp64));
-        tp_nsets = nsets;
-        tp_cross = cross;
-        tp_fp64 = fp64;
-    }
     PBI4G_CHECK(powsum.ensure(sizeof(double) * 3 * nb));
-    PBI4G_CHECK(S.ensure(sizeof(double) * std::max(1, tp.nslots)));
     const bool tc = tc_mode != 0 && !fp64 && !cross;
+    if (!tc) {
+        if (tp_nsets != nsets || tp_cross != cross || tp_fp64 != (int)fp64) {
+            PBI4G_CHECK(tp.build(sh, cross ? 1 : nsets, cross, fp64));
+            tp_nsets = nsets;
+            tp_cross = cross;
+            tp_fp64 = fp64;
+        }
+        PBI4G_CHECK(S.ensure(sizeof(double) * std::max(1, tp.nslots)));
+    }
     const int form = tc_mode == 1 ? 1 : (tc_mode == 2 ? 2 : 0);  // trisum_tm forms
     if (tc && !tm_supported(sh))
         return set_error(PBI4G_ERR_UNSUPPORTED, "tensor-core triangle sums: map grid %d with %d shells", N, nb);

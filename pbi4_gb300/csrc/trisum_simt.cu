@@ -31,6 +31,7 @@
 // the products in shared memory and 44% of their entries triangles.  FP64 at 96^3 points
 // and 10 shells: 1.4 ms against 6.7 ms, at the FP64 pipe's rate (0.5 TFMA/s).
 #include <algorithm>
+#include <iterator>
 #include <vector>
 
 #include "bispec.cuh"
@@ -296,47 +297,56 @@ int TriPlan::build(const Shells &sh, int nsets_, int cross, bool dbl, int qoff) 
     setrows = nb;
     nslots = (int)(sh.itot * nsets);
     nrows = cross ? 2 * nb : qoff + nsets * nb;
-    // entries (f, g, q shell) -> triangle
-    using Entry = std::pair<std::pair<int, int>, int>;
-    std::vector<std::vector<Entry>> ent(nb);  // by factor map f, sorted by (g, q shell)
+    // entries (g nb + q shell, triangle) of each factor map f, sorted, and q nb + g, sorted
+    std::vector<std::vector<std::pair<int, int>>> ent(nb);
+    std::vector<std::vector<int>> by_q(nb);
     const int q0set = cross ? cross * nb : qoff;
     for (int64_t m = 0; m < sh.itot; m++) {
-        const int l = sh.tri[3 * m], j = sh.tri[3 * m + 1], i = sh.tri[3 * m + 2];
-        if (!cross) ent[j - 1].push_back({{i - 1, l - 1}, (int)m});
-        else ent[l - 1].push_back({{j - 1, i - 1}, (int)m});
+        const int l = sh.tri[3 * m] - 1, j = sh.tri[3 * m + 1] - 1, i = sh.tri[3 * m + 2] - 1;
+        const int f = cross ? l : j, g = cross ? j : i, q = cross ? i : l;
+        ent[f].push_back({g * nb + q, (int)m});
+        by_q[f].push_back(q * nb + g);
     }
-    for (auto &e : ent) std::sort(e.begin(), e.end());
+    for (int f = 0; f < nb; f++) {  // (one of the two is sorted already)
+        if (!std::is_sorted(ent[f].begin(), ent[f].end())) std::sort(ent[f].begin(), ent[f].end());
+        if (!std::is_sorted(by_q[f].begin(), by_q[f].end())) std::sort(by_q[f].begin(), by_q[f].end());
+    }
     // Cover the entries of one run of factor maps with G x Q windows: strips of Q (or G)
     // columns from the first uncovered one, each cut into windows from its last row down;
     // by columns or by rows, whichever needs fewer windows.
-    using Cells = std::vector<std::pair<int, int>>;  // (column, row), sorted
-    std::vector<int> rows;
-    auto cover = [&rows](Cells &cells, int R, int C) {
-        std::sort(cells.begin(), cells.end());
+    std::vector<char> row_used(nb, 0);
+    auto cover = [&](const std::vector<int> &cells, int R, int C) {  // cells: column nb + row, sorted
         std::vector<std::pair<int, int>> w;  // (first column, first row)
-        for (auto it = cells.begin(); it != cells.end();) {
-            const int c0 = it->first;
-            rows.clear();
-            for (; it != cells.end() && it->first < c0 + C; ++it) rows.push_back(it->second);
-            std::sort(rows.begin(), rows.end());
-            int lo = 1 << 30;  // first row of the last window
-            for (auto r = rows.rbegin(); r != rows.rend(); ++r)
-                if (*r < lo) {
-                    lo = std::max(0, *r - R + 1);
-                    w.push_back({c0, lo});
-                }
+        for (size_t k = 0; k < cells.size();) {
+            const int c0 = cells[k] / nb, end = (c0 + C) * nb;
+            int lo = nb, hi = -1;
+            for (; k < cells.size() && cells[k] < end; k++) {
+                const int r = cells[k] % nb;
+                row_used[r] = 1;
+                lo = std::min(lo, r);
+                hi = std::max(hi, r);
+            }
+            for (int r = hi, first = nb; r >= lo; r--) {
+                if (row_used[r] && r < first) w.push_back({c0, first = std::max(0, r - R + 1)});
+                row_used[r] = 0;
+            }
         }
         return w;
     };
+    std::vector<int> qg, gq, tmp;
     auto tiles_from = [&](int first) {  // runs of tf factor maps, the first of `first` maps
         std::vector<int4> tl;
         for (int f0 = 0, f1 = first; f0 < nb; f0 = f1, f1 += tf) {
-            Cells qg, gq;
-            for (int f = f0; f < std::min(f1, nb); f++)
-                for (auto &kv : ent[f]) {
-                    qg.push_back({kv.first.second, kv.first.first});
-                    gq.push_back(kv.first);
-                }
+            qg.clear();
+            gq.clear();
+            for (int f = f0; f < std::min(f1, nb); f++) {
+                tmp.clear();
+                std::merge(qg.begin(), qg.end(), by_q[f].begin(), by_q[f].end(), std::back_inserter(tmp));
+                qg.swap(tmp);
+                const size_t mid = gq.size();
+                for (auto &e : ent[f]) gq.push_back(e.first);
+                std::inplace_merge(gq.begin(), gq.begin() + mid, gq.end());
+            }
             const auto a = cover(qg, tg, tq), b = cover(gq, tq, tg);
             if (a.size() <= b.size())
                 for (auto &w : a) tl.push_back(make_int4(f0, w.second, w.first, f1));
@@ -357,23 +367,25 @@ int TriPlan::build(const Shells &sh, int nsets_, int cross, bool dbl, int qoff) 
     ntiles = (int)tl.size();
     const int E = tf * tg * tq * nsets;
     std::vector<int> st((size_t)ntiles * E, -1);
-    for (int t = 0; t < ntiles; t++) {
-        for (int x = 0; x < tf; x++) {
-            const int f = tl[t].x + x;
-            if (f >= std::min(nb, tl[t].w)) continue;
-            for (int p = 0; p < tg; p++)
-                for (int b = 0; b < tq; b++) {
-                    const std::pair<int, int> gq(tl[t].y + p, tl[t].z + b);
-                    auto it = std::lower_bound(ent[f].begin(), ent[f].end(), gq,
-                                               [](const Entry &e, const std::pair<int, int> &k) { return e.first < k; });
-                    if (it == ent[f].end() || it->first != gq || it->second < 0) continue;
-                    for (int s = 0; s < nsets; s++)
-                        st[(size_t)t * E + ((s * tq + b) * tf + x) * tg + p] = it->second * nsets + s;
-                    it->second = -1;  // windows may overlap: each triangle belongs to one tile
-                }
+    std::vector<std::vector<int>> run(nb);  // first factor map -> tiles
+    for (int t = 0; t < ntiles; t++) run[tl[t].x].push_back(t);
+    std::vector<int> at((size_t)nb * nb, -1);  // the triangles of one f, by (g, q shell)
+    for (int f0 = 0; f0 < nb; f0++) {
+        if (run[f0].empty()) continue;
+        for (int f = f0; f < std::min(nb, tl[run[f0][0]].w); f++) {
+            for (auto &e : ent[f]) at[e.first] = e.second;
+            for (int t : run[f0])
+                for (int p = 0; p < std::min(tg, nb - tl[t].y); p++)
+                    for (int b = 0; b < std::min(tq, nb - tl[t].z); b++) {
+                        int &m = at[(tl[t].y + p) * nb + tl[t].z + b];
+                        if (m < 0) continue;
+                        for (int s = 0; s < nsets; s++)
+                            st[(size_t)t * E + ((s * tq + b) * tf + f - f0) * tg + p] = m * nsets + s;
+                        m = -1;  // windows may overlap: each triangle belongs to one tile
+                    }
         }
-        tl[t].z += q0set;
     }
+    for (auto &t : tl) t.z += q0set;
     // groups of equal size, at most a CTA of tiles each
     const int warps = std::max(1, (ntiles + 31) / 32);
     ngroups = (warps + max_warps - 1) / max_warps;
