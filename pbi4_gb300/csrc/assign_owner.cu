@@ -909,8 +909,15 @@ bool owner_direct(int N, int64_t npart) {
     return owner_supported(N) || (N >= 2 * kT && N <= 2048 && npart <= ((int64_t)1 << 26));
 }
 
-// (whatever the grid: a shared scratch of a large grid also serves plans of few tiles)
-static constexpr size_t kPlaceBytes = sizeof(unsigned) * (size_t)kSmallBlocks * kSmallTiles;  // 2.5 MB
+static int small_blocks(int64_t npart) {
+    return (int)std::min<int64_t>(kSmallBlocks, (npart + kSmallThreads - 1) / kSmallThreads);
+}
+// `place` for grids up to N (a shared scratch of a large grid also serves plans of few tiles) and
+// up to npart particles: at most 16 bytes a particle and 8 KB
+static size_t place_bytes(int N, int64_t npart) {
+    const size_t nt = (size_t)((N + kT - 1) / kT);
+    return sizeof(unsigned) * (size_t)small_blocks(npart) * std::min<size_t>(nt * nt * nt, kSmallTiles);
+}
 
 bool OwnerWork::fits(int N, int64_t npart) const {
     const int nt = (N + kT - 1) / kT;
@@ -918,7 +925,7 @@ bool OwnerWork::fits(int N, int64_t npart) const {
     const size_t n = (size_t)(npart > 0 ? npart : 1);
     return count.p && count.bytes >= (ntiles + 2) * 4 && start.bytes >= (ntiles + 1) * 4 &&
            cursor.bytes >= (ntiles + 1) * 4 && sorted.bytes >= 8 * n * sizeof(PTile) && wsorted.bytes >= 8 * n * 4 && wmax.bytes >= 8 &&
-           place.bytes >= kPlaceBytes;
+           place.bytes >= place_bytes(N, (int64_t)n);
 }
 
 int OwnerWork::ensure(int N, int64_t npart) {
@@ -937,7 +944,7 @@ int OwnerWork::ensure(int N, int64_t npart) {
     PBI4G_CHECK(sorted.ensure(8 * n * sizeof(PTile)));
     PBI4G_CHECK(wsorted.ensure(8 * n * 4));
     PBI4G_CHECK(wmax.ensure(8));
-    PBI4G_CHECK(place.ensure(kPlaceBytes));
+    PBI4G_CHECK(place.ensure(place_bytes(N, (int64_t)n)));
     return PBI4G_OK;
 }
 
@@ -947,8 +954,10 @@ void OwnerWork::release() {
 
 size_t OwnerWork::footprint(int N, int64_t npart) {
     const size_t nt = (size_t)((N + kT - 1) / kT);
-    // (32 bytes a particle more than ensure takes: callers have their budgets from this size)
-    return 3 * (nt * nt * nt + 2) * 4 + (size_t)npart * (32 + 8 * (sizeof(PTile) + 4)) + 64;
+    // (`place` takes less than 32 bytes a particle from 512 particles on: callers have their
+    // budgets from this size, so it stays)
+    return 3 * (nt * nt * nt + 2) * 4 + std::max((size_t)npart * 32, place_bytes(N, npart)) +
+           (size_t)npart * 8 * (sizeof(PTile) + 4) + 64;
 }
 
 void owner_ptrs_host(const OwnerWork &wk, unsigned char (&block)[kOwnerPtrBytes]) {
@@ -1012,8 +1021,7 @@ int assign_owner(OwnerWork &wk, const void *d_ptrs, int N, int nintp, bool inter
     // few tiles: a block counts its share in shared memory, over about two blocks an SM
     const bool small = ntiles <= kSmallTiles;
     const int threads = small ? kSmallThreads : kSortThreads;
-    const int blocks = small ? (int)std::min<int64_t>(kSmallBlocks, (npart + threads - 1) / threads)
-                             : grid_blocks(npart, threads);
+    const int blocks = small ? small_blocks(npart) : grid_blocks(npart, threads);
     pf.begin(sort_stage, st);
     // counts and the tile counter
     auto sort = [&](auto ind, auto general, auto few) -> int {

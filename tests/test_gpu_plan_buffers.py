@@ -1,15 +1,22 @@
-"""What a plan allocates: no tables of a form it does not use."""
+"""What a plan allocates: no tables of a form it does not use, and no more than its footprint
+says."""
 import numpy as np
 import pytest
 
 from pbi4_gb300._lib import lib
-from pbi4_gb300.estimator import Estimator, EstimatorConfig
+from pbi4_gb300.estimator import AssignScratch, Estimator, EstimatorConfig, footprint
 
 pytestmark = pytest.mark.gpu
 
 
 def _allocs():
     return int(lib().pbi4g_device_allocs())
+
+
+def _free():
+    import torch
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
 
 
 def test_tensor_form_builds_its_own_tables_only():
@@ -29,3 +36,59 @@ def test_tensor_form_builds_its_own_tables_only():
         made[prec] = _allocs() - n
         est.close()
     assert made["tf32split"] == made["fp32"] + 2
+
+
+def test_small_scratch_within_its_footprint():
+    """Scratches for a few particles: 128 of them, so that the driver's pages (2 MiB) show only
+    once.  (A scratch's buffers below 1 MiB share pages.)"""
+    AssignScratch(32, 1).close()  # the context and the module
+    free = _free()
+    made = [AssignScratch(64, 1000) for _ in range(128)]
+    held = free - _free()
+    want = sum(s.bytes for s in made)
+    for s in made:
+        s.close()
+    assert held <= want + (16 << 20), (held, want)
+
+
+@pytest.mark.parametrize("grid,npart", [(32, 1), (32, 100), (32, 513), (256, 300), (48, 20000), (208, 20000), (256, 40)])
+def test_scratch_serves_every_smaller_box(grid, npart):
+    """A scratch of the largest grid and particle number holds the boxes of smaller ones."""
+    import torch
+    sc = AssignScratch(grid, npart)
+    rng = np.random.default_rng(grid)
+    for g in sorted({32, grid, max(32, grid // 32 * 16), min(grid, 192)}):
+        for n in {1, max(1, npart // 3), npart}:
+            est = Estimator(EstimatorConfig(grid=g, box=1000.0, do_bispectrum=False))
+            pos = torch.from_numpy(rng.random((3, n))).cuda()
+            est.density(n, pos)
+            own = est.delta_half()
+            est.use_scratch(sc)
+            est.density(n, pos)
+            assert est.delta_half().tobytes() == own.tobytes()
+            est.close()
+    sc.close()
+
+
+@pytest.mark.parametrize("kw", [dict(grid=256, kbin_bs=8.0, kcenter_bs=8.0, nbins_bs=8, multipoles=True),
+                                dict(grid=128, kbin_bs=1.0, kcenter_bs=1.0, nbins_bs=41, multipoles=True),
+                                dict(grid=160, kbin_bs=1.0, kcenter_bs=1.0, nbins_bs=53, multipoles=False),
+                                dict(grid=128, kbin_bs=1.0, kcenter_bs=1.0, nbins_bs=20, multipoles=True, map_budget_mb=16)])
+@pytest.mark.parametrize("precision", ["fp32", "fp16split"])
+def test_plan_within_its_footprint(kw, precision):
+    import torch
+    cfg = EstimatorConfig(box=1000.0, precision=precision, **kw)
+    n = 20000
+    pos = torch.rand((3, n), dtype=torch.float64, device="cuda")
+    out = Estimator(cfg).alloc_outputs()
+    warm = Estimator(cfg)  # loads the modules, counts the triangles
+    warm.run_device(n, pos, *out)
+    warm.check()
+    warm.close()
+    free = _free()
+    est = Estimator(cfg)
+    est.run_device(n, pos, *out)
+    est.check()
+    held = free - _free()
+    est.close()
+    assert held <= footprint(cfg, n), (held, footprint(cfg, n))
