@@ -322,12 +322,14 @@ int bk_finalize(const Shells &sh, int nsets, int cross, const double *S, const d
 static std::mutex g_counts_mutex;
 static std::map<std::tuple<int, float, float, int, int, int>, std::vector<int64_t>> g_counts_cache;
 
-static int upload_counts(Shells &sh) {
+// sh.counts says that counts_f32 holds them: it is set last
+static int upload_counts(Shells &sh, const std::vector<int64_t> &counts) {
     const double gridD = (double)sh.N * sh.N * sh.N;
     std::vector<float> c32(sh.itot);
-    for (int64_t m = 0; m < sh.itot; m++) c32[m] = (float)(gridD * (double)sh.counts[m]);
+    for (int64_t m = 0; m < sh.itot; m++) c32[m] = (float)(gridD * (double)counts[m]);
     PBI4G_CHECK(sh.counts_f32.ensure(sizeof(float) * std::max<int64_t>(1, sh.itot)));
     PBI4G_CUDA(cudaMemcpy(sh.counts_f32.p, c32.data(), sizeof(float) * sh.itot, cudaMemcpyHostToDevice));
+    sh.counts = counts;
     return PBI4G_OK;
 }
 
@@ -394,10 +396,7 @@ int triangle_counts(Shells &sh, cudaStream_t st, int64_t *launches) {
     {
         std::lock_guard<std::mutex> g(g_counts_mutex);
         auto it = g_counts_cache.find(ckey);
-        if (it != g_counts_cache.end()) {
-            sh.counts = it->second;
-            return upload_counts(sh);
-        }
+        if (it != g_counts_cache.end()) return upload_counts(sh, it->second);
     }
     const int N = sh.Nm, nb = sh.nb, NH = N / 2 + 1;  // indicator maps on the map grid
     if (N > 2046) return set_error(PBI4G_ERR_UNSUPPORTED, "counts: map grid %d", N);
@@ -463,23 +462,21 @@ int triangle_counts(Shells &sh, cudaStream_t st, int64_t *launches) {
     PBI4G_CUDA(cudaMemcpyAsync(Sh.data(), S.p, sizeof(double) * tp.nslots, cudaMemcpyDeviceToHost, st));
     PBI4G_CUDA(cudaStreamSynchronize(st));
     const double gridD = (double)N * N * N;
-    sh.counts.resize(sh.itot);
+    std::vector<int64_t> counts(sh.itot);
     double maxdev = 0;
     for (int64_t m = 0; m < sh.itot; m++) {
         double v = Sh[m] / gridD;
         long long c = llround(v);
         maxdev = std::max(maxdev, fabs(v - (double)c));
-        sh.counts[m] = c;
+        counts[m] = c;
     }
-    if (maxdev > 0.25) {
-        sh.counts.clear();
+    if (maxdev > 0.25)
         return set_error(PBI4G_ERR_RANGE, "triangle counts not resolved to integers (max deviation %g)", maxdev);
-    }
     {
         std::lock_guard<std::mutex> g(g_counts_mutex);
-        g_counts_cache[ckey] = sh.counts;
+        g_counts_cache[ckey] = counts;
     }
-    return upload_counts(sh);
+    return upload_counts(sh, counts);
 }
 
 }  // namespace pbi4g

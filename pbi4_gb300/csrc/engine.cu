@@ -840,14 +840,15 @@ int pbi4g_plan_set_counts(pbi4g_plan *p, const double *counts_host) {
     if (!p->cfg.do_bispectrum) return set_error(PBI4G_ERR_INVALID, "plan has no bispectrum");
     Shells &sh = p->bk.sh;
     const double gridD = (double)p->N * p->N * p->N;
-    sh.counts.assign(sh.itot, 0);
+    std::vector<int64_t> counts(sh.itot);
     std::vector<float> c32(sh.itot);
     for (int64_t m = 0; m < sh.itot; m++) {
         c32[m] = (float)counts_host[m];
-        sh.counts[m] = llround(counts_host[m] / gridD);
+        counts[m] = llround(counts_host[m] / gridD);
     }
     PBI4G_CHECK(sh.counts_f32.ensure(sizeof(float) * std::max<int64_t>(1, sh.itot)));
     PBI4G_CUDA(cudaMemcpy(sh.counts_f32.p, c32.data(), sizeof(float) * sh.itot, cudaMemcpyHostToDevice));
+    sh.counts = counts;  // (says that counts_f32 holds them)
     return PBI4G_OK;
 }
 

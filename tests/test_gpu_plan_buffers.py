@@ -1,9 +1,9 @@
-"""What a plan allocates: no tables of a form it does not use, and no more than its footprint
-says."""
+"""What a plan allocates: no tables of a form it does not use, no more than its footprint says,
+and what becomes of a box that finds no room."""
 import numpy as np
 import pytest
 
-from pbi4_gb300._lib import lib
+from pbi4_gb300._lib import Pbi4GpuError, lib
 from pbi4_gb300.estimator import AssignScratch, Estimator, EstimatorConfig, footprint
 
 pytestmark = pytest.mark.gpu
@@ -92,3 +92,33 @@ def test_plan_within_its_footprint(kw, precision):
     held = free - _free()
     est.close()
     assert held <= footprint(cfg, n), (held, footprint(cfg, n))
+
+
+def _run(est, pos):
+    import torch
+    out = est.alloc_outputs()
+    est.run_device(pos.shape[1], torch.from_numpy(pos).cuda(), *out)
+    est.check()
+    return [o.cpu().numpy() for o in out]
+
+
+def test_counts_without_room_are_counted_again():
+    """A box whose triangle counts find no room on the device fails; the next one makes them."""
+    import torch
+    cfg = EstimatorConfig(grid=64, box=1000.0, kbin_bs=4.0, kcenter_bs=4.0, nbins_bs=4)
+    pos = np.random.default_rng(8).random((3, 5000))
+    est = Estimator(cfg)
+    ref = _run(est, pos)  # (counted once a process)
+    est.close()
+    est = Estimator(cfg)
+    est.density(5000, torch.from_numpy(pos).cuda())
+    bout = est.alloc_outputs()[1]
+    try:
+        assert lib().pbi4g_debug_fail_alloc(1) == 0
+        with pytest.raises(Pbi4GpuError):
+            est.bispectrum(bout)
+    finally:
+        lib().pbi4g_debug_fail_alloc(0)
+    est.bispectrum(bout)
+    np.testing.assert_array_equal(bout.cpu().numpy()[8], ref[1][8])
+    est.close()
