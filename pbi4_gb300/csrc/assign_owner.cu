@@ -928,6 +928,8 @@ bool OwnerWork::fits(int N, int64_t npart) const {
            place.bytes >= place_bytes(N, (int64_t)n);
 }
 
+int64_t OwnerWork::particles() const { return (int64_t)(sorted.bytes / (8 * sizeof(PTile))); }
+
 int OwnerWork::ensure(int N, int64_t npart) {
     if (fixed) {
         if (fits(N, npart)) return PBI4G_OK;

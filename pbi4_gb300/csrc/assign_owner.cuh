@@ -9,6 +9,7 @@ struct OwnerWork {
     bool fixed = false;  // a shared scratch: sized once, never reallocated (ensure fails instead)
     int ensure(int N, int64_t npart);
     bool fits(int N, int64_t npart) const;
+    int64_t particles() const;  // that its records hold
     void release();
     static size_t footprint(int N, int64_t npart);
 };

@@ -267,6 +267,7 @@ struct pbi4g_plan {
     BkEngine bk;
     bool have_delta = false;
     int64_t npart = 0;
+    int64_t rec_refused = INT64_MAX;  // boxes from so many particles on do without records (give_up_records)
     Prof prof;
     // captured form (pbi4g_plan_graph_*): `batch` box slots of at most `cap` particles
     struct Graphs {
@@ -302,6 +303,26 @@ static int check_config(const pbi4g_config *c) {
     for (int k = 0; k < 6; k++)
         if (c->reserved[k]) return set_error(PBI4G_ERR_INVALID, "reserved config fields must be zero");
     return PBI4G_OK;
+}
+
+// Grids that are not a multiple of 16 can be assigned without records (288 bytes a particle),
+// in a 64-bit grid in global memory: their records give way to any other buffer that finds no
+// room.  A plan that has given up records of npart particles does not try so many again (a
+// box would otherwise repeat the failing allocations, or fail another stage's).
+static void give_up_records(pbi4g_plan *p, int64_t npart) {
+    cudaStreamSynchronize(p->st);
+    p->ow.release();
+    cudaGetLastError();  // (a failed allocation's)
+    p->rec_refused = std::min(p->rec_refused, npart);
+}
+
+// f(), and once more without the plan's records where it found no room beside them
+template <class F> static int with_room(pbi4g_plan *p, F &&f) {
+    const int rc = f();
+    const int64_t held = p->fp64 || owner_supported(p->N) ? 0 : p->ow.particles();
+    if ((rc != PBI4G_ERR_NOMEM && rc != PBI4G_ERR_CUFFT) || held == 0) return rc;
+    give_up_records(p, held);
+    return f();
 }
 
 extern "C" {
@@ -548,11 +569,11 @@ static int owner_bind(pbi4g_plan *p, int64_t npart) {
 static int density_impl(pbi4g_plan *p, int64_t npart, const double *d_pos, const double *d_weight, const BoxPar *bp) {
     const int N = p->N;
     int bits;
-    bool owner = !p->fp64 && (bp ? owner_supported(N) : owner_direct(N, npart));
-    if (owner && !bp && !owner_supported(N) && p->ow_cur->ensure(N, npart) != PBI4G_OK) {
+    bool owner = !p->fp64 && (bp || owner_supported(N) ? owner_supported(N)
+                                                       : owner_direct(N, npart) && npart < p->rec_refused);
+    if (owner && !owner_supported(N) && p->ow.ensure(N, npart) != PBI4G_OK) {
         // no room for this grid's records: the 64-bit grid in global memory
-        p->ow_cur->release();
-        cudaGetLastError();
+        give_up_records(p, npart);
         owner = false;
     }
     if (owner) {
@@ -595,7 +616,7 @@ static int density_impl(pbi4g_plan *p, int64_t npart, const double *d_pos, const
 int pbi4g_plan_density(pbi4g_plan *p, int64_t npart, const double *d_pos, const double *d_weight) {
     if (!p) return set_error(PBI4G_ERR_INVALID, "null plan");
     if (npart < 1) return set_error(PBI4G_ERR_INVALID, "npart must be >= 1");
-    return density_impl(p, npart, d_pos, d_weight, nullptr);
+    return with_room(p, [&] { return density_impl(p, npart, d_pos, d_weight, nullptr); });
 }
 
 int pbi4g_plan_powerspectrum(pbi4g_plan *p, double *d_pout) {
@@ -616,7 +637,10 @@ int pbi4g_plan_powerspectrum(pbi4g_plan *p, double *d_pout) {
 
 static int bispectrum_impl(pbi4g_plan *p, double *d_bout, const BoxPar *bp);
 
-int pbi4g_plan_bispectrum(pbi4g_plan *p, double *d_bout) { return bispectrum_impl(p, d_bout, nullptr); }
+int pbi4g_plan_bispectrum(pbi4g_plan *p, double *d_bout) {
+    if (!p) return set_error(PBI4G_ERR_INVALID, "null plan/output");
+    return with_room(p, [&] { return bispectrum_impl(p, d_bout, nullptr); });
+}
 
 static int bispectrum_impl(pbi4g_plan *p, double *d_bout, const BoxPar *bp) {
     if (!p || !d_bout) return set_error(PBI4G_ERR_INVALID, "null plan/output");
@@ -762,18 +786,18 @@ int pbi4g_plan_run_host(pbi4g_plan *p, int64_t npart, const double *pos, const d
                         double *bout) {
     if (!p || !pos || !pout) return set_error(PBI4G_ERR_INVALID, "null argument");
     if (p->cfg.do_bispectrum && !bout) return set_error(PBI4G_ERR_INVALID, "null bout");
-    PBI4G_CHECK(p->pos_stage.ensure(sizeof(double) * 3 * (size_t)npart));
+    PBI4G_CHECK(with_room(p, [&] { return p->pos_stage.ensure(sizeof(double) * 3 * (size_t)npart); }));
     PBI4G_CUDA(cudaMemcpyAsync(p->pos_stage.p, pos, sizeof(double) * 3 * (size_t)npart, cudaMemcpyHostToDevice, p->st));
     const double *dw = nullptr;
     if (weight) {
-        PBI4G_CHECK(p->w_stage.ensure(sizeof(double) * (size_t)npart));
+        PBI4G_CHECK(with_room(p, [&] { return p->w_stage.ensure(sizeof(double) * (size_t)npart); }));
         PBI4G_CUDA(cudaMemcpyAsync(p->w_stage.p, weight, sizeof(double) * (size_t)npart, cudaMemcpyHostToDevice, p->st));
         dw = p->w_stage.as<double>();
     }
     const size_t pb = sizeof(double) * 5 * p->cfg.nbins_ps;
     const size_t bb = p->cfg.do_bispectrum ? sizeof(double) * (p->cfg.multipoles ? 11 : 9) * p->bk.sh.itot : 0;
-    PBI4G_CHECK(p->pout_d.ensure(pb));
-    if (bb) PBI4G_CHECK(p->bout_d.ensure(bb));
+    PBI4G_CHECK(with_room(p, [&] { return p->pout_d.ensure(pb); }));
+    if (bb) PBI4G_CHECK(with_room(p, [&] { return p->bout_d.ensure(bb); }));
     PBI4G_CHECK(pbi4g_plan_run_device(p, npart, p->pos_stage.as<double>(), dw, p->pout_d.as<double>(),
                                       bb ? p->bout_d.as<double>() : nullptr));
     PBI4G_CUDA(cudaMemcpyAsync(pout, p->pout_d.p, pb, cudaMemcpyDeviceToHost, p->st));

@@ -1,5 +1,6 @@
 """What a plan allocates: no tables of a form it does not use, no more than its footprint says,
-and what becomes of a box that finds no room."""
+and on grids that are not a multiple of 16, whose assignment can do without its particle
+records, no box that fails for the room they take."""
 import numpy as np
 import pytest
 
@@ -94,12 +95,61 @@ def test_plan_within_its_footprint(kw, precision):
     assert held <= footprint(cfg, n), (held, footprint(cfg, n))
 
 
+GEN = dict(grid=50, box=1000.0, nintp=4, interlacing=True, multipoles=True, kbin_bs=3.0, kcenter_bs=3.0, nbins_bs=4)
+
+
 def _run(est, pos):
     import torch
     out = est.alloc_outputs()
     est.run_device(pos.shape[1], torch.from_numpy(pos).cuda(), *out)
     est.check()
     return [o.cpu().numpy() for o in out]
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp16split"])
+def test_records_give_way_to_later_stages(precision):
+    """Whatever allocation of a box fails for want of room while the records are held: the
+    records are given up and the box goes through, with the same density."""
+    cfg = EstimatorConfig(precision=precision, **GEN)
+    pos = np.random.default_rng(5).random((3, 5000))
+    est = Estimator(cfg)
+    est.triangle_counts()  # (counted once a process)
+    n = _allocs()
+    ref = _run(est, pos)
+    n = _allocs() - n
+    delta = est.delta_half().tobytes()
+    est.close()
+    for k in range(1, n + 1):
+        est = Estimator(cfg)
+        try:
+            assert lib().pbi4g_debug_fail_alloc(k) == 0
+            got = _run(est, pos)
+        finally:
+            lib().pbi4g_debug_fail_alloc(0)
+        assert est.delta_half().tobytes() == delta, k
+        for a, b in zip(got, ref):
+            np.testing.assert_allclose(a, b, rtol=1e-5, atol=1e-6 * np.abs(b).max())
+        _run(est, pos)
+        made = _allocs()
+        _run(est, pos)  # no second attempt at the same size
+        assert _allocs() == made, k
+        est.close()
+
+
+def test_records_tried_again_for_fewer_particles():
+    pos = np.random.default_rng(6).random((3, 6000))
+    est = Estimator(EstimatorConfig(precision="fp32", **dict(GEN, multipoles=False)))
+    try:
+        assert lib().pbi4g_debug_fail_alloc(1) == 0
+        _run(est, pos)
+    finally:
+        lib().pbi4g_debug_fail_alloc(0)
+    made = _allocs()
+    _run(est, pos)
+    assert _allocs() == made
+    _run(est, np.ascontiguousarray(pos[:, :3000]))
+    assert _allocs() > made  # the records of half as many
+    est.close()
 
 
 def test_counts_without_room_are_counted_again():
