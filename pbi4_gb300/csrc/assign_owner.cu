@@ -555,9 +555,12 @@ __device__ __forceinline__ unsigned atom_shared(unsigned a, unsigned v) {
 //    cell's sum is at least -kSumBias and a sum beyond 32 bits loses a positive multiple of
 //    2^32.  The tile's contributions are also summed in 64-bit registers: the cells hold
 //    their true sums exactly when the two totals agree.  If they do not, or a position lay
-//    outside the box, or a particle weight is negative, a second pass (HIGH) sums the
-//    contributions' bits from 16 up: with less than 2^16 records, the sum of the low 16 bits
-//    is what the first pass's sum holds beyond it.
+//    outside the box, or a particle weight is negative, a second pass (HIGH or FLAGGED) sums
+//    the contributions' part above 16 bits: with less than 2^16 records, the sum of what is
+//    left of them, 0 to 2^16 each, is what the first pass's sum holds beyond it.  HIGH takes
+//    the part, at most 2^12, as the floor of the contribution before it is rounded, from the
+//    low bits of a sum with 1.5 2^23; contributions that may be anything (FLAGGED) are
+//    converted and shifted, at a quarter of that rate.
 //    kFree: up to so many records no cell can reach 2^32 (a contribution is at most
 //    2^28 times the largest weight of the stencil), and the totals are not compared.
 //  * SPLIT: one grid at a time, the integer cut into the part above its low L bits and those
@@ -567,20 +570,20 @@ __device__ __forceinline__ unsigned atom_shared(unsigned a, unsigned v) {
 //  * WIDE: one grid at a time as 64-bit sums, low words and high words (array 0 and 1):
 //    the low word's atomic returns the old word, from which follows the carry.
 // The sums are the same integers in every form.  (2 10^6 particles in 256^3, order 4 on two
-// grids: 64-bit words 483 us, SHORT 258; 10^8: 19.9 ms, SHORT 9.3.  Where
-// every tile has a cell beyond 16 particles, SHORT and HIGH take 516 against 475 us, and 3.83
-// against 4.12 ms at 2 10^7.)
+// grids: 64-bit words 481 us, SHORT 266; 10^8: 19.9 ms, SHORT 9.7.  Where every tile has a
+// cell beyond 16 particles, SHORT and HIGH take 491 against 448 us, and 3.61 against 3.93 ms at
+// 2 10^7; with FLAGGED for HIGH 522 us and 3.63 ms.)
 constexpr unsigned kSumBias = 1u << 24;
 constexpr unsigned kShortRecords = (1u << 16) - 1, kSplitRecords = 1u << 23;
 constexpr int kAhead = 4;
 __host__ __device__ constexpr unsigned free_records(int ni) { return ni == 4 ? 52u : (ni == 3 ? 36u : 15u); }
-enum Form { SHORT, HIGH, SPLIT, WIDE };
+enum Form { SHORT, HIGH, FLAGGED, SPLIT, WIDE };
 
 // Add the tile's items: an item is one record's stencil on one grid (NG = 2: both grids in
 // turn, each into its own array; NG = 1: grid g0).  LPI lanes take an item, lane (j, i) of
 // them the z column of cells (i, j, 0 .. NI - 1): the x and y weights and their product are
 // formed once per column, the z weights per cell, in the reference's order
-// ((w_x w_y) w_z) weight.  The scale (2^S; with GEN 2^(S - L) in SPLIT and 1 in WIDE) rides in the
+// ((w_x w_y) w_z) weight.  The scale (2^S; 2^(S - 16) in HIGH; with GEN 2^(S - L) in SPLIT and 1 in WIDE) rides in the
 // product (a power of two: the same bits as scaling at the end), so a contribution rounds
 // straight to an integer below 2^30.  GEN (grids that are not a multiple of 16): every
 // contribution is kept to 2^-bits, the resolution these grids had when their particles were
@@ -638,6 +641,8 @@ __device__ __forceinline__ long long add_items(unsigned b, unsigned e, int g0, f
                 red_shared(cell + l * PZ, (unsigned)q);
                 part += q;
             } else if constexpr (F == HIGH) {
+                red_shared(cell + l * PZ, (unsigned)(__float_as_int(__fadd_rd(wv, 12582912.f)) - 0x4B400000));
+            } else if constexpr (F == FLAGGED) {
                 red_shared(cell + l * PZ, (unsigned)(__float2int_rn(wv) >> 16));
             } else if constexpr (F == SPLIT) {
                 int hi, lo;
@@ -796,8 +801,12 @@ __global__ void __launch_bounds__(kThreads, 2) owner_tile_kernel(const TileGeom 
                 // the first pass's sums wait in the grid
                 cells([&](uint4 &v, float4 *o) { *reinterpret_cast<uint4 *>(o) = v; });
                 __syncthreads();
-                add_items<NI, G, W, false, HIGH>(b, e, 0, scale, bits, 0, sorted, wsorted, acc, flags,
-                                                 [&] { clear(NW, 0u); });
+                auto none = [&] { clear(NW, 0u); };
+                if (s_bad[par][2])
+                    add_items<NI, G, W, false, FLAGGED>(b, e, 0, scale, bits, 0, sorted, wsorted, acc, flags, none);
+                else
+                    add_items<NI, G, W, false, HIGH>(b, e, 0, scale * ldexp_bits(-16), bits, 0, sorted, wsorted, acc,
+                                                     flags, none);
                 __syncthreads();
                 cells([&](uint4 &v, float4 *o) {
                     const uint4 low = *reinterpret_cast<const uint4 *>(o);
