@@ -164,7 +164,7 @@ int pbi4g_plan_destroy(pbi4g_plan *plan);
 int pbi4g_plan_set_stream(pbi4g_plan *plan, void *stream);
 
 /* Shared assignment scratch.  The FP32 and tensor-core forms count-sort the
- * particles into per-tile records (up to 8 per particle: 3.2 GB at 10^7
+ * particles into per-tile records (up to 8 per particle: 2.9 GB at 10^7
  * particles) in buffers each plan owns, and the captured form holds `batch` position
  * slots of its capacity.  Plans that run one after another on one stream (a
  * serving slot) can share one scratch instead: pbi4g_plan_use_scratch points the

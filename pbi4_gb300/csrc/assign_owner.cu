@@ -1,5 +1,5 @@
 // assign_owner.cu -- mass assignment for the FP32 / mixed estimator plan:
-// owner-computes 16^3 tiles, 64-bit fixed-point accumulation in shared memory,
+// owner-computes tiles, fixed-point sums in 32-bit shared words whose exactness is checked,
 // FP32 grids written with plain stores.
 //
 // Same indices and weights as powerI4.f90:68-249 (see assign.cu); the weights
@@ -20,12 +20,13 @@
 // Tiles are 16^3 cells on grids that are a multiple of 16 and 10 to 16 cells an
 // axis on others (TileGeom).
 //
-// The sort is bound by instruction issue and the FP64 pipe, not by its 25 MB of
-// positions (2.1e6 particles in 256^3, PCS on two grids): count 37 us (FP64 pipe
+// The sort is bound by instruction issue and the FP64 pipe, not by its 50 MB of
+// positions, read twice (2.1e6 particles in 256^3, PCS on two grids): count 37 us (FP64 pipe
 // 67% busy with two operations a coordinate; issue 54%), scatter 75 us (issue 62%).
 // With prepared particles written by the count and read back by the scatter, and
-// the cells from FP64 arithmetic, the two took 154 us.
-// The tiles are bound by instruction issue (67% at 2 10^6 random particles in 256^3, 258 us;
+// the cells from FP64 arithmetic, the two took 154 us.  (Of 10^8 particles in random order on the
+// same 4096 tiles that form takes 12.5 ms, this one 14; the tiles gain 10 ms there.)
+// The tiles are bound by instruction issue (67% at 2 10^6 random particles in 256^3, 266 us;
 // 54 instructions a record of two grids) and next by the shared atomics; in dense boxes the
 // other way round.  Of the 483 us before, with 64-bit atomics on the cells inside the tile, the
 // tests of every cell, its branch and coefficients reloaded for want of registers took half.

@@ -457,8 +457,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     } else if (warp < kMmaWarp) {
         // ---------------------------------------------------------------- drain
         // each chunk's accumulator is added into FP32 registers (round to nearest);
-        // every kFold chunks those are folded into a Kahan-compensated sum (in TMEM, or
-        // an L2-resident scratch), written out at the end
+        // every kFold chunks those are folded into a Kahan-compensated sum in TMEM, written out
+        // at the end
         // (the two warpgroups take half of the unit's columns each, in groups of 8)
         const int quad = warp & 3, cgrp = (warp - kProdWarps) >> 2;
         // NG: groups of 8 columns per warpgroup (a unit of 16 NG columns)

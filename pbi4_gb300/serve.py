@@ -21,7 +21,7 @@ Admission is by device footprint: a batch starts when a slot is free and the
 plan it needs fits under the HBM budget; idle plans are evicted least recently
 used to make room, and a request whose plan can never fit is rejected.  The
 plans that run on one slot share its assignment record buffers (AssignScratch,
-3.2 GB at 10^7 particles), so a resident plan holds only its grids, tables and
+2.9 GB at 10^7 particles), so a resident plan holds only its grids, tables and
 maps.  Each
 batch is issued asynchronously on its slot's stream (pageable positions are
 staged by the driver, outputs land in pinned buffers) followed by an event; the
@@ -103,7 +103,7 @@ class Server:
         self.batch = int(batch)
         self.lookahead = int(lookahead)
         # one set of assignment record buffers per slot, shared by every plan up to
-        # scratch_grid_max that runs there (a plan's own would be 3.2 GB at 10^7
+        # scratch_grid_max that runs there (a plan's own would be 2.9 GB at 10^7
         # particles), counted as resident; larger grids keep their own
         self.shared_scratch = bool(shared_scratch)
         self.scratch_grid_max = int(scratch_grid_max)
